@@ -121,11 +121,13 @@ struct xnb_batch {
     int hw = 0;
     e.far_coords = 0;
     e.unpacked = 0;
+    e.list_slot = 0;
     for (size_t s = 0; s < sys.size(); ++s)
       if (sys[s].active) {
         hw = static_cast<int>(s) + 1;
         if (sys[s].d.far_coords) e.far_coords = 1;
         if (!sys[s].d.packed_lo) e.unpacked = 1;
+        e.list_slot = std::max(e.list_slot, sys[s].d.list_slot);
       }
     e.nsys = hw;
     e.sm_count = sm_count;
@@ -312,6 +314,7 @@ SysDesc make_desc(const xnb_lj_params& p) {
   d.pre_margin_f = static_cast<float>(4.0 * err_at(p.rcut));
   for (int a = 0; a < 3; ++a) {
     d.period_f[a] = static_cast<float>(d.period[a]);
+    d.period_lo_f[a] = static_cast<float>(d.period[a] - static_cast<double>(d.period_f[a]));
     d.outer_lo_f[a] = static_cast<float>(d.outer_lo[a] - d.origin[a]);
     d.outer_hi_f[a] = static_cast<float>(d.outer_hi[a] - d.origin[a]);
   }
@@ -330,6 +333,17 @@ SysDesc make_desc(const xnb_lj_params& p) {
     // the packed residual's absolute error grows with X: beyond X = 1024 sigma
     // (lo_step 2^-24) the mixed traversal gathers the FP32 residual mirror instead
     d.packed_lo = e <= 10 ? 1 : 0;
+  }
+  {
+    // An image displacement summed from FP32 pairs (image_axis): each mirror
+    // pair hi + lo is within 2^-48 X of x - origin, the period's pair within
+    // 2^-48 X, and the three additions of the small parts (at most 4 X 2^-24)
+    // round within 8 X 2^-48; the FP64 one rounds within 2^-53 of its absolute
+    // coordinates twice. The sum of both, doubled.
+    double O = 0.0;
+    for (int a = 0; a < 3; ++a) O = std::max(O, std::max(std::fabs(p.origin[a]), std::fabs(p.extent[a])));
+    d.image_tie_f = std::nextafter(
+        static_cast<float>(2.0 * (16.0 * X * std::ldexp(1.0, -48) + 4.0 * (O + X) * std::ldexp(1.0, -53))), 1.0f);
   }
   // FP32 cell index of the rebin: the mirror pf = fl32(x - origin) and
   // fl32(1/cell_size) put pf * inv within 3.01 u |q| of the quotient q of the

@@ -1,0 +1,252 @@
+// Mixed-precision Lennard-Jones forces over full lists, in two stages per block:
+// the form for batches too small to fill the GPU with one thread per particle.
+//
+// One thread walking a particle's list (k_force, xnb_step_kernels.cu) waits for
+// ~40 dependent rounds of gathers; below some 10^5 particles nothing hides that
+// latency. The values have to stay those of that walk, bit for bit: FP32 force
+// factors pd, and the sums of pd x_b, pd y_b, pd z_b, pd (and the energies) in
+// FP64, each added in list order.
+//   Stage 1 (FP32): a warp takes one particle at a time, 32 list entries per
+//     step: mirror gathers, r^2, the cutoff (FP64 inside the proven band) and
+//     pd; a ballot appends the pairs within rc to the particle's rows in shared
+//     memory, in list order: their FP64 coordinates (image applied) and pd.
+//   Stage 2 (FP64): a lane per (particle, sum) runs its sequential FMA chain
+//     over the rows, nothing but two shared loads and the FMA per term. A warp
+//     issues one FP64 instruction per 64 cycles whatever else it does, so 32
+//     chains share each.
+#include <algorithm>
+
+#include "xnb_launch.cuh"
+#include "xnb_lj_pair.cuh"
+#include "xnb_traverse.cuh"
+
+namespace xnb {
+
+namespace {
+
+// A particle of the block.
+struct Row {
+  float4 own;            // the particle's mirror
+  const uint32_t* list;
+  uint32_t n;            // list length, 0 for a slot that is not walked
+  uint32_t sys;          // kNone for such a slot
+  uint32_t count;        // pairs in the row (this chunk)
+  uint32_t pad;
+};
+constexpr uint32_t kNone = 0xFFFFFFFFu;
+
+// The packed residual fields as FP32 numbers (a 10-bit field, its sign bit
+// flipped, under the exponent of 2^23): differences are exact, q_b - q_a for x
+// and z, 1024 (q_b - q_a) for y.
+__device__ __forceinline__ float field_x(uint32_t w) { return __uint_as_float((w & 0x3FFu) ^ 0x4B000200u); }
+__device__ __forceinline__ float field_y(uint32_t w) { return __uint_as_float((w & 0xFFC00u) ^ 0x4B080000u); }
+__device__ __forceinline__ float field_z(uint32_t w) { return __uint_as_float((w >> 20) ^ 0x4B000200u); }
+
+// One axis of an image entry's displacement in FP32 pairs: hi_b - hi_a by
+// TwoDiff (Knuth), the image offset added to its high part (exact: the two are
+// within a factor of two of each other), the small parts summed. The rounded
+// sum is the FP64 displacement's FP32 rounding unless its remainder lies within
+// `tie` (the bound on both errors) of half an ulp: those entries take FP64.
+__device__ __forceinline__ float image_axis(float hb, float ha, float lb, float la, uint32_t digit, float p, float pl,
+                                            float tie, bool& sure) {
+  const float s = __fadd_rn(hb, -ha);
+  const float t = __fadd_rn(s, -hb);
+  const float err = __fadd_rn(__fadd_rn(hb, -__fadd_rn(s, -t)), -__fadd_rn(ha, t));
+  const float sh = digit == 1u ? 0.f : (digit == 2u ? p : -p), sl = digit == 1u ? 0.f : (digit == 2u ? pl : -pl);
+  const float hi = __fadd_rn(s, sh);
+  const float rest = __fadd_rn(__fadd_rn(err, sl), __fadd_rn(lb, -la));
+  const float d = __fadd_rn(hi, rest);
+  const float lo = __fadd_rn(__fadd_rn(hi, -d), rest);
+  const uint32_t ex = __float_as_uint(d) & 0x7f800000u;
+  const float half = __uint_as_float(ex - (24u << 23));  // half an ulp of d (ex checked below)
+  sure = sure && ex > (40u << 23) && fabsf(__fadd_rn(fabsf(lo), -half)) > tie &&
+         fabsf(__fadd_rn(fabsf(lo), -0.5f * half)) > tie;
+  return d;
+}
+
+template <bool PE, bool KICK>
+__global__ void __launch_bounds__(256, 4)
+    k_force_mixed(uint32_t n_part, BatchSource src, DevArrays a, uint32_t group, uint32_t chunk) {
+  constexpr uint32_t kSums = PE ? 5 : 4;   // x, y, z, pd and the energy
+  constexpr uint32_t kPer = 32 / kSums;    // particles per warp in stage 2
+  extern __shared__ __align__(16) unsigned char force_smem[];
+  const uint32_t lane = threadIdx.x & 31u, wib = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
+  const uint32_t stride = chunk + 1u;  // odd: the rows of a warp's lanes start on different banks
+  Row* const info = reinterpret_cast<Row*>(force_smem);
+  double* const rows = reinterpret_cast<double*>(info + group);  // per particle kSums rows: x, y, z, pd (, energy)
+  const uint32_t first = blockIdx.x * group;
+
+  uint32_t my_n = 0;
+  if (threadIdx.x < group) {
+    const uint32_t i = first + threadIdx.x;
+    uint32_t s = 0;
+    const uint32_t* list = nullptr;
+    const bool ok = i < n_part && src.locate(i, s, list, my_n);
+    if (!ok) my_n = 0;
+    Row r;
+    r.own = ok ? src.pf[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+    r.list = list;
+    r.n = my_n;
+    r.sys = ok ? s : kNone;
+    r.count = 0;
+    r.pad = 0;
+    info[threadIdx.x] = r;
+  }
+  __syncthreads();
+
+  // the warps that sum: group / kPer of them, from another one in each block
+  // (a warp's FP64 work runs on its own quarter of the SM)
+  const uint32_t turn = (wib + blockIdx.x) % nwarp;
+  const uint32_t row = turn * kPer + lane / kSums;
+  const uint32_t ax = lane % kSums;
+  const bool worker = lane < kPer * kSums && row < group && info[min(row, group - 1u)].sys != kNone;
+  double acc = 0.0;
+
+  for (uint32_t kb = 0;; kb += chunk) {
+    // ---- stage 1 ----
+    for (uint32_t p = wib; p < group; p += nwarp) {
+      const Row r = info[p];
+      uint32_t count = 0;
+      double* const out = rows + static_cast<size_t>(p) * kSums * stride;
+      if (r.n > kb) {
+        const uint32_t i = first + p;
+        const SysDesc& S = src.sys[r.sys];
+        const uint32_t pbase = S.part_base;
+        const float r2_in = S.rc2_f - S.rc_margin_f, r2_out = S.rc2_f + S.rc_margin_f, r2_min = S.rc_margin_f;
+        const float sig2 = S.sig2_f, eps24 = S.eps24_f, step = S.lo_step_f;
+        const uint32_t wa = __float_as_uint(r.own.w);
+        const float qx = field_x(wa), qy = field_y(wa), qz = field_z(wa);
+        const uint32_t* __restrict__ L = r.list;
+        const uint32_t self_e = ((i - pbase) << 5) | static_cast<uint32_t>(kImageCenter);
+        const uint32_t kend = min(r.n, kb + chunk);
+        uint32_t e = kb + lane < kend ? __ldg(L + kb + lane) : self_e;
+        for (uint32_t k0 = kb; k0 < kend; k0 += 32u) {
+          const uint32_t ent = e, code = ent & 31u;
+          const uint32_t j = pbase + (ent >> 5);
+          const float4 hb = __ldg(src.pf + j);
+          double xb = __ldg(src.rx + j), yb = __ldg(src.ry + j), zb = __ldg(src.rz + j);
+          e = k0 + 32u + lane < kend ? __ldg(L + k0 + 32u + lane) : self_e;
+          const bool valid = k0 + lane < kend;
+          const uint32_t wb = __float_as_uint(hb.w);
+          // within 2u|d| + 2 lo_step of the FP64 displacement (u = 2^-24)
+          float dx = fmaf(field_x(wb) - qx, step, hb.x - r.own.x);
+          float dy = fmaf(field_y(wb) - qy, step * 0.0009765625f, hb.y - r.own.y);
+          float dz = fmaf(field_z(wb) - qz, step, hb.z - r.own.z);
+          if (code != static_cast<uint32_t>(kImageCenter)) {
+            const float4 lb = __ldg(src.pflo + j), la = __ldg(src.pflo + i);
+            const uint32_t cx = code % 3u, cy = (code / 3u) % 3u, cz = code / 9u;
+            const float tie = S.image_tie_f;
+            bool sure = true;
+            dx = image_axis(hb.x, r.own.x, lb.x, la.x, cx, S.period_f[0], S.period_lo_f[0], tie, sure);
+            dy = image_axis(hb.y, r.own.y, lb.y, la.y, cy, S.period_f[1], S.period_lo_f[1], tie, sure);
+            dz = image_axis(hb.z, r.own.z, lb.z, la.z, cz, S.period_f[2], S.period_lo_f[2], tie, sure);
+            // image_coord: x + (+-1.0 * period)
+            if (cx != 1u) xb = __dadd_rn(xb, cx == 2u ? S.period[0] : -S.period[0]);
+            if (cy != 1u) yb = __dadd_rn(yb, cy == 2u ? S.period[1] : -S.period[1]);
+            if (cz != 1u) zb = __dadd_rn(zb, cz == 2u ? S.period[2] : -S.period[2]);
+            if (!sure) {
+              dx = narrow_f64(__dsub_rn(xb, src.rx[i]));
+              dy = narrow_f64(__dsub_rn(yb, src.ry[i]));
+              dz = narrow_f64(__dsub_rn(zb, src.rz[i]));
+            }
+          }
+          const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+          bool in = valid && r2 < r2_in && r2 > r2_min;
+          if (valid && !in && !(r2 > r2_out)) {
+            // inside the FP32 band: the FP64 decision
+            const double d2 = norm2_rn(__dsub_rn(xb, src.rx[i]), __dsub_rn(yb, src.ry[i]), __dsub_rn(zb, src.rz[i]));
+            in = d2 > 0.0 && d2 <= S.rcut2;
+          }
+          const unsigned m = __ballot_sync(0xffffffffu, in);
+          if (in) {
+            // the hardware reciprocal (within 1 ulp) is part of the FP32 force magnitude
+            float ir2;
+            asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(ir2) : "f"(r2));
+            const float s2 = sig2 * ir2;
+            const float s6 = s2 * s2 * s2;
+            const float pd = eps24 * s6 * fmaf(-2.0f, s6, 1.0f) * ir2;
+            double* const o = out + count + __popc(m & ((1u << lane) - 1u));
+            o[0] = xb;
+            o[stride] = yb;
+            o[2u * stride] = zb;
+            o[3u * stride] = widen_f32_fast(pd);
+            if (PE) o[4u * stride] = widen_f32_fast(0.5f * fmaf(S.eps4_f * s6, s6 - 1.0f, -S.e_shift_f));
+          }
+          count += __popc(m);
+        }
+        // zero terms up to a multiple of four pairs
+        if (lane < ((0u - count) & 3u)) {
+#pragma unroll
+          for (uint32_t t = 0; t < kSums; ++t) out[t * stride + count + lane] = 0.0;
+        }
+      }
+      if (lane == 0) info[p].count = count;
+    }
+    __syncthreads();
+    // ---- stage 2 ----
+    if (worker) {
+      const uint32_t count = (info[row].count + 3u) & ~3u;
+      const double* const mine = rows + (static_cast<size_t>(row) * kSums + ax) * stride;
+      const double* const factor = rows + (static_cast<size_t>(row) * kSums + 3u) * stride;
+      const bool axis = ax < 3u;  // a coordinate times pd; pd and the energy are summed as they are
+      for (uint32_t k = 0; k < count; k += 4u) {
+        double x[4], f[4];
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+          x[t] = mine[k + t];
+          f[t] = axis ? factor[k + t] : 1.0;
+        }
+#pragma unroll
+        for (int t = 0; t < 4; ++t) acc = fma(f[t], x[t], acc);
+      }
+    }
+    if (!__syncthreads_or(my_n > kb + chunk)) break;
+  }
+
+  // ---- the particle's sums ----
+  const double psum = __shfl_sync(0xffffffffu, acc, lane - ax + 3u);
+  if (!worker || ax == 3u) return;
+  const SysDesc& S = src.sys[info[row].sys];
+  const uint32_t i = first + row;
+  if (PE && ax == 4u) {
+    a.pe[i] = acc;
+    return;
+  }
+  // the FP64 displacement folded out of the sum: sum pd (r_b - r_a)
+  double f = fma(-(ax == 0u ? src.rx : (ax == 1u ? src.ry : src.rz))[i], psum, acc);
+  if (S.divide_by_mass) f = __ddiv_rn(f, S.mass);
+  (ax == 0u ? a.fx : (ax == 1u ? a.fy : a.fz))[i] = f;
+  if (KICK) {
+    double* const v = ax == 0u ? a.vx : (ax == 1u ? a.vy : a.vz);
+    v[i] = fma(f, S.dt_half, v[i]);
+  }
+}
+
+template <bool PE, bool KICK>
+void go(const Extent& ex, const SysDesc* sys, const SysState* st, const DevArrays& a, int sys_only,
+        cudaStream_t stream) {
+  constexpr uint32_t sums = PE ? 5 : 4, group = 32u / sums;
+  const BatchSource src(sys, st, a, sys_only);
+  // list entries per chunk: a multiple of 32 that the usual lists fit
+  const uint32_t chunk = std::min(std::max((ex.list_slot * 2u / 3u + 31u) / 32u * 32u, 32u), 256u);
+  const size_t smem = group * (sizeof(Row) + static_cast<size_t>(chunk + 1u) * sums * sizeof(double));
+  const unsigned grid = (ex.n_part + group - 1u) / group;
+  // stage 1: a warp per particle while every block has an SM of its own, then
+  // two particles per warp (32,000 atoms: 43 us with 128 threads, 61 us with 256)
+  const unsigned threads = grid <= static_cast<unsigned>(ex.sm_count) ? group * 32u : group * 16u;
+  cudaFuncSetAttribute(k_force_mixed<PE, KICK>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+  k_force_mixed<PE, KICK><<<grid, threads, smem, stream>>>(ex.n_part, src, a, group, chunk);
+}
+
+}  // namespace
+
+int launch_force_mixed(const Extent& ex, const SysDesc* sys, const SysState* st, const DevArrays& a, bool with_pe,
+                       bool second_half, int sys_only, cudaStream_t stream) {
+  if (with_pe && second_half) go<true, true>(ex, sys, st, a, sys_only, stream);
+  else if (with_pe) go<true, false>(ex, sys, st, a, sys_only, stream);
+  else if (second_half) go<false, true>(ex, sys, st, a, sys_only, stream);
+  else go<false, false>(ex, sys, st, a, sys_only, stream);
+  return 1;
+}
+
+}  // namespace xnb

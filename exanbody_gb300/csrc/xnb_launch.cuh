@@ -20,6 +20,7 @@ struct Extent {
   int force_lanes;   // threads per particle of the FP64 / mixed full-list traversal (1, 2 or 4)
   int far_coords;    // some resident system lies far from the coordinate origin (SysDesc::far_coords)
   int unpacked;      // some resident system reads the residual mirror, not packed residuals (SysDesc::packed_lo)
+  uint32_t list_slot;  // largest list slot of the resident systems
   int force_form;    // kForceThread or kForceStaged (mixed full-list traversal)
   uint32_t n_seg;    // cell segments of the staged traversal (DevArrays::seg)
 };
@@ -42,6 +43,14 @@ int launch_first_half(const Extent& ex, const SysDesc* sys, SysState* st, const 
 // reactions with FP64 reductions (three kernels: zero, traverse, finish).
 int launch_force(const Extent& ex, const SysDesc* sys, SysState* st, const DevArrays& a, int precision,
                  bool with_pe, bool second_half, int sys_only, cudaStream_t stream, bool newton = false);
+
+// The mixed full-list forces in the two-stage form (xnb_force_mixed.cu): the same
+// bits as one thread per particle, faster while the particles are too few to fill
+// the GPU that way. Per call, two-stage / one-thread: 864 atoms 10 / 87 us, 32,000
+// 43 / 96 us, 62,500 72 / 105 us, 131,072 135 / 137 us (178 / 165 us with energies).
+constexpr uint32_t kMixedSplitMax = 100000;
+int launch_force_mixed(const Extent& ex, const SysDesc* sys, const SysState* st, const DevArrays& a, bool with_pe,
+                       bool second_half, int sys_only, cudaStream_t stream);
 
 // Compact list entries of the flagged systems after a build, and the staged
 // mixed force traversal (+ kick) over the cell segments (xnb_force_staged.cu).

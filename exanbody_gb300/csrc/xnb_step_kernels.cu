@@ -600,6 +600,8 @@ int launch_force(const Extent& ex, const SysDesc* sys, SysState* st, const DevAr
   }
   if (precision == kMixed && ex.force_form == kForceStaged && a.nbr16 && a.seg && !ex.unpacked)
     return launch_force_staged(ex, sys, st, a, with_pe, second_half, sys_only, stream);
+  if (precision == kMixed && !ex.unpacked && ex.n_part <= kMixedSplitMax)
+    return launch_force_mixed(ex, sys, st, a, with_pe, second_half, sys_only, stream);
 #define XNB_FORCE_CASE(PP)                                                           \
   if (precision == PP) {                                                             \
     if (with_pe && second_half) force_dispatch<PP, true, true>(ex, sys, st, a, sys_only, stream);   \

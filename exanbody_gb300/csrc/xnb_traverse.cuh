@@ -36,6 +36,19 @@ struct BatchSource {
         cell_sys(a.cell_sys), nbr(a.nbr), nbr_start(a.nbr_start), nbr_cnt(a.nbr_cnt), nbr_half(a.nbr_half),
         sys_only(sys_only_) {}
 
+  // Particle i's system and list; false for slots that are not walked.
+  __device__ __forceinline__ bool locate(uint32_t i, uint32_t& s, const uint32_t*& list, uint32_t& n) const {
+    const uint32_t cl = pcell[i];
+    if (cl == 0xFFFFFFFFu) return false;
+    const uint32_t q = cell_sys[cl];
+    if (sys_only >= 0 && q != static_cast<uint32_t>(sys_only)) return false;
+    if (st[q].error) return false;  // lists of a failed system are not trusted
+    s = q;
+    list = nbr + sys[q].list_base + nbr_start[i];
+    n = nbr_cnt[i];
+    return true;
+  }
+
   __device__ __forceinline__ bool begin(uint32_t i, bool symmetric, bool want_lo, pair::ParticleContext& c) const {
     const uint32_t cl = pcell[i];
     if (cl == 0xFFFFFFFFu) return false;
