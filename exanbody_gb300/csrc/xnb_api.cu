@@ -560,6 +560,7 @@ int xnb_batch_create(const xnb_batch_config* cfg, xnb_batch** out) {
   rc = rc ? rc : dalloc(b, &a.rbf, P);
   rc = rc ? rc : dalloc(b, &a.nbr_half, P);
   rc = rc ? rc : dalloc(b, &a.any_rebuild, 4);
+  rc = rc ? rc : dalloc(b, &a.grid_ctl, 1);
   rc = rc ? rc : dalloc(b, &a.t_id, P);
   rc = rc ? rc : dalloc(b, &a.ptype, P);
   rc = rc ? rc : dalloc(b, &a.t_ptype, P);
@@ -595,6 +596,7 @@ int xnb_batch_create(const xnb_batch_config* cfg, xnb_batch** out) {
   cudaMemset(a.cell_start, 0, (Cc + 1) * sizeof(uint32_t));
   cudaMemset(b->d_st, 0, sizeof(SysState) * cfg->max_systems);
   cudaMemset(a.any_rebuild, 0, sizeof(unsigned int));
+  cudaMemset(a.grid_ctl, 0, sizeof(GridBarrier));
   cudaMemset(a.nbr_wide_n, 0, sizeof(unsigned int));
   cudaMemset(a.nbr_sub_n, 0, sizeof(unsigned int));
   cudaMemset(a.cside, 1, Cc + 1);
@@ -1111,9 +1113,17 @@ int xnb_step(xnb_batch* b, int32_t nsteps, int32_t precision, int32_t flags, voi
   const Extent ex = b->extent();
   const bool exact = precision == XNB_PREC_FP64_EXACT;
   const bool energy = (flags & XNB_STEP_ENERGY) != 0;
+  const bool fused = !(flags & XNB_STEP_HOST_SYNC) && fused_rebin_fits(ex);
   for (int k = 0; k < nsteps; ++k) {
     // verlet_first_half + trigger_move_particles
     b->launches += launch_first_half(ex, b->d_sys, b->d_st, b->a, true, true, true, 1.0, 0.5, exact, -1, st);
+    if (fused) {
+      b->launches += launch_rebin_fused(ex, b->d_sys, b->d_st, b->a, exact, st);
+      b->launches += launch_neighbors(ex, b->d_sys, b->d_st, b->a, b->stage_cap, list_buf(b), st, b->build_form,
+                                      b->subcell_prune != 0, false);
+      b->launches += launch_force(ex, b->d_sys, b->d_st, b->a, precision, energy, true, -1, st, newton);
+      continue;
+    }
     b->launches += launch_mark_rebuild(ex, b->d_st, 1, -1, b->a.any_rebuild, st);
     bool rebuild = true;
     if (flags & XNB_STEP_HOST_SYNC) {
@@ -1167,7 +1177,7 @@ int xnb_step_persistent(xnb_batch* b, int32_t nsteps, int32_t precision, int32_t
     StepCtl h{};
     XCK(cudaMemcpyAsync(&h, b->d_ctl, sizeof(StepCtl), cudaMemcpyDeviceToHost, st));
     XCK(cudaStreamSynchronize(st));
-    if (h.error) return fail(XNB_ERR_DEVICE, "a grid barrier of the persistent step loop ran out of time");
+    if (h.bar.error) return fail(XNB_ERR_DEVICE, "a grid barrier of the persistent step loop ran out of time");
     if (check) return fail(XNB_ERR_ARG, "the barrier check did not run out");
     remaining -= static_cast<int>(h.steps_done);
     if (h.stopped) {

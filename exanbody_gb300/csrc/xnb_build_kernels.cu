@@ -1,6 +1,9 @@
 // Rebuild-path kernels: move/rebin with periodic wrap, AMR in-cell ordering,
 // backup_r, and the cell-grid neighbour build; plus the device scan they use.
+#include <algorithm>
+
 #include "xnb_build_common.cuh"
+#include "xnb_grid_barrier.cuh"
 #include "xnb_launch.cuh"
 
 namespace xnb {
@@ -29,9 +32,8 @@ __device__ __forceinline__ int sub_grid_side(uint32_t n, double density) {
 // move_particles_across_cells.h:115-152): dst = domain_periodic_location(r)
 // (core/include/exanb/core/domain.h:160-191, wrapping r by whole cells), and the
 // particle leaves its cell when dst differs or it lies >= epsilon outside dst's bounds.
-__global__ void __launch_bounds__(256)
-    k_rebin_dest(uint32_t n_part, const SysDesc* __restrict__ sys, SysState* st, DevArrays a) {
-  if (*a.any_rebuild == 0) return;
+__device__ __forceinline__ void rebin_dest(uint32_t n_part, const SysDesc* __restrict__ sys, SysState* st,
+                                           const DevArrays& a) {
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n_part; i += gridDim.x * blockDim.x) {
     const uint32_t c = a.pcell[i];
     if (c == kInvalid) continue;
@@ -121,15 +123,18 @@ __global__ void __launch_bounds__(256)
     a.pdest[i] = mover ? (dst | kMoverBit) : c;
   }
 }
+__global__ void __launch_bounds__(256)
+    k_rebin_dest(uint32_t n_part, const SysDesc* __restrict__ sys, SysState* st, DevArrays a) {
+  if (*a.any_rebuild == 0) return;
+  rebin_dest(n_part, sys, st, a);
+}
 
 // ---------------------------------------------------------------------------
 // K_r2: per source cell, compaction of the staying particles and list of movers.
 // The hole left by a mover is filled with the current last particle, scanning
 // from the top (move_particles_across_cells.h:186-207).
-__global__ void __launch_bounds__(128)
-    k_rebin_compact(uint32_t n_cells, const SysDesc* __restrict__ sys, const SysState* __restrict__ st,
-                    DevArrays a) {
-  if (*a.any_rebuild == 0) return;
+__device__ __forceinline__ void rebin_compact(uint32_t n_cells, const SysDesc* __restrict__ sys, const SysState* st,
+                                              const DevArrays& a) {
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t warps = gridDim.x * (blockDim.x >> 5);
   for (uint32_t c = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); c < n_cells; c += warps) {
@@ -160,6 +165,11 @@ __global__ void __launch_bounds__(128)
       a.cell_nmov[c] = nmov;
     }
   }
+}
+__global__ void __launch_bounds__(128)
+    k_rebin_compact(uint32_t n_cells, const SysDesc* __restrict__ sys, const SysState* st, DevArrays a) {
+  if (*a.any_rebuild == 0) return;
+  rebin_compact(n_cells, sys, st, a);
 }
 
 // The (up to) 27 source cells around destination cell c, sorted by global cell
@@ -212,9 +222,8 @@ __device__ __forceinline__ SrcInfo arrivals_of(const SysDesc& S, const DevArrays
 }
 
 // K_r3: new particle count of every cell (flagged systems: stayers + arrivals).
-__global__ void __launch_bounds__(128)
-    k_rebin_count(uint32_t n_cells, const SysDesc* __restrict__ sys, const SysState* __restrict__ st, DevArrays a) {
-  if (*a.any_rebuild == 0) return;
+__device__ __forceinline__ void rebin_count(uint32_t n_cells, const SysDesc* __restrict__ sys, const SysState* st,
+                                            const DevArrays& a) {
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t warps = gridDim.x * (blockDim.x >> 5);
   for (uint32_t c = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); c < n_cells; c += warps) {
@@ -233,12 +242,15 @@ __global__ void __launch_bounds__(128)
     if (lane == 0) a.cell_cnt[c] = a.cell_stay[c] + tot;
   }
 }
+__global__ void __launch_bounds__(128)
+    k_rebin_count(uint32_t n_cells, const SysDesc* __restrict__ sys, const SysState* st, DevArrays a) {
+  if (*a.any_rebuild == 0) return;
+  rebin_count(n_cells, sys, st, a);
+}
 
 // K_r5: gather stayers then arrivals of each destination cell into the scratch arrays.
-__global__ void __launch_bounds__(128)
-    k_rebin_scatter(uint32_t n_cells, const SysDesc* __restrict__ sys, const SysState* __restrict__ st,
-                    DevArrays a) {
-  if (*a.any_rebuild == 0) return;
+__device__ __forceinline__ void rebin_scatter(uint32_t n_cells, const SysDesc* __restrict__ sys, const SysState* st,
+                                              const DevArrays& a) {
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t warps = gridDim.x * (blockDim.x >> 5);
   for (uint32_t c = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); c < n_cells; c += warps) {
@@ -275,13 +287,42 @@ __global__ void __launch_bounds__(128)
     }
   }
 }
+__global__ void __launch_bounds__(128)
+    k_rebin_scatter(uint32_t n_cells, const SysDesc* __restrict__ sys, const SysState* st, DevArrays a) {
+  if (*a.any_rebuild == 0) return;
+  rebin_scatter(n_cells, sys, st, a);
+}
+
+// backup_r of one particle (io/backup_r.cpp:56-79): its 32-bit encoding relative
+// to the cell, and what that restores to. The FP64 and mixed step loops keep the
+// position itself instead: their displacement trigger then differs from the
+// reference's by the encoding's quantum (cell_size / 2^32) at most.
+__device__ __forceinline__ void store_backup(const SysDesc& S, const DevArrays& a, uint32_t i, const double (&lo)[3],
+                                             double x, double y, double z) {
+  const uint32_t bx = encode_u32(x, lo[0], S.cell_size, S.inv_cell);
+  const uint32_t by = encode_u32(y, lo[1], S.cell_size, S.inv_cell);
+  const uint32_t bz = encode_u32(z, lo[2], S.cell_size, S.inv_cell);
+  a.bkx[i] = bx;
+  a.bky[i] = by;
+  a.bkz[i] = bz;
+  const double rx = restore_u32(bx, lo[0], S.cell_size);
+  const double ry = restore_u32(by, lo[1], S.cell_size);
+  const double rz = restore_u32(bz, lo[2], S.cell_size);
+  a.rbx[i] = rx;
+  a.rby[i] = ry;
+  a.rbz[i] = rz;
+  a.rbf[i] = make_pf(S, rx, ry, rz);
+}
 
 // K_r6: final in-cell order (rebuild_amr's stable sort by sub-cell,
 // amr_grid_algorithm.h:131-374, when the cell is dense enough for a sub-grid),
-// cell table update, and backup_r (io/backup_r.cpp:56-79).
-__global__ void __launch_bounds__(128)
-    k_rebin_finalize(uint32_t n_cells, const SysDesc* __restrict__ sys, SysState* st, DevArrays a) {
-  if (*a.any_rebuild == 0) return;
+// cell table update, and backup_r (io/backup_r.cpp:56-79): kBackupExact keeps
+// the encoding (store_backup), kBackupPlain the position itself, both while the
+// position is in registers.
+constexpr int kBackupExact = 1, kBackupPlain = 2;
+template <int BACKUP>
+__device__ __forceinline__ void rebin_finalize(uint32_t n_cells, const SysDesc* __restrict__ sys, SysState* st,
+                                               const DevArrays& a) {
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t warps = gridDim.x * (blockDim.x >> 5);
   for (uint32_t c = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); c < n_cells; c += warps) {
@@ -294,11 +335,15 @@ __global__ void __launch_bounds__(128)
     // the FP64 division of sub_grid_side only for counts that can give a side > 1
     // (a warp-wide FP64 instruction costs the same for one lane as for 32)
     const int side = (S.amr_enabled && n >= S.amr_min_n) ? sub_grid_side(n, S.sub_grid_density) : 1;
-    // backup_r runs afterwards in k_backup, one thread per particle
     if (lane == 0) a.cside[c] = static_cast<uint8_t>(side);
-    if (side > 1) {
+    double lo[3];
+    if (side > 1 || BACKUP == kBackupExact) {
       cell_ijk(S, c - S.cell_base, ci, cj, ck);
-      const double lo[3] = {cell_lo(S, 0, ci), cell_lo(S, 1, cj), cell_lo(S, 2, ck)};
+      lo[0] = cell_lo(S, 0, ci);
+      lo[1] = cell_lo(S, 1, cj);
+      lo[2] = cell_lo(S, 2, ck);
+    }
+    if (side > 1) {
       // sub-cell key of each particle (Grid::particle_pcoord, grid.h:184-190), kept in pdest
       for (uint32_t q = lane; q < n; q += 32) {
         const double r[3] = {a.t_rx[ns + q], a.t_ry[ns + q], a.t_rz[ns + q]};
@@ -338,6 +383,14 @@ __global__ void __launch_bounds__(128)
       make_pf2(S, x, y, z, mhi, mlo);
       a.pf[dst] = mhi;
       a.pflo[dst] = mlo;
+      if constexpr (BACKUP == kBackupExact) {
+        store_backup(S, a, dst, lo, x, y, z);
+      } else {
+        a.rbx[dst] = x;
+        a.rby[dst] = y;
+        a.rbz[dst] = z;
+        a.rbf[dst] = make_float4(mhi.x, mhi.y, mhi.z, 0.f);
+      }
       a.pcell[dst] = c;
       if (side > 1) a.skey[dst] = static_cast<uint16_t>(a.pdest[src]);
     }
@@ -348,26 +401,17 @@ __global__ void __launch_bounds__(128)
     }
   }
 }
+template <int BACKUP>
+__global__ void __launch_bounds__(128)
+    k_rebin_finalize(uint32_t n_cells, const SysDesc* __restrict__ sys, SysState* st, DevArrays a) {
+  if (*a.any_rebuild == 0) return;
+  rebin_finalize<BACKUP>(n_cells, sys, st, a);
+}
 
-// backup_r alone (io/backup_r.cpp:42-79) for flagged systems. EXACT = false
-// (the FP64 and mixed paths) keeps the backup position itself instead of its
-// 32-bit cell-relative encoding: the displacement trigger then differs from the
-// reference's by the encoding's quantum (cell_size / 2^32) at most.
-template <bool EXACT>
+// backup_r alone (io/backup_r.cpp:42-79) for flagged systems.
 __global__ void __launch_bounds__(256)
     k_backup(uint32_t n_part, const SysDesc* __restrict__ sys, SysState* st, DevArrays a) {
   if (*a.any_rebuild == 0) return;
-  if constexpr (!EXACT) {
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n_part; i += gridDim.x * blockDim.x) {
-      const uint32_t c = a.pcell[i];
-      if (c == kInvalid || !sys_flagged(st, a.cell_sys[c])) continue;
-      const double x = a.rx[i], y = a.ry[i], z = a.rz[i];
-      a.rbx[i] = x;
-      a.rby[i] = y;
-      a.rbz[i] = z;
-      a.rbf[i] = make_pf(sys[a.cell_sys[c]], x, y, z);
-    }
-  } else {
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n_part; i += gridDim.x * blockDim.x) {
     const uint32_t c = a.pcell[i];
     if (c == kInvalid) continue;
@@ -377,15 +421,7 @@ __global__ void __launch_bounds__(256)
     int ci, cj, ck;
     cell_ijk(S, c - S.cell_base, ci, cj, ck);
     const double lo[3] = {cell_lo(S, 0, ci), cell_lo(S, 1, cj), cell_lo(S, 2, ck)};
-    const uint32_t bx = encode_u32(a.rx[i], lo[0], S.cell_size, S.inv_cell);
-    const uint32_t by = encode_u32(a.ry[i], lo[1], S.cell_size, S.inv_cell);
-    const uint32_t bz = encode_u32(a.rz[i], lo[2], S.cell_size, S.inv_cell);
-    a.bkx[i] = bx; a.bky[i] = by; a.bkz[i] = bz;
-    a.rbx[i] = restore_u32(bx, lo[0], S.cell_size);
-    a.rby[i] = restore_u32(by, lo[1], S.cell_size);
-    a.rbz[i] = restore_u32(bz, lo[2], S.cell_size);
-    a.rbf[i] = make_pf(S, a.rbx[i], a.rby[i], a.rbz[i]);
-  }
+    store_backup(S, a, i, lo, a.rx[i], a.ry[i], a.rz[i]);
   }
 }
 
@@ -397,6 +433,122 @@ __global__ void k_arm(int nsys, SysState* st, const unsigned int* any, bool rebi
   if (s < nsys && st[s].rebuild) {
     st[s].rebuild_armed = 1;
     if (rebinned) st[s].keys_fresh = 1;
+  }
+}
+
+// Exclusive scan of one batch's cell counts by one block (the fused rebin).
+__device__ __forceinline__ void scan_cells_one_block(const uint32_t* in, uint32_t n, unsigned long long* out) {
+  constexpr uint32_t kItems = 8;
+  __shared__ unsigned long long wsum[32];
+  __shared__ unsigned long long carry;
+  const uint32_t lane = threadIdx.x & 31u, wib = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
+  if (threadIdx.x == 0) carry = 0;
+  for (uint32_t b0 = 0; b0 < n; b0 += blockDim.x * kItems) {
+    const uint32_t base = b0 + threadIdx.x * kItems;
+    uint32_t v[kItems];
+    unsigned long long t = 0;
+#pragma unroll
+    for (uint32_t k = 0; k < kItems; ++k) {
+      v[k] = base + k < n ? in[base + k] : 0u;
+      t += v[k];
+    }
+    unsigned long long inc = t;
+    for (int off = 1; off < 32; off <<= 1) {
+      const unsigned long long y = __shfl_up_sync(0xffffffffu, inc, off);
+      if (lane >= static_cast<uint32_t>(off)) inc += y;
+    }
+    if (lane == 31u) wsum[wib] = inc;
+    __syncthreads();
+    unsigned long long run = carry + inc - t;
+    for (uint32_t q = 0; q < wib; ++q) run += wsum[q];
+    unsigned long long tot = 0;
+    for (uint32_t q = 0; q < nwarp; ++q) tot += wsum[q];
+#pragma unroll
+    for (uint32_t k = 0; k < kItems; ++k) {
+      if (base + k < n) out[base + k] = run;
+      run += v[k];
+      if (base + k + 1u == n) out[n] = run;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) carry += tot;
+    __syncthreads();
+  }
+}
+
+// The trigger's decision and the whole rebin (K_r1 .. K_r6, the resets of the
+// build that follows) of a small batch in one cooperative launch. A step without
+// a rebuild costs one launch that returns at once, where the separate kernels
+// cost twelve (0.7 us each inside a graph, 2.3 us when launched one by one); a
+// rebuild costs six grid barriers. The phases are the separate kernels' bodies.
+template <int BACKUP>
+__global__ void __launch_bounds__(256)
+    k_rebin_fused(uint32_t n_part, uint32_t n_cells, int nsys, const SysDesc* __restrict__ sys, SysState* st,
+                  DevArrays a) {
+  int flagged = 0;
+  for (int s = static_cast<int>(threadIdx.x); s < nsys; s += static_cast<int>(blockDim.x))
+    flagged |= __ldcg(&st[s].moved) != 0ull ? 1 : 0;
+  if (!__syncthreads_or(flagged)) {
+    if (blockIdx.x == 0) {
+      for (int s = static_cast<int>(threadIdx.x); s < nsys; s += static_cast<int>(blockDim.x)) st[s].rebuild = 0;
+      if (threadIdx.x == 0) *a.any_rebuild = 0;
+    }
+    return;
+  }
+  if (blockIdx.x == 0) {
+    // what the other blocks read before the first barrier is `moved` alone
+    unsigned int mine = 0;
+    for (int s = static_cast<int>(threadIdx.x); s < nsys; s += static_cast<int>(blockDim.x)) {
+      const bool r = __ldcg(&st[s].moved) != 0ull;
+      st[s].rebuild = r ? 1u : 0u;
+      if (!r) continue;
+      ++mine;
+      st[s].rebuilds += 1;
+      st[s].rebuild_armed = 1;
+      st[s].keys_fresh = 1;
+      // the build that follows (k_nbr_reset)
+      st[s].list_used = 0;
+      st[s].max_nbr = 0;
+      st[s].lists_fresh = 1;
+      st[s].compact_bad = 0;
+      st[s].half_bad = 0;
+    }
+    if (threadIdx.x == 0) {
+      *a.any_rebuild = 0;
+      *a.nbr_wide_n = 0;
+      *a.nbr_sub_n = 0;
+    }
+    __syncthreads();
+    if (mine) atomicAdd(a.any_rebuild, mine);
+  }
+  bool ok = grid_barrier(a.grid_ctl, gridDim.x);
+  if (ok) {
+    if (blockIdx.x == 0)
+      for (int s = static_cast<int>(threadIdx.x); s < nsys; s += static_cast<int>(blockDim.x)) st[s].moved = 0;
+    rebin_dest(n_part, sys, st, a);
+    ok = grid_barrier(a.grid_ctl, gridDim.x);
+  }
+  if (ok) {
+    rebin_compact(n_cells, sys, st, a);
+    ok = grid_barrier(a.grid_ctl, gridDim.x);
+  }
+  if (ok) {
+    rebin_count(n_cells, sys, st, a);
+    ok = grid_barrier(a.grid_ctl, gridDim.x);
+  }
+  if (ok) {
+    if (blockIdx.x == 0) scan_cells_one_block(a.cell_cnt, n_cells, a.cell_scan);
+    ok = grid_barrier(a.grid_ctl, gridDim.x);
+  }
+  if (ok) {
+    rebin_scatter(n_cells, sys, st, a);
+    ok = grid_barrier(a.grid_ctl, gridDim.x);
+  }
+  if (ok) {
+    rebin_finalize<BACKUP>(n_cells, sys, st, a);
+  } else if (threadIdx.x == 0) {
+    // a barrier ran out of time: the systems being rebuilt stop
+    for (int s = 0; s < nsys; ++s)
+      if (__ldcg(&st[s].rebuild)) atomicOr(&st[s].error, kErrBarrier);
   }
 }
 
@@ -979,22 +1131,43 @@ int launch_rebin(const Extent& ex, const SysDesc* sys, SysState* st, const DevAr
   k_rebin_count<<<wg, 128, 0, stream>>>(ex.n_cells, sys, st, a);
   const int ns = launch_scan_u32_to_u64(a.cell_cnt, a.cell_scan, ex.n_cells, a.scan_blocks, stream, a.any_rebuild);
   k_rebin_scatter<<<wg, 128, 0, stream>>>(ex.n_cells, sys, st, a);
-  k_rebin_finalize<<<wg, 128, 0, stream>>>(ex.n_cells, sys, st, a);
-  if (exact_backup) k_backup<true><<<thread_grid(ex.n_part, 256, ex.sm_count), 256, 0, stream>>>(ex.n_part, sys, st, a);
-  else k_backup<false><<<thread_grid(ex.n_part, 256, ex.sm_count), 256, 0, stream>>>(ex.n_part, sys, st, a);
+  if (exact_backup) k_rebin_finalize<kBackupExact><<<wg, 128, 0, stream>>>(ex.n_cells, sys, st, a);
+  else k_rebin_finalize<kBackupPlain><<<wg, 128, 0, stream>>>(ex.n_cells, sys, st, a);
   k_arm<<<(ex.nsys + 127) / 128, 128, 0, stream>>>(ex.nsys, st, a.any_rebuild, true);
-  return 7 + ns;
+  return 6 + ns;
+}
+
+bool fused_rebin_fits(const Extent& ex) {
+  return ex.n_part > 0 && ex.n_part <= kFusedRebinMaxParticles && ex.n_cells > 0 && ex.n_cells <= kFusedRebinMaxCells;
+}
+
+int launch_rebin_fused(const Extent& ex, const SysDesc* sys, SysState* st, const DevArrays& a, bool exact_backup,
+                       cudaStream_t stream) {
+  // a warp per cell, at most one block per SM: always co-resident
+  const unsigned grid = std::min((ex.n_cells + 7u) / 8u, static_cast<unsigned>(ex.sm_count));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(256);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, exact_backup ? k_rebin_fused<kBackupExact> : k_rebin_fused<kBackupPlain>, ex.n_part,
+                     ex.n_cells, ex.nsys, sys, st, a);
+  return 1;
 }
 
 int launch_backup(const Extent& ex, const SysDesc* sys, SysState* st, const DevArrays& a, cudaStream_t stream) {
   if (ex.n_part == 0) return 0;
-  k_backup<true><<<thread_grid(ex.n_part, 256, ex.sm_count), 256, 0, stream>>>(ex.n_part, sys, st, a);
+  k_backup<<<thread_grid(ex.n_part, 256, ex.sm_count), 256, 0, stream>>>(ex.n_part, sys, st, a);
   k_arm<<<(ex.nsys + 127) / 128, 128, 0, stream>>>(ex.nsys, st, a.any_rebuild, false);
   return 2;
 }
 
 int launch_neighbors(const Extent& ex, const SysDesc* sys, SysState* st, const DevArrays& a, int cap, int lbuf,
-                     cudaStream_t stream, int form, bool prune) {
+                     cudaStream_t stream, int form, bool prune, bool reset) {
   if (ex.n_cells == 0) return 0;
   const size_t smem = static_cast<size_t>(cap) * sizeof(float4) + static_cast<size_t>(4) * 2 * lbuf * sizeof(uint32_t);
   // warp-per-cell form: the stage alone (hits go straight to the slots)
@@ -1007,7 +1180,7 @@ int launch_neighbors(const Extent& ex, const SysDesc* sys, SysState* st, const D
     per_sm = 1;
   const long long want_w = (static_cast<long long>(ex.n_cells) + 3) / 4;
   const int grid_w = static_cast<int>(std::max(1ll, std::min(want_w, static_cast<long long>(per_sm) * ex.sm_count)));
-  k_nbr_reset<<<(ex.nsys + 127) / 128, 128, 0, stream>>>(ex.nsys, st, a.any_rebuild, a.nbr_wide_n, a.nbr_sub_n);
+  if (reset) k_nbr_reset<<<(ex.nsys + 127) / 128, 128, 0, stream>>>(ex.nsys, st, a.any_rebuild, a.nbr_wide_n, a.nbr_sub_n);
   // half-shell form: masks first; systems it cannot take go through the warp-per-cell build
   const bool half = form == kBuildHalf && a.nmask != nullptr;
   const int nh = half ? launch_neighbors_half_test(ex, sys, st, a, stream) : 0;
@@ -1019,7 +1192,7 @@ int launch_neighbors(const Extent& ex, const SysDesc* sys, SysState* st, const D
   k_neighbors<<<warp_grid(ex.n_cells, 1, ex.sm_count), 128, smem, stream>>>(ex.n_cells, sys, st, a, cap, lbuf);
   // compact entries for the staged force traversal
   const int nc = ex.force_form == kForceStaged ? launch_compact_lists(ex, sys, st, a, stream) : 0;
-  return 3 + nh + ne + nsub + nc;
+  return 2 + (reset ? 1 : 0) + nh + ne + nsub + nc;
 }
 
 }  // namespace xnb

@@ -35,6 +35,15 @@ enum ErrorBits : uint32_t {
   kErrFarMover = 1u << 1,       // a particle moved further than one cell between rebuilds
   kErrCellIndex = 1u << 2,      // a particle outside the periodic domain grid
   kErrStage = 1u << 3,          // staging capacity exceeded (programming error)
+  kErrBarrier = 1u << 4,        // a grid barrier of the fused rebin ran out of time
+};
+
+// State of a grid barrier (xnb_grid_barrier.cuh); zeroed once, left ready by each launch.
+struct GridBarrier {
+  unsigned int arrive;      // blocks arrived at the current barrier
+  unsigned int generation;  // barriers completed
+  unsigned int error;       // 1: a wait ran out
+  unsigned int pad;
 };
 
 // Per-system constants, device resident (SysDesc[nsys]).
@@ -110,6 +119,7 @@ struct DevArrays {
   float4* pf;                      // FP32 hi part of (x - origin, y - origin, z - origin), refreshed with r;
                                    // .w packs the three residuals as 10-bit multiples of lo_step_f (lo_field)
   float4* pflo;                    // FP32 residual (x - origin) - hi, so hi + lo carries ~48 bits
+  GridBarrier* grid_ctl;           // of the fused rebin
   unsigned int* any_rebuild;       // number of systems flagged for the rebuild path this step
   uint64_t* id;
   uint8_t* ptype;                  // particle type (field::type), 0 unless set

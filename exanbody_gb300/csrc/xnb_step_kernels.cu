@@ -2,6 +2,7 @@
 // Lennard-Jones pair-force traversal over the neighbour lists.
 #include <algorithm>
 
+#include "xnb_grid_barrier.cuh"
 #include "xnb_launch.cuh"
 #include "xnb_lj_pair.cuh"
 #include "xnb_traverse.cuh"
@@ -462,56 +463,15 @@ void force_dispatch(const Extent& ex, const SysDesc* sys, const SysState* st, co
 // every block reads step k's word after the first barrier of step k, and block
 // 0 clears the other word during step k's forces, after every block has read it
 // at step k - 1 and before step k + 1 sets it.
-__device__ __forceinline__ unsigned int ld_acquire_u32(const unsigned int* p) {
-  unsigned int v;
-  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-
-__device__ __forceinline__ unsigned long long global_ns() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
-
-// Blocks count in; the last one resets the count and bumps the generation, the
-// others poll the generation for at most wait_ns. A wait that runs out records
-// the error and returns false (the loop then ends without another barrier).
-__device__ bool grid_barrier(StepCtl* ctl, unsigned int nblocks, unsigned long long wait_ns) {
-  __syncthreads();
-  int ok = 1;
-  if (threadIdx.x == 0) {
-    const unsigned int gen = ld_acquire_u32(&ctl->generation);
-    __threadfence();
-    if (atomicAdd(&ctl->arrive, 1u) == nblocks - 1u) {
-      atomicExch(&ctl->arrive, 0u);
-      __threadfence();
-      atomicAdd(&ctl->generation, 1u);
-    } else {
-      const unsigned long long t0 = global_ns();
-      while (ld_acquire_u32(&ctl->generation) == gen) {
-        if (global_ns() - t0 > wait_ns) {
-          atomicOr(&ctl->error, 1u);
-          ok = 0;
-          break;
-        }
-        __nanosleep(100);
-      }
-    }
-    __threadfence();
-  }
-  return __syncthreads_and(ok) != 0;
-}
-
 template <bool EXACT, int P, bool PE, bool PACKED = true>
 __global__ void __maxnreg__(72)
     k_steps_persistent(uint32_t n_part, int nsys, const SysDesc* __restrict__ sys, SysState* __restrict__ st,
                        DevArrays a, BatchSource src, LJForce<P, PE, true, PACKED> f, StepCtl* ctl, int max_steps,
                        unsigned int nblocks, unsigned long long wait_ns, bool check) {
-  if (check && !grid_barrier(ctl, nblocks + 1u, wait_ns)) return;
+  if (check && !grid_barrier(&ctl->bar, nblocks + 1u, wait_ns)) return;
   for (int k = 0; k < max_steps; ++k) {
     first_half_body<EXACT>(n_part, nsys, sys, st, a, true, true, true, 1.0, 0.5, -1, &ctl->fired[k & 1]);
-    if (!grid_barrier(ctl, nblocks, wait_ns)) return;
+    if (!grid_barrier(&ctl->bar, nblocks, wait_ns)) return;
     if (ld_acquire_u32(&ctl->fired[k & 1])) {
       if (blockIdx.x == 0 && threadIdx.x == 0) {
         ctl->steps_done = static_cast<unsigned int>(k);
@@ -522,7 +482,7 @@ __global__ void __maxnreg__(72)
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n_part; i += gridDim.x * blockDim.x)
       pair::traverse_particle(src, i, f);
     if (blockIdx.x == 0 && threadIdx.x == 0) ctl->fired[(k + 1) & 1] = 0u;
-    if (!grid_barrier(ctl, nblocks, wait_ns)) return;
+    if (!grid_barrier(&ctl->bar, nblocks, wait_ns)) return;
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     ctl->steps_done = static_cast<unsigned int>(max_steps);
