@@ -792,24 +792,114 @@ __global__ void __launch_bounds__(128, 8)
 }
 
 // ---------------------------------------------------------------------------
-// Warp-per-cell form of the same build, for every cell whose candidates fit the
-// warp's stage (cap); the others are appended to a.nbr_wide for k_neighbors.
-// Each warp stages its cell's candidates itself (no block barrier), then tests
+// Warp-per-cell form of the same build. The warp stages the candidates that can
+// lie within nbh_dist of any of the cell's particles -- those within reach of
+// the particles' bounding box, about 3/4 of the 27-cell block; the FP32 distance
+// to the box rounds like the pair test and never exceeds it, so what is left out
+// is what the test would refuse -- and tests up to
 // kWarpP particles per staged load: lanes hold 32 candidates, and a ballot per
-// particle appends its hits in order straight to the particle's list slot
-// (an entry past the slot lands on its last word; the count flags the
-// overflow). Two rare cases leave the fast test through
-// warp-uniform branches: a chunk holding a candidate whose ghost filter is
-// undecided in FP32, and an FP32 distance inside the error band around nbh^2
-// (both then take the reference's FP64 decision, as in k_neighbors).
-// Six particles per staged load fit 96 registers (8 bytes spilled), so 5 blocks
-// of 4 warps stay resident per SM (5 x 40 KB of stage at cap 640); eight per
-// load need 126 registers and hold 4 blocks, and take 13% longer per rebuild.
+// particle appends its hits in order straight to the particle's list slot (an
+// entry past the slot lands on its last word; the count flags the overflow).
+// The candidates come as runs of x-adjacent cells, contiguous in memory, so no
+// lane searches for its cell; a ballot compacts them in order. Two rare cases
+// leave the fast test through warp-uniform branches: a chunk holding a candidate
+// whose ghost filter is undecided in FP32, and an FP32 distance inside the error
+// band around nbh^2 (both then take the reference's FP64 decision). A cell whose
+// kept candidates exceed the stage (cap) is appended to a.nbr_wide for
+// k_neighbors.
+// The build is bound by instruction issue. Six particles per staged load fit 96
+// registers, so 5 blocks of 4 warps stay resident per SM; the last particles of
+// a cell are tested four or two at a time, not padded to six.
 constexpr int kWarpP = 6;  // particles tested per staged candidate load in the warp-per-cell build
 
+// FP32 values as integers in the same order (no NaN).
+__device__ __forceinline__ int ordered_int(float f) {
+  const int b = __float_as_int(f);
+  return b ^ ((b >> 31) & 0x7fffffff);
+}
+__device__ __forceinline__ float from_ordered(int k) { return __int_as_float(k ^ ((k >> 31) & 0x7fffffff)); }
+
+// What one warp of the warp-per-cell build works on.
+struct WarpCell {
+  uint32_t sa, na;        // the cell's particles
+  uint32_t off_self;      // stage index of its first particle
+  uint32_t mpad;          // staged candidates, padded to whole chunks
+  uint32_t slot;
+  uint32_t* seg;          // the system's list segment
+  uint32_t* sink;
+  float nb_lo, nb_hi, nb_zero;
+  unsigned lt;
+};
+
+// Particles p0 .. p0 + NP - 1 of the cell against the whole stage.
+template <int NP>
+__device__ __forceinline__ void warp_pass(const SysDesc& S, const DevArrays& a, const WarpCell& w, const float4* srel,
+                                          float4 own, uint32_t p0, uint32_t lane, uint32_t& acc_max,
+                                          unsigned long long& acc_sum) {
+  // particles past the cell's end sit at -1e18: never within reach of a
+  // candidate (real ones, or the +1e18 dummies), so they need no test
+  float px[NP], py[NP], pz[NP];
+  uint32_t cur[NP], half[NP];
+#pragma unroll
+  for (int k = 0; k < NP; ++k) {
+    const uint32_t pk = p0 + k;
+    float4 q;
+    if (w.na <= 32) {
+      q.x = __shfl_sync(0xffffffffu, own.x, pk & 31u);
+      q.y = __shfl_sync(0xffffffffu, own.y, pk & 31u);
+      q.z = __shfl_sync(0xffffffffu, own.z, pk & 31u);
+    } else {
+      q = pk < w.na ? a.pf[w.sa + pk] : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    const bool valid = pk < w.na;
+    px[k] = valid ? q.x : -1.0e18f;
+    py[k] = valid ? q.y : -1.0e18f;
+    pz[k] = valid ? q.z : -1.0e18f;
+    cur[k] = 0;
+    half[k] = 0;
+  }
+  const uint32_t i0 = w.sa + p0;
+  const uint32_t self0 = ((i0 - S.part_base) << 5) | static_cast<uint32_t>(kImageCenter);
+  const uint32_t low0 = w.off_self + p0;
+  // hits go straight to the particles' slots (consecutive particles, stride
+  // slot); a system without slots yet (the sizing build) only counts, its
+  // hits landing in the warp's sink
+  uint32_t* const pslot = w.slot ? w.seg + static_cast<size_t>(i0 - S.part_base) * w.slot : w.sink;
+  const uint32_t pstride = w.slot ? w.slot : 1u;
+  for (uint32_t t0 = 0; t0 < w.mpad; t0 += 32) {
+    const float4 b = srel[t0 + lane];
+    const uint32_t ent = __float_as_uint(b.w);
+    // the particles' own entries (lower-half ends) sit at stage indices low0 + k;
+    // entries in [kAmbiguousBit, kInvalid): ghost filter undecided in FP32
+    const bool self_chunk = t0 < low0 + NP && low0 < t0 + 32u;
+    if (self_chunk || __any_sync(0xffffffffu, ent - kAmbiguousBit < kInvalid - kAmbiguousBit))
+      nbr_chunk<NP, true, true>(S, a, b, px, py, pz, i0, self0, t0, low0, w.nb_lo, w.nb_hi, w.nb_zero, w.lt, pslot,
+                                pstride, cur, half);
+    else
+      nbr_chunk<NP, false, false>(S, a, b, px, py, pz, i0, self0, t0, low0, w.nb_lo, w.nb_hi, w.nb_zero, w.lt, pslot,
+                                  pstride, cur, half);
+  }
+#pragma unroll
+  for (int k = 0; k < NP; ++k) {
+    const uint32_t pk = p0 + k;
+    if (pk < w.na) {
+      const uint32_t i = w.sa + pk;
+      if (lane == 0) {
+        a.nbr_cnt[i] = cur[k];
+        a.nbr_half[i] = half[k];
+        a.nbr_start[i] = (i - S.part_base) * w.slot;  // the host keeps npart * slot below 2^32
+      }
+      acc_max = max(acc_max, cur[k]);
+      acc_sum += cur[k];
+    }
+  }
+}
+
+// split warps share a cell (each stages it and takes every split-th group of
+// particles): batches with fewer cells than the GPU holds warps.
 __global__ void __launch_bounds__(128, 5)
     k_neighbors_warp(uint32_t n_cells, const SysDesc* __restrict__ sys, SysState* st, DevArrays a, int cap,
-                     bool prune, bool half_form) {
+                     bool prune, bool half_form, uint32_t split) {
   if (*a.any_rebuild == 0) return;
   extern __shared__ float4 stage_w[];
   const uint32_t lane = threadIdx.x & 31;
@@ -817,24 +907,30 @@ __global__ void __launch_bounds__(128, 5)
   const uint32_t nwarp = blockDim.x >> 5;
   float4* srel = stage_w + static_cast<size_t>(wib) * cap;
   __shared__ uint32_t sink[4][kWarpP];  // hits of systems without list slots (blocks of 4 warps)
-  const unsigned lt = lanemask_lt();
+  WarpCell w;
+  w.lt = lanemask_lt();
+  w.sink = sink[wib];
   uint32_t acc_s = kInvalid, acc_max = 0;
   unsigned long long acc_sum = 0;
   const uint32_t nw_all = gridDim.x * nwarp;
-  for (uint32_t c = blockIdx.x * nwarp + wib; c < n_cells; c += nw_all) {
+  for (uint32_t u = blockIdx.x * nwarp + wib; u < n_cells * split; u += nw_all) {
+    const uint32_t c = u / split, part = u - c * split;
     const uint32_t s = a.cell_sys[c];
     if (s == kInvalid || !sys_flagged(st, s)) continue;
     if (half_form && !st[s].half_bad) continue;  // built by the half-shell kernels
     const uint32_t na = a.cell_n[c];
-    if (na == 0) continue;
+    if (na <= part * kWarpP) continue;
     if (prune && a.cside[c] >= 2 && st[s].keys_fresh) {
-      if (lane == 0) a.nbr_sub[atomicAdd(a.nbr_sub_n, 1u)] = c;
+      if (lane == 0 && part == 0) a.nbr_sub[atomicAdd(a.nbr_sub_n, 1u)] = c;
       continue;
     }
     const SysDesc& S = sys[s];
     const uint32_t sa = a.cell_start[c];
     int ci, cj, ck;
     cell_ijk(S, c - S.cell_base, ci, cj, ck);
+    w.nb_hi = S.nbh2_f + S.nbh_margin_f;
+    w.nb_lo = S.nbh2_f - S.nbh_margin_f;
+    w.nb_zero = S.nbh_margin_f;
 
     // group table: lane g < 27 describes neighbour cell g in (dk, dj, di) order
     uint32_t g_start = 0, g_n = 0, g_code = kImageCenter;
@@ -853,130 +949,100 @@ __global__ void __launch_bounds__(128, 5)
       g_n = a.cell_n[src];
       g_code = static_cast<uint32_t>(img[0] + 3 * img[1] + 9 * img[2]);
     }
-    uint32_t g_off = g_n;  // inclusive scan over lanes
-    for (int off = 1; off < 32; off <<= 1) {
-      const uint32_t v = __shfl_up_sync(0xffffffffu, g_off, off);
-      if (lane >= static_cast<uint32_t>(off)) g_off += v;
+    // the three cells of a row are one contiguous run unless x wraps around:
+    // the first lane of the row then takes them all
+    {
+      const uint32_t n1 = __shfl_down_sync(0xffffffffu, g_n, 1), n2 = __shfl_down_sync(0xffffffffu, g_n, 2);
+      if (ci > 0 && ci < S.dims[0] - 1) g_n = lane % 3u == 0u ? g_n + n1 + n2 : 0u;
     }
-    const uint32_t ncand = __shfl_sync(0xffffffffu, g_off, 26);
-    g_off -= g_n;
-    const uint32_t slot = S.list_slot;
-    if (ncand > static_cast<uint32_t>(cap)) {
-      if (lane == 0) a.nbr_wide[atomicAdd(a.nbr_wide_n, 1u)] = c;
+
+    // the particles' bounding box
+    float4 own = make_float4(0.f, 0.f, 0.f, 0.f);
+    float bl[3] = {3.0e38f, 3.0e38f, 3.0e38f}, bh[3] = {-3.0e38f, -3.0e38f, -3.0e38f};
+    for (uint32_t q = lane; q < na; q += 32) {
+      const float4 v = a.pf[sa + q];
+      if (q == lane) own = v;
+      bl[0] = fminf(bl[0], v.x);
+      bl[1] = fminf(bl[1], v.y);
+      bl[2] = fminf(bl[2], v.z);
+      bh[0] = fmaxf(bh[0], v.x);
+      bh[1] = fmaxf(bh[1], v.y);
+      bh[2] = fmaxf(bh[2], v.z);
+    }
+#pragma unroll
+    for (int ax = 0; ax < 3; ++ax) {
+      bl[ax] = from_ordered(__reduce_min_sync(0xffffffffu, ordered_int(bl[ax])));
+      bh[ax] = from_ordered(__reduce_max_sync(0xffffffffu, ordered_int(bh[ax])));
+    }
+
+    // stage: 32 candidates of a run per iteration, the next 32 already loading
+    uint32_t m = 0, off_self = 0;
+    {
+      unsigned todo = __ballot_sync(0xffffffffu, lane < 27u && g_n > 0u);
+      uint32_t at = 0, left = 0, code = kImageCenter;  // the run being read
+      auto next_run = [&]() {
+        const int g = __ffs(todo) - 1;
+        todo &= todo - 1u;
+        at = __shfl_sync(0xffffffffu, g_start, g);
+        left = __shfl_sync(0xffffffffu, g_n, g);
+        code = __shfl_sync(0xffffffffu, g_code, g);
+      };
+      next_run();
+      float4 pb = lane < left ? __ldg(a.pf + at + lane) : make_float4(0.f, 0.f, 0.f, 0.f);
+      for (;;) {
+        const float4 cb = pb;
+        const uint32_t c_at = at, c_code = code, c_left = left;
+        at += 32u;
+        left = left > 32u ? left - 32u : 0u;
+        bool more = true;
+        if (left == 0) {
+          more = todo != 0;
+          if (more) next_run();
+        }
+        if (more) pb = lane < left ? __ldg(a.pf + at + lane) : make_float4(0.f, 0.f, 0.f, 0.f);
+        const float4 rb = stage_from(S, cb, c_at + lane, c_code);
+        const float ex = fmaxf(fmaxf(bl[0] - rb.x, rb.x - bh[0]), 0.f);
+        const float ey = fmaxf(fmaxf(bl[1] - rb.y, rb.y - bh[1]), 0.f);
+        const float ez = fmaxf(fmaxf(bl[2] - rb.z, rb.z - bh[2]), 0.f);
+        const bool keep = lane < c_left && fmaf(ex, ex, fmaf(ey, ey, ez * ez)) <= w.nb_hi;
+        const unsigned km = __ballot_sync(0xffffffffu, keep);
+        // the cell's own particles are all kept (distance 0)
+        const uint32_t self = sa - c_at;
+        if (c_code == static_cast<uint32_t>(kImageCenter) && self < 32u && self < c_left)
+          off_self = m + __popc(km & ((1u << self) - 1u));
+        const uint32_t pos = m + __popc(km & w.lt);
+        if (keep && pos < static_cast<uint32_t>(cap)) srel[pos] = rb;
+        m += __popc(km);
+        if (!more) break;
+      }
+    }
+    if (m > static_cast<uint32_t>(cap)) {
+      __syncwarp();
+      if (lane == 0 && part == 0) a.nbr_wide[atomicAdd(a.nbr_wide_n, 1u)] = c;
       continue;
     }
+    const uint32_t mpad = (m + 31u) & ~31u;  // <= cap (a multiple of 32)
+    if (m + lane < mpad) srel[m + lane] = make_float4(1.0e18f, 1.0e18f, 1.0e18f, __uint_as_float(kInvalid));
+    __syncwarp();
     if (s != acc_s) {
       if (lane == 0) flush_list_stats(st, sys, acc_s, acc_max, acc_sum);
       acc_s = s;
       acc_max = 0;
       acc_sum = 0;
     }
-    const uint32_t off_self = __shfl_sync(0xffffffffu, g_off, 13);
-    float4 own = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (na <= 32 && lane < na) own = a.pf[sa + lane];
-
-    // stage: candidate u belongs to the last group g with g_off[g] <= u; four
-    // candidates per lane are located and loaded before any is converted
-    const uint32_t mpad = (ncand + 31u) & ~31u;
-    for (uint32_t t0 = 0; t0 < mpad; t0 += 128u) {
-      float4 pb[4];
-      uint32_t jj[4], gcs[4];
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const uint32_t u = t0 + 32u * k + lane;
-        uint32_t g = 0;
-#pragma unroll
-        for (uint32_t step = 16; step > 0; step >>= 1) {
-          const uint32_t probe = g + step;
-          const uint32_t po = __shfl_sync(0xffffffffu, g_off, probe < 27u ? probe : 26u);
-          if (probe < 27u && po <= u) g = probe;
-        }
-        const uint32_t gs = __shfl_sync(0xffffffffu, g_start, g);
-        const uint32_t go = __shfl_sync(0xffffffffu, g_off, g);
-        gcs[k] = __shfl_sync(0xffffffffu, g_code, g);
-        jj[k] = gs + (u - go);
-        pb[k] = u < ncand ? __ldg(a.pf + jj[k]) : make_float4(0.f, 0.f, 0.f, 0.f);
-      }
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const uint32_t u = t0 + 32u * k + lane;
-        if (u < ncand) srel[u] = stage_from(S, pb[k], jj[k], gcs[k]);
-        else if (u < mpad) srel[u] = make_float4(1.0e18f, 1.0e18f, 1.0e18f, __uint_as_float(kInvalid));
-      }
+    w.sa = sa;
+    w.na = na;
+    w.off_self = off_self;
+    w.mpad = mpad;
+    w.slot = S.list_slot;
+    w.seg = a.nbr + S.list_base;
+    for (uint32_t p0 = part * kWarpP; p0 < na; p0 += kWarpP * split) {
+      const uint32_t rest = na - p0;
+      if (rest > 4u) warp_pass<6>(S, a, w, srel, own, p0, lane, acc_max, acc_sum);
+      else if (rest > 2u) warp_pass<4>(S, a, w, srel, own, p0, lane, acc_max, acc_sum);
+      else warp_pass<2>(S, a, w, srel, own, p0, lane, acc_max, acc_sum);
     }
-    __syncwarp();
-
-    const float nb_hi = S.nbh2_f + S.nbh_margin_f;
-    const float nb_lo = S.nbh2_f - S.nbh_margin_f;
-    const float nb_zero = S.nbh_margin_f;
-    uint32_t* const seg = a.nbr + S.list_base;
-    for (uint32_t p0 = 0; p0 < na; p0 += kWarpP) {
-      // particles past the cell's end sit at -1e18: never within reach of a
-      // candidate (real ones, or the +1e18 dummies), so they need no test
-      float px[kWarpP], py[kWarpP], pz[kWarpP];
-      uint32_t cur[kWarpP], half[kWarpP];
-#pragma unroll
-      for (int k = 0; k < kWarpP; ++k) {
-        const uint32_t pk = p0 + k;
-        float4 q;
-        if (na <= 32) {
-          q.x = __shfl_sync(0xffffffffu, own.x, pk & 31u);
-          q.y = __shfl_sync(0xffffffffu, own.y, pk & 31u);
-          q.z = __shfl_sync(0xffffffffu, own.z, pk & 31u);
-        } else {
-          q = pk < na ? a.pf[sa + pk] : make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-        const bool valid = pk < na;
-        px[k] = valid ? q.x : -1.0e18f;
-        py[k] = valid ? q.y : -1.0e18f;
-        pz[k] = valid ? q.z : -1.0e18f;
-        cur[k] = 0;
-        half[k] = 0;
-      }
-      const uint32_t i0 = sa + p0;
-      const uint32_t self0 = ((i0 - S.part_base) << 5) | static_cast<uint32_t>(kImageCenter);
-      const uint32_t low0 = off_self + p0;
-      // hits go straight to the particles' slots (consecutive particles, stride
-      // slot); a system without slots yet (the sizing build) only counts, its
-      // hits landing in the warp's sink
-      uint32_t* const pslot = slot ? seg + static_cast<size_t>(i0 - S.part_base) * slot : sink[wib];
-      const uint32_t pstride = slot ? slot : 1u;
-      for (uint32_t t0 = 0; t0 < mpad; t0 += 32) {
-        const float4 b = srel[t0 + lane];
-        const uint32_t ent = __float_as_uint(b.w);
-        // the particles' own entries (lower-half ends) sit at stage indices low0 + k
-        const bool self_chunk = t0 < low0 + kWarpP && low0 < t0 + 32u;
-        // entries in [kAmbiguousBit, kInvalid): ghost filter undecided in FP32
-        if (__any_sync(0xffffffffu, ent - kAmbiguousBit < kInvalid - kAmbiguousBit)) {
-          if (self_chunk)
-            nbr_chunk<kWarpP, true, true>(S, a, b, px, py, pz, i0, self0, t0, low0, nb_lo, nb_hi, nb_zero, lt, pslot,
-                                          pstride, cur, half);
-          else
-            nbr_chunk<kWarpP, true, false>(S, a, b, px, py, pz, i0, self0, t0, low0, nb_lo, nb_hi, nb_zero, lt, pslot,
-                                           pstride, cur, half);
-        } else if (self_chunk) {
-          nbr_chunk<kWarpP, false, true>(S, a, b, px, py, pz, i0, self0, t0, low0, nb_lo, nb_hi, nb_zero, lt, pslot,
-                                         pstride, cur, half);
-        } else {
-          nbr_chunk<kWarpP, false, false>(S, a, b, px, py, pz, i0, self0, t0, low0, nb_lo, nb_hi, nb_zero, lt, pslot,
-                                          pstride, cur, half);
-        }
-      }
-#pragma unroll
-      for (int k = 0; k < kWarpP; ++k) {
-        const uint32_t pk = p0 + k;
-        if (pk < na) {
-          const uint32_t i = sa + pk;
-          if (lane == 0) {
-            a.nbr_cnt[i] = cur[k];
-            a.nbr_half[i] = half[k];
-            a.nbr_start[i] = (i - S.part_base) * slot;  // the host keeps npart * slot below 2^32
-          }
-          acc_max = max(acc_max, cur[k]);
-          acc_sum += cur[k];
-        }
-      }
-    }
+    __syncwarp();  // the stage is refilled for the next cell
   }
   if (lane == 0) flush_list_stats(st, sys, acc_s, acc_max, acc_sum);
 }
@@ -1178,14 +1244,17 @@ int launch_neighbors(const Extent& ex, const SysDesc* sys, SysState* st, const D
   int per_sm = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_neighbors_warp, 128, smem_w) != cudaSuccess || per_sm < 1)
     per_sm = 1;
-  const long long want_w = (static_cast<long long>(ex.n_cells) + 3) / 4;
+  // four or two warps per cell while that leaves no warp of the GPU without one
+  const long long warps = static_cast<long long>(per_sm) * ex.sm_count * 4;
+  const uint32_t split = ex.n_cells * 4ll <= warps ? 4u : (ex.n_cells * 2ll <= warps ? 2u : 1u);
+  const long long want_w = (static_cast<long long>(ex.n_cells) * split + 3) / 4;
   const int grid_w = static_cast<int>(std::max(1ll, std::min(want_w, static_cast<long long>(per_sm) * ex.sm_count)));
   if (reset) k_nbr_reset<<<(ex.nsys + 127) / 128, 128, 0, stream>>>(ex.nsys, st, a.any_rebuild, a.nbr_wide_n, a.nbr_sub_n);
   // half-shell form: masks first; systems it cannot take go through the warp-per-cell build
   const bool half = form == kBuildHalf && a.nmask != nullptr;
   const int nh = half ? launch_neighbors_half_test(ex, sys, st, a, stream) : 0;
   if (form == kBuildRows) launch_neighbors_rows(ex, sys, st, a, stream, prune);
-  else k_neighbors_warp<<<grid_w, 128, smem_w, stream>>>(ex.n_cells, sys, st, a, cap, prune, half);
+  else k_neighbors_warp<<<grid_w, 128, smem_w, stream>>>(ex.n_cells, sys, st, a, cap, prune, half, split);
   const int ne = half ? launch_neighbors_half_emit(ex, sys, st, a, stream) : 0;
   // dense cells (sub-grid side >= 2), before the block-per-cell build, which takes the ones it passes on
   const int nsub = prune ? launch_neighbors_sub(ex, sys, st, a, cap, stream) : 0;
