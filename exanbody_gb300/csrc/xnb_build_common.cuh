@@ -144,6 +144,53 @@ __device__ __forceinline__ void nbr_chunk(const SysDesc& S, const DevArrays& a, 
   }
 }
 
+// The same chunk when nothing in it needs a closer look: no own entry, no
+// undecided ghost filter, room for 32 more entries in every slot (the caller
+// checks those), and every distance outside the FP32 band (checked here: false,
+// with nothing appended, when one is not -- nbr_chunk then decides). Particles
+// come as packed pairs; band is at least the half width of the band around
+// nbh2. Per particle: three packed FP32 operations, a compare, a ballot and the
+// append; the band is watched by minima over all particles.
+template <int NP>
+__device__ __forceinline__ bool nbr_chunk_clear(const float4 b, const unsigned long long (&px)[NP / 2],
+                                                const unsigned long long (&py)[NP / 2],
+                                                const unsigned long long (&pz)[NP / 2], float nb_lo, float nb_zero,
+                                                unsigned long long minus_nbh2, float band, unsigned lt,
+                                                uint32_t* out, uint32_t stride, uint32_t (&cur)[NP]) {
+  float dd[NP];
+  float off = 3.0e38f, least = 3.0e38f;
+  unsigned long long bx2, by2, bz2;
+  asm("mov.b64 %0, {%1, %1};" : "=l"(bx2) : "f"(b.x));
+  asm("mov.b64 %0, {%1, %1};" : "=l"(by2) : "f"(b.y));
+  asm("mov.b64 %0, {%1, %1};" : "=l"(bz2) : "f"(b.z));
+#pragma unroll
+  for (int k = 0; k < NP / 2; ++k) {
+    unsigned long long dx, dy, dz, d, t;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(dx) : "l"(px[k]), "l"(bx2));
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(dy) : "l"(py[k]), "l"(by2));
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(dz) : "l"(pz[k]), "l"(bz2));
+    asm("mul.rn.f32x2 %0, %1, %1;" : "=l"(d) : "l"(dz));
+    asm("fma.rn.f32x2 %0, %1, %1, %2;" : "=l"(d) : "l"(dy), "l"(d));
+    asm("fma.rn.f32x2 %0, %1, %1, %2;" : "=l"(d) : "l"(dx), "l"(d));
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(t) : "l"(d), "l"(minus_nbh2));
+    float t0, t1;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(t0), "=f"(t1) : "l"(t));
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(dd[2 * k]), "=f"(dd[2 * k + 1]) : "l"(d));
+    off = fminf(fminf(fabsf(t0), fabsf(t1)), off);
+    least = fminf(fminf(dd[2 * k], dd[2 * k + 1]), least);
+  }
+  if (__any_sync(0xffffffffu, off <= band || least <= nb_zero)) return false;
+  const uint32_t e = __float_as_uint(b.w);
+#pragma unroll
+  for (int k = 0; k < NP; ++k) {
+    const bool hit = dd[k] < nb_lo;
+    const unsigned m = __ballot_sync(0xffffffffu, hit);
+    if (hit) out[k * stride + cur[k] + __popc(m & lt)] = e;
+    cur[k] += __popc(m);
+  }
+  return true;
+}
+
 // Per-warp list statistics, flushed to the system's state when the warp moves
 // on to another system's cells and at the end.
 __device__ __forceinline__ void flush_list_stats(SysState* st, const SysDesc* sys, uint32_t s, uint32_t mx,

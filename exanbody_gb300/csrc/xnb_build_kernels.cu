@@ -807,10 +807,12 @@ __global__ void __launch_bounds__(128, 8)
 // band around nbh^2 (both then take the reference's FP64 decision). A cell whose
 // kept candidates exceed the stage (cap) is appended to a.nbr_wide for
 // k_neighbors.
-// The build is bound by instruction issue. Six particles per staged load fit 96
-// registers, so 5 blocks of 4 warps stay resident per SM; the last particles of
-// a cell are tested four or two at a time, not padded to six.
-constexpr int kWarpP = 6;  // particles tested per staged candidate load in the warp-per-cell build
+// The build is bound by instruction issue (479 warp instructions per atom before
+// the chunk test was split into nbr_chunk_clear and nbr_chunk). Four particles
+// per staged load fit 95 registers, 5 blocks of 4 warps per SM; six spill there
+// (1.18 against 1.03 ms per build of 1,972,156 atoms), four at 6 blocks 1.07 ms.
+// The last particles of a cell are tested two at a time, not padded to four.
+constexpr int kWarpP = 4;  // particles tested per staged candidate load in the warp-per-cell build
 
 // FP32 values as integers in the same order (no NaN).
 __device__ __forceinline__ int ordered_int(float f) {
@@ -824,18 +826,25 @@ struct WarpCell {
   uint32_t sa, na;        // the cell's particles
   uint32_t off_self;      // stage index of its first particle
   uint32_t mpad;          // staged candidates, padded to whole chunks
+  bool undecided;         // some have an undecided ghost filter
   uint32_t slot;
   uint32_t* seg;          // the system's list segment
   uint32_t* sink;
-  float nb_lo, nb_hi, nb_zero;
+  float nb_lo, nb_hi, nb_zero, band;
   unsigned lt;
+};
+
+// List lengths of one cell: lane p's particle, and this lane's largest and sum.
+struct CellCounts {
+  uint32_t cnt, half;
+  bool mine;
+  uint32_t most, sum;
 };
 
 // Particles p0 .. p0 + NP - 1 of the cell against the whole stage.
 template <int NP>
 __device__ __forceinline__ void warp_pass(const SysDesc& S, const DevArrays& a, const WarpCell& w, const float4* srel,
-                                          float4 own, uint32_t p0, uint32_t lane, uint32_t& acc_max,
-                                          unsigned long long& acc_sum) {
+                                          float4 own, uint32_t p0, uint32_t lane, CellCounts& counts) {
   // particles past the cell's end sit at -1e18: never within reach of a
   // candidate (real ones, or the +1e18 dummies), so they need no test
   float px[NP], py[NP], pz[NP];
@@ -866,18 +875,45 @@ __device__ __forceinline__ void warp_pass(const SysDesc& S, const DevArrays& a, 
   // hits landing in the warp's sink
   uint32_t* const pslot = w.slot ? w.seg + static_cast<size_t>(i0 - S.part_base) * w.slot : w.sink;
   const uint32_t pstride = w.slot ? w.slot : 1u;
+  unsigned long long px2[NP / 2], py2[NP / 2], pz2[NP / 2], minus_nbh2;
+#pragma unroll
+  for (int k = 0; k < NP / 2; ++k) {
+    asm("mov.b64 %0, {%1, %2};" : "=l"(px2[k]) : "f"(px[2 * k]), "f"(px[2 * k + 1]));
+    asm("mov.b64 %0, {%1, %2};" : "=l"(py2[k]) : "f"(py[2 * k]), "f"(py[2 * k + 1]));
+    asm("mov.b64 %0, {%1, %2};" : "=l"(pz2[k]) : "f"(pz[2 * k]), "f"(pz[2 * k + 1]));
+  }
+  asm("mov.b64 %0, {%1, %1};" : "=l"(minus_nbh2) : "f"(-S.nbh2_f));
+  const uint32_t self_t0 = low0 & ~31u, self_span = ((low0 + NP - 1u) & ~31u) - self_t0;
+  uint32_t room = 0;  // chunks that fit every slot whatever they hold
   for (uint32_t t0 = 0; t0 < w.mpad; t0 += 32) {
     const float4 b = srel[t0 + lane];
     const uint32_t ent = __float_as_uint(b.w);
     // the particles' own entries (lower-half ends) sit at stage indices low0 + k;
     // entries in [kAmbiguousBit, kInvalid): ghost filter undecided in FP32
-    const bool self_chunk = t0 < low0 + NP && low0 < t0 + 32u;
-    if (self_chunk || __any_sync(0xffffffffu, ent - kAmbiguousBit < kInvalid - kAmbiguousBit))
+    if (room == 0) {
+      uint32_t most = cur[0];
+#pragma unroll
+      for (int k = 1; k < NP; ++k) most = max(most, cur[k]);
+      room = w.slot > most ? (w.slot - most) >> 5 : 0u;
+    }
+    const bool close = t0 - self_t0 <= self_span || room == 0 ||
+                       (w.undecided && __any_sync(0xffffffffu, ent - kAmbiguousBit < kInvalid - kAmbiguousBit));
+    if (close || !nbr_chunk_clear<NP>(b, px2, py2, pz2, w.nb_lo, w.nb_zero, minus_nbh2, w.band, w.lt, pslot, pstride,
+                                      cur))
       nbr_chunk<NP, true, true>(S, a, b, px, py, pz, i0, self0, t0, low0, w.nb_lo, w.nb_hi, w.nb_zero, w.lt, pslot,
                                 pstride, cur, half);
-    else
-      nbr_chunk<NP, false, false>(S, a, b, px, py, pz, i0, self0, t0, low0, w.nb_lo, w.nb_hi, w.nb_zero, w.lt, pslot,
-                                  pstride, cur, half);
+    room -= room != 0 ? 1u : 0u;
+  }
+  if (w.na <= 32) {
+    // lane p keeps particle p's counts; they are written together
+#pragma unroll
+    for (int k = 0; k < NP; ++k)
+      if (lane == p0 + k) {
+        counts.cnt = cur[k];
+        counts.half = half[k];
+        counts.mine = lane < w.na;
+      }
+    return;
   }
 #pragma unroll
   for (int k = 0; k < NP; ++k) {
@@ -888,9 +924,9 @@ __device__ __forceinline__ void warp_pass(const SysDesc& S, const DevArrays& a, 
         a.nbr_cnt[i] = cur[k];
         a.nbr_half[i] = half[k];
         a.nbr_start[i] = (i - S.part_base) * w.slot;  // the host keeps npart * slot below 2^32
+        counts.most = max(counts.most, cur[k]);
+        counts.sum += cur[k];
       }
-      acc_max = max(acc_max, cur[k]);
-      acc_sum += cur[k];
     }
   }
 }
@@ -906,6 +942,9 @@ __global__ void __launch_bounds__(128, 5)
   const uint32_t wib = threadIdx.x >> 5;
   const uint32_t nwarp = blockDim.x >> 5;
   float4* srel = stage_w + static_cast<size_t>(wib) * cap;
+  constexpr int kSteps = 32;
+  __shared__ uint4 lists[4][kSteps];
+  uint4* const list = lists[wib];  // first candidate, candidates left, image code
   __shared__ uint32_t sink[4][kWarpP];  // hits of systems without list slots (blocks of 4 warps)
   WarpCell w;
   w.lt = lanemask_lt();
@@ -931,6 +970,7 @@ __global__ void __launch_bounds__(128, 5)
     w.nb_hi = S.nbh2_f + S.nbh_margin_f;
     w.nb_lo = S.nbh2_f - S.nbh_margin_f;
     w.nb_zero = S.nbh_margin_f;
+    w.band = 1.001f * fmaxf(w.nb_hi - S.nbh2_f, S.nbh2_f - w.nb_lo);
 
     // group table: lane g < 27 describes neighbour cell g in (dk, dj, di) order
     uint32_t g_start = 0, g_n = 0, g_code = kImageCenter;
@@ -975,45 +1015,57 @@ __global__ void __launch_bounds__(128, 5)
       bh[ax] = from_ordered(__reduce_max_sync(0xffffffffu, ordered_int(bh[ax])));
     }
 
-    // stage: 32 candidates of a run per iteration, the next 32 already loading
+    // stage: 32 candidates of a run per step, the steps listed first so that
+    // the loads of four are in flight together
     uint32_t m = 0, off_self = 0;
+    bool undecided = false;  // a candidate whose ghost filter FP32 does not decide
     {
-      unsigned todo = __ballot_sync(0xffffffffu, lane < 27u && g_n > 0u);
-      uint32_t at = 0, left = 0, code = kImageCenter;  // the run being read
-      auto next_run = [&]() {
-        const int g = __ffs(todo) - 1;
-        todo &= todo - 1u;
-        at = __shfl_sync(0xffffffffu, g_start, g);
-        left = __shfl_sync(0xffffffffu, g_n, g);
-        code = __shfl_sync(0xffffffffu, g_code, g);
-      };
-      next_run();
-      float4 pb = lane < left ? __ldg(a.pf + at + lane) : make_float4(0.f, 0.f, 0.f, 0.f);
-      for (;;) {
-        const float4 cb = pb;
-        const uint32_t c_at = at, c_code = code, c_left = left;
-        at += 32u;
-        left = left > 32u ? left - 32u : 0u;
-        bool more = true;
-        if (left == 0) {
-          more = todo != 0;
-          if (more) next_run();
+      const uint32_t steps = lane < 27u ? (g_n + 31u) >> 5 : 0u;
+      uint32_t at = steps;  // inclusive scan
+      for (int off = 1; off < 32; off <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xffffffffu, at, off);
+        if (lane >= static_cast<uint32_t>(off)) at += v;
+      }
+      const uint32_t total = __shfl_sync(0xffffffffu, at, 31);
+      at -= steps;
+      for (uint32_t t0 = 0; t0 < total; t0 += kSteps) {
+        __syncwarp();  // the previous list's readers are done
+        for (uint32_t q = 0; q < steps; ++q)
+          if (at + q - t0 < kSteps) list[at + q - t0] = make_uint4(g_start + 32u * q, g_n - 32u * q, g_code, 0u);
+        __syncwarp();
+        const uint32_t t1 = min(total - t0, static_cast<uint32_t>(kSteps));
+        for (uint32_t t = 0; t < t1; t += 4u) {
+          uint4 run[4];
+          float4 pb[4];
+#pragma unroll
+          for (uint32_t q = 0; q < 4u; ++q) {
+            run[q] = list[min(t + q, t1 - 1u)];
+            if (t + q >= t1) run[q].y = 0;
+            pb[q] = lane < run[q].y ? __ldg(a.pf + run[q].x + lane) : make_float4(0.f, 0.f, 0.f, 0.f);
+          }
+#pragma unroll
+          for (uint32_t q = 0; q < 4u; ++q) {
+            float4 rb = pb[q];
+            if (run[q].z == static_cast<uint32_t>(kImageCenter)) {
+              rb.w = __uint_as_float(((run[q].x + lane - S.part_base) << 5) | static_cast<uint32_t>(kImageCenter));
+            } else {
+              rb = stage_from(S, pb[q], run[q].x + lane, run[q].z);
+              undecided |= __float_as_uint(rb.w) - kAmbiguousBit < kInvalid - kAmbiguousBit;
+            }
+            const float ex = fmaxf(fmaxf(bl[0] - rb.x, rb.x - bh[0]), 0.f);
+            const float ey = fmaxf(fmaxf(bl[1] - rb.y, rb.y - bh[1]), 0.f);
+            const float ez = fmaxf(fmaxf(bl[2] - rb.z, rb.z - bh[2]), 0.f);
+            const bool keep = lane < run[q].y && fmaf(ex, ex, fmaf(ey, ey, ez * ez)) <= w.nb_hi;
+            const unsigned km = __ballot_sync(0xffffffffu, keep);
+            // the cell's own particles are all kept (distance 0)
+            const uint32_t self = sa - run[q].x;
+            if (run[q].z == static_cast<uint32_t>(kImageCenter) && self < 32u && self < run[q].y)
+              off_self = m + __popc(km & ((1u << self) - 1u));
+            const uint32_t pos = m + __popc(km & w.lt);
+            if (keep && pos < static_cast<uint32_t>(cap)) srel[pos] = rb;
+            m += __popc(km);
+          }
         }
-        if (more) pb = lane < left ? __ldg(a.pf + at + lane) : make_float4(0.f, 0.f, 0.f, 0.f);
-        const float4 rb = stage_from(S, cb, c_at + lane, c_code);
-        const float ex = fmaxf(fmaxf(bl[0] - rb.x, rb.x - bh[0]), 0.f);
-        const float ey = fmaxf(fmaxf(bl[1] - rb.y, rb.y - bh[1]), 0.f);
-        const float ez = fmaxf(fmaxf(bl[2] - rb.z, rb.z - bh[2]), 0.f);
-        const bool keep = lane < c_left && fmaf(ex, ex, fmaf(ey, ey, ez * ez)) <= w.nb_hi;
-        const unsigned km = __ballot_sync(0xffffffffu, keep);
-        // the cell's own particles are all kept (distance 0)
-        const uint32_t self = sa - c_at;
-        if (c_code == static_cast<uint32_t>(kImageCenter) && self < 32u && self < c_left)
-          off_self = m + __popc(km & ((1u << self) - 1u));
-        const uint32_t pos = m + __popc(km & w.lt);
-        if (keep && pos < static_cast<uint32_t>(cap)) srel[pos] = rb;
-        m += __popc(km);
-        if (!more) break;
       }
     }
     if (m > static_cast<uint32_t>(cap)) {
@@ -1034,14 +1086,25 @@ __global__ void __launch_bounds__(128, 5)
     w.na = na;
     w.off_self = off_self;
     w.mpad = mpad;
+    w.undecided = __any_sync(0xffffffffu, undecided);
     w.slot = S.list_slot;
     w.seg = a.nbr + S.list_base;
+    CellCounts counts{0u, 0u, false, 0u, 0u};
     for (uint32_t p0 = part * kWarpP; p0 < na; p0 += kWarpP * split) {
       const uint32_t rest = na - p0;
-      if (rest > 4u) warp_pass<6>(S, a, w, srel, own, p0, lane, acc_max, acc_sum);
-      else if (rest > 2u) warp_pass<4>(S, a, w, srel, own, p0, lane, acc_max, acc_sum);
-      else warp_pass<2>(S, a, w, srel, own, p0, lane, acc_max, acc_sum);
+      if (rest > 2u) warp_pass<4>(S, a, w, srel, own, p0, lane, counts);
+      else warp_pass<2>(S, a, w, srel, own, p0, lane, counts);
     }
+    if (counts.mine) {
+      const uint32_t i = sa + lane;
+      a.nbr_cnt[i] = counts.cnt;
+      a.nbr_half[i] = counts.half;
+      a.nbr_start[i] = (i - S.part_base) * w.slot;  // the host keeps npart * slot below 2^32
+      counts.most = counts.cnt;
+      counts.sum = counts.cnt;
+    }
+    acc_max = max(acc_max, __reduce_max_sync(0xffffffffu, counts.most));
+    acc_sum += __reduce_add_sync(0xffffffffu, counts.sum);
     __syncwarp();  // the stage is refilled for the next cell
   }
   if (lane == 0) flush_list_stats(st, sys, acc_s, acc_max, acc_sum);
