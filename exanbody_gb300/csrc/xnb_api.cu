@@ -271,6 +271,8 @@ SysDesc make_desc(const xnb_lj_params& p) {
   d.eps4 = 4. * p.epsilon;
   d.eps24 = 24. * p.epsilon;
   d.sig2 = p.sigma * p.sigma;
+  d.pd_a = d.sig2 > 0.0 ? d.eps24 / d.sig2 : 0.0;
+  d.pd_b = -2.0 * d.pd_a;
   d.mass = p.mass;
   d.divide_by_mass = p.divide_by_mass;
   d.amr_enabled = p.amr_enabled;

@@ -156,7 +156,7 @@ __global__ void __launch_bounds__(kStagedThreads, 2)
                    int sys_only) {
   extern __shared__ __align__(16) unsigned char staged_smem[];
   StagedSmem& sm = *reinterpret_cast<StagedSmem*>(staged_smem);
-  const LJForce<kMixed, PE, KICK> f{sys, a};
+  const LJForce<PE, KICK> f{sys, a};
   const BatchSource src(sys, st, a, sys_only);
   for (uint32_t sg = blockIdx.x; sg < n_seg; sg += gridDim.x) {
     const uint4 seg = a.seg[sg];  // first cell (global), cells, system
@@ -234,7 +234,7 @@ __global__ void __launch_bounds__(kStagedThreads, 2)
       }
       pair::ParticleContext c;
       if (!src.begin(i, false, false, c)) continue;
-      typename LJForce<kMixed, PE, KICK>::Acc q;
+      typename LJForce<PE, KICK>::Acc q;
       f.start(q, c);
       const uint32_t m = a.pcell[i] - seg.x;  // the particle's cell within the segment
       const uint16_t* __restrict__ L16 = a.nbr16 + S.list_base + a.nbr_start[i];

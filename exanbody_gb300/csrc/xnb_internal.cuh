@@ -83,6 +83,7 @@ struct SysDesc {
   float image_tie_f;             // bound on the error of an image displacement formed from FP32 pairs
   int32_t packed_lo;             // 1: the mixed traversal reads the packed residuals (X < 1024); 0: DevArrays::pflo
   double inv_cell;               // fl(1/cell_size): reciprocal pre-decision of the backup encoding
+  double pd_a, pd_b;             // 24 eps / sigma^2 and -48 eps / sigma^2 (FP64 pair factor)
   double m24eps, eps4, sig2, eps24;  // -24*eps, 4*eps (lennard_jones.cu:54-55), sigma^2, 24*eps
   int32_t dims[3];
   int32_t divide_by_mass;

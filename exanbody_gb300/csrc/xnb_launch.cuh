@@ -52,6 +52,11 @@ constexpr uint32_t kMixedSplitMax = 100000;
 int launch_force_mixed(const Extent& ex, const SysDesc* sys, const SysState* st, const DevArrays& a, bool with_pe,
                        bool second_half, int sys_only, cudaStream_t stream);
 
+// FP64 and FP64_EXACT forces over full lists, or FP64 over their lower halves
+// with FP64 reductions into cleared fields (newton; no kick) (xnb_force_pairs.cu).
+int launch_force_pairs(const Extent& ex, const SysDesc* sys, const SysState* st, const DevArrays& a, int precision,
+                       bool newton, bool with_pe, bool second_half, int sys_only, cudaStream_t stream);
+
 // Compact list entries of the flagged systems after a build, and the staged
 // mixed force traversal (+ kick) over the cell segments (xnb_force_staged.cu).
 // all = true: every resident system's current lists (when the staged form is switched on)

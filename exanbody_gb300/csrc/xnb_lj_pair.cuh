@@ -107,20 +107,16 @@ __device__ __forceinline__ void mixed_pair(const SysDesc& S, uint32_t e, double 
 // stream in (cell_enc, p_b) order with dr = r_b - r_a and keeps 0 < d2 <= rc^2;
 // LennardJonesForceFunctor (contribs/md/lennard_jones/lennard_jones.cu:67-102)
 // sums pair_de*dr sequentially and adds the sum onto the zeroed force.
-// One thread per particle, full lists: no atomics, fixed summation order.
-//   P = kFp64Exact : the functor's own operations and roundings (sqrt, 1/r,
-//                    no contraction): bit-identical to the CPU restatement.
-//   P = kFp64      : same selection of pairs (exact d2 test), force from
-//                    1/d2 by Newton-Raphson, FMA accumulation.
-//   P = kMixed     : raw entries (the functor forms the displacement): FP64
-//                    displacement and FP64 accumulation; r^2, r^-6 and the
-//                    force magnitude in FP32; the cutoff decision is made in
-//                    FP32 where a proven margin allows and in FP64 otherwise, so
-//                    the pair set is the FP64 one. The displacement is applied
-//                    once per particle (sum pd*r_b - r_a*sum pd, all in FP64)
-//                    and the FP32 factor is widened on the integer pipes: a
-//                    pair costs 3 DFMA + 1 DADD on the FP64 pipe.
-template <int P, bool PE, bool KICK, bool PACKED = true>
+// One thread per particle, full lists: no atomics, fixed summation order. The
+// mixed path takes raw entries (the functor forms the displacement): FP64
+// displacement and FP64 accumulation; r^2, r^-6 and the force magnitude in FP32;
+// the cutoff decision is made in FP32 where a proven margin allows and in FP64
+// otherwise, so the pair set is the FP64 one. The displacement is applied once
+// per particle (sum pd*r_b - r_a*sum pd, all in FP64) and the FP32 factor is
+// widened on the integer pipes: a pair costs 3 DFMA + 1 DADD on the FP64 pipe.
+// (The FP64 paths: xnb_force_pairs.cuh; small mixed batches, with these bits:
+// xnb_force_mixed.cu.)
+template <bool PE, bool KICK, bool PACKED = true>
 struct LJForce {
   const SysDesc* __restrict__ sys;
   DevArrays a;
@@ -137,36 +133,6 @@ struct LJForce {
     q.fx = q.fy = q.fz = q.pe = q.psum = 0.0;
     return true;
   }
-  __device__ __forceinline__ void pair(Acc& q, const pair::ParticleContext& c, const pair::PairData& p) const {
-    const SysDesc& S = sys[c.sys];
-    if (P == kFp64Exact) {
-      // lj_compute_energy (lennard_jones.cu:46-56) then pair_de *= w / r with w = 1
-      const double r = __dsqrt_rn(p.d2);
-      const double inv_r = __ddiv_rn(1.0, r);
-      const double ratio = __dmul_rn(S.sigma, inv_r);
-      const double ratio2 = __dmul_rn(ratio, ratio);
-      const double ratio6 = __dmul_rn(__dmul_rn(ratio2, ratio2), ratio2);
-      const double ratio12 = __dmul_rn(ratio6, ratio6);
-      double de = __dmul_rn(__dmul_rn(S.m24eps, __dsub_rn(__dmul_rn(2.0, ratio12), ratio6)), inv_r);
-      de = __dmul_rn(de, inv_r);
-      q.fx = __dadd_rn(q.fx, __dmul_rn(de, p.dx));
-      q.fy = __dadd_rn(q.fy, __dmul_rn(de, p.dy));
-      q.fz = __dadd_rn(q.fz, __dmul_rn(de, p.dz));
-      if (PE) {
-        const double en = __dmul_rn(S.eps4, __dsub_rn(ratio12, ratio6));
-        q.pe = __dadd_rn(q.pe, __dmul_rn(0.5, __dsub_rn(en, S.e_shift)));
-      }
-    } else {
-      const double ir2 = rcp_nr(p.d2);
-      const double s2 = S.sig2 * ir2;
-      const double s6 = s2 * s2 * s2;
-      const double pd = S.eps24 * s6 * fma(-2.0, s6, 1.0) * ir2;
-      q.fx = fma(pd, p.dx, q.fx);
-      q.fy = fma(pd, p.dy, q.fy);
-      q.fz = fma(pd, p.dz, q.fz);
-      if (PE) q.pe += 0.5 * fma(S.eps4 * s6, s6 - 1.0, -S.e_shift);
-    }
-  }
   __device__ __forceinline__ void entry(Acc& q, const pair::ParticleContext& c, const pair::RawEntry& r) const {
     const SysDesc& S = sys[c.sys];
     mixed_pair<PE, PACKED>(S, r.e, r.xb, r.yb, r.zb, r.hb, r.lb, c.x, c.y, c.z, c.hi, c.lo, S.rcut2, q.fx, q.fy,
@@ -182,19 +148,9 @@ struct LJForce {
   __device__ __forceinline__ void stop(Acc& q, const pair::ParticleContext& c) const {
     const SysDesc& S = sys[c.sys];
     const uint32_t i = c.i;
-    double fx = q.fx, fy = q.fy, fz = q.fz;
-    if (P == kMixed) {
-      fx = fma(-c.x, q.psum, fx);
-      fy = fma(-c.y, q.psum, fy);
-      fz = fma(-c.z, q.psum, fz);
-    }
-    // the force field was zeroed (zero_particle_force.cu:39-46) and receives the
-    // sum; 0 + s differs from s only for s = -0, which the exact path keeps
-    if (P == kFp64Exact) {
-      fx = __dadd_rn(0.0, fx);
-      fy = __dadd_rn(0.0, fy);
-      fz = __dadd_rn(0.0, fz);
-    }
+    double fx = fma(-c.x, q.psum, q.fx);
+    double fy = fma(-c.y, q.psum, q.fy);
+    double fz = fma(-c.z, q.psum, q.fz);
     if (S.divide_by_mass) {
       // divide_force_by_type_scalar (compute/vec3_typescalar_op.cu:156, math_functors.h:140)
       fx = __ddiv_rn(fx, S.mass);
@@ -208,15 +164,9 @@ struct LJForce {
     if (KICK) {
       // verlet_second_half: push_f_v with dt_scale 0.5 (numerical-scheme.msp:17-18)
       const double h = S.dt_half;
-      if (P == kFp64Exact) {
-        a.vx[i] = __dadd_rn(a.vx[i], __dmul_rn(fx, h));
-        a.vy[i] = __dadd_rn(a.vy[i], __dmul_rn(fy, h));
-        a.vz[i] = __dadd_rn(a.vz[i], __dmul_rn(fz, h));
-      } else {
-        a.vx[i] = fma(fx, h, a.vx[i]);
-        a.vy[i] = fma(fy, h, a.vy[i]);
-        a.vz[i] = fma(fz, h, a.vz[i]);
-      }
+      a.vx[i] = fma(fx, h, a.vx[i]);
+      a.vy[i] = fma(fy, h, a.vy[i]);
+      a.vz[i] = fma(fz, h, a.vz[i]);
     }
   }
 };
@@ -225,16 +175,14 @@ struct LJForce {
 
 namespace xnb {
 namespace pair {
-// The mixed path takes raw entries (their residuals come packed with the hi
-// mirror, so the residual mirrors are gathered only without packing), two per
-// iteration (both entries' gathers in flight together; list order unchanged);
-// the FP64 paths take the traversal's FP64 pairs within rc.
-template <int P, bool PE, bool KICK, bool PACKED>
-struct ComputePairTraits<LJForce<P, PE, KICK, PACKED>> : DefaultPairTraits {
-  static constexpr bool RawEntries = (P == kMixed);
-  static constexpr bool GatherMirrors = (P == kMixed && !PACKED);
-  static constexpr int EntriesPerIteration = (P == kMixed) ? 2 : 1;
+// Raw entries (their residuals come packed with the hi mirror, so the residual
+// mirrors are gathered only without packing), two per iteration (both entries'
+// gathers in flight together; list order unchanged).
+template <bool PE, bool KICK, bool PACKED>
+struct ComputePairTraits<LJForce<PE, KICK, PACKED>> : DefaultPairTraits {
+  static constexpr bool RawEntries = true;
+  static constexpr bool GatherMirrors = !PACKED;
+  static constexpr int EntriesPerIteration = 2;
 };
 }  // namespace pair
 }  // namespace xnb
-

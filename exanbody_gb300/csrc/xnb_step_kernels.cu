@@ -2,6 +2,7 @@
 // Lennard-Jones pair-force traversal over the neighbour lists.
 #include <algorithm>
 
+#include "xnb_force_pairs.cuh"
 #include "xnb_grid_barrier.cuh"
 #include "xnb_launch.cuh"
 #include "xnb_lj_pair.cuh"
@@ -144,19 +145,19 @@ __global__ void __launch_bounds__(256)
 
 // 72 registers: 7 blocks of 128 threads per SM (measured faster than the
 // unconstrained 79 despite a few spilled bytes).
-template <int P, bool PE, bool KICK, bool PACKED = true>
-__global__ void __maxnreg__(72) k_force(uint32_t n_part, BatchSource src, LJForce<P, PE, KICK, PACKED> f) {
+template <bool PE, bool KICK, bool PACKED = true>
+__global__ void __maxnreg__(72) k_force(uint32_t n_part, BatchSource src, LJForce<PE, KICK, PACKED> f) {
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n_part; i += gridDim.x * blockDim.x)
     pair::traverse_particle(src, i, f);
 }
 
-// LANES threads per particle (FP64 and mixed): each takes every LANES-th
+// LANES threads per particle: each takes every LANES-th
 // 8-entry block of the particle's list and the partial sums are combined in a
 // fixed order, so the result is reproducible (it agrees with the one-lane
 // traversal to rounding). The whole warp iterates together: the shuffles of
 // the combination span it.
-template <int P, bool PE, bool KICK, int LANES>
-__global__ void __maxnreg__(72) k_force_lanes(uint32_t n_part, BatchSource src, LJForce<P, PE, KICK> f) {
+template <bool PE, bool KICK, int LANES>
+__global__ void __maxnreg__(72) k_force_lanes(uint32_t n_part, BatchSource src, LJForce<PE, KICK> f) {
   const uint64_t total = static_cast<uint64_t>(n_part) * LANES;
   const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
   for (uint64_t base = static_cast<uint64_t>(blockIdx.x) * blockDim.x; base < total; base += stride) {
@@ -173,10 +174,9 @@ __global__ void __maxnreg__(72) k_force_lanes(uint32_t n_part, BatchSource src, 
 // reduction in L2. Each pair inside rc is evaluated once. The order in which
 // reactions arrive varies from run to run, so results agree to rounding, not
 // bit for bit; FP64_EXACT always uses the full-list kernel above.
-// FAR: instantiated only when a system of the batch lies far from the
-// coordinate origin (Extent::far_coords), so the common kernel carries no
-// partner-side evaluation.
-template <int P, bool PE, bool FAR = false>
+// kFp64 runs it only when a system of the batch lies far from the coordinate
+// origin (Extent::far_coords; the common case is launch_force_pairs).
+template <int P, bool PE>
 __global__ void __launch_bounds__(256)
     k_force_half(uint32_t n_part, const SysDesc* __restrict__ sys, const SysState* __restrict__ st, DevArrays a,
                  int sys_only) {
@@ -227,7 +227,7 @@ __global__ void __launch_bounds__(256)
         yb = image_coord(yb, py, static_cast<int>((code / 3u) % 3u));
         zb = image_coord(zb, pz, static_cast<int>(code / 9u));
       }
-      if (FAR && P == kFp64 && code != static_cast<uint32_t>(kImageCenter) && S.far_coords) {
+      if (P == kFp64 && code != static_cast<uint32_t>(kImageCenter) && S.far_coords) {
         // Far from the coordinate origin (coordinates beyond 4 periods) the
         // partner's reaction through a periodic image is evaluated as the
         // partner's own full-list traversal would: b sees a through the
@@ -423,34 +423,25 @@ inline int grid_capped(uint32_t n, int threads, int sm_count, int per_sm) {
   return static_cast<int>(g < 1 ? 1 : g);
 }
 
-template <int P, bool PE, bool KICK>
+template <bool PE, bool KICK>
 void force_dispatch(const Extent& ex, const SysDesc* sys, const SysState* st, const DevArrays& a, int sys_only,
                     cudaStream_t stream) {
   const int threads = ex.force_block > 0 ? ex.force_block : 64;
   const BatchSource src(sys, st, a, sys_only);
-  if constexpr (P == kMixed) {
-    // a batch holding a box of X >= 1024 sigma: residual mirrors gathered, one thread per particle
-    if (ex.unpacked) {
-      const LJForce<P, PE, KICK, false> fu{sys, a};
-      k_force<P, PE, KICK, false><<<grid_for(ex.n_part, threads), threads, 0, stream>>>(ex.n_part, src, fu);
-      return;
-    }
+  // a batch holding a box of X >= 1024 sigma: residual mirrors gathered, one thread per particle
+  if (ex.unpacked) {
+    const LJForce<PE, KICK, false> fu{sys, a};
+    k_force<PE, KICK, false><<<grid_for(ex.n_part, threads), threads, 0, stream>>>(ex.n_part, src, fu);
+    return;
   }
-  const LJForce<P, PE, KICK> f{sys, a};
-  // the bit-exact path keeps one thread per particle (the reference's summation order)
-  if constexpr (P != kFp64Exact) {
-    if (ex.force_lanes == 2) {
-      k_force_lanes<P, PE, KICK, 2><<<grid_for(ex.n_part * 2u, threads), threads, 0, stream>>>(ex.n_part, src, f);
-      return;
-    }
-    if (ex.force_lanes == 4) {
-      k_force_lanes<P, PE, KICK, 4><<<grid_for(ex.n_part * 4u, threads), threads, 0, stream>>>(ex.n_part, src, f);
-      return;
-    }
-  }
-  k_force<P, PE, KICK><<<grid_for(ex.n_part, threads), threads, 0, stream>>>(ex.n_part, src, f);
+  const LJForce<PE, KICK> f{sys, a};
+  if (ex.force_lanes == 2)
+    k_force_lanes<PE, KICK, 2><<<grid_for(ex.n_part * 2u, threads), threads, 0, stream>>>(ex.n_part, src, f);
+  else if (ex.force_lanes == 4)
+    k_force_lanes<PE, KICK, 4><<<grid_for(ex.n_part * 4u, threads), threads, 0, stream>>>(ex.n_part, src, f);
+  else
+    k_force<PE, KICK><<<grid_for(ex.n_part, threads), threads, 0, stream>>>(ex.n_part, src, f);
 }
-
 
 // ---------------------------------------------------------------------------
 // Persistent step loop: one cooperative launch advances the batch step after
@@ -466,7 +457,7 @@ void force_dispatch(const Extent& ex, const SysDesc* sys, const SysState* st, co
 template <bool EXACT, int P, bool PE, bool PACKED = true>
 __global__ void __maxnreg__(72)
     k_steps_persistent(uint32_t n_part, int nsys, const SysDesc* __restrict__ sys, SysState* __restrict__ st,
-                       DevArrays a, BatchSource src, LJForce<P, PE, true, PACKED> f, StepCtl* ctl, int max_steps,
+                       DevArrays a, BatchSource src, LJForce<PE, true, PACKED> f, StepCtl* ctl, int max_steps,
                        unsigned int nblocks, unsigned long long wait_ns, bool check) {
   if (check && !grid_barrier(&ctl->bar, nblocks + 1u, wait_ns)) return;
   for (int k = 0; k < max_steps; ++k) {
@@ -479,8 +470,15 @@ __global__ void __maxnreg__(72)
       }
       return;
     }
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n_part; i += gridDim.x * blockDim.x)
-      pair::traverse_particle(src, i, f);
+    if constexpr (P == kMixed) {
+      for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n_part; i += gridDim.x * blockDim.x)
+        pair::traverse_particle(src, i, f);
+    } else {
+      __shared__ pairs::WarpSmem sm[4];  // blocks of 4 warps
+      const uint32_t w = threadIdx.x >> 5;
+      for (uint32_t first = (blockIdx.x * 4u + w) * pairs::kPer; first < n_part; first += gridDim.x * 4u * pairs::kPer)
+        pairs::eight_particles<P, PE, true, false>(first, n_part, src, a, sm[w]);
+    }
     if (blockIdx.x == 0 && threadIdx.x == 0) ctl->fired[(k + 1) & 1] = 0u;
     if (!grid_barrier(&ctl->bar, nblocks, wait_ns)) return;
   }
@@ -514,7 +512,7 @@ int persistent_launch(const Extent& ex, const SysDesc* sys, SysState* st, const 
   // a barrier waits at most 4 s in a run (a phase of the largest batches lasts
   // milliseconds), 20 ms in the timeout check
   const unsigned long long wait_ns = check ? 20000000ull : 4000000000ull;
-  LJForce<P, PE, true, PACKED> f{sys, a};
+  LJForce<PE, true, PACKED> f{sys, a};
   cudaLaunchKernelEx(&cfg, kern, ex.n_part, ex.nsys, sys, st, a, BatchSource(sys, st, a, -1), f, ctl, max_steps,
                      grid, wait_ns, check);
   return 1;
@@ -544,9 +542,8 @@ int launch_force(const Extent& ex, const SysDesc* sys, SysState* st, const DevAr
     const int g = grid_capped(ex.n_part, threads, ex.sm_count, 8);
     k_zero_force<<<g, threads, 0, stream>>>(ex.n_part, st, a, sys_only, with_pe);
     if (precision == kFp64) {
-      if (ex.far_coords) {
-        if (with_pe) k_force_half<kFp64, true, true><<<g, threads, 0, stream>>>(ex.n_part, sys, st, a, sys_only);
-        else k_force_half<kFp64, false, true><<<g, threads, 0, stream>>>(ex.n_part, sys, st, a, sys_only);
+      if (!ex.far_coords) {
+        launch_force_pairs(ex, sys, st, a, precision, true, with_pe, false, sys_only, stream);
       } else {
         if (with_pe) k_force_half<kFp64, true><<<g, threads, 0, stream>>>(ex.n_part, sys, st, a, sys_only);
         else k_force_half<kFp64, false><<<g, threads, 0, stream>>>(ex.n_part, sys, st, a, sys_only);
@@ -562,19 +559,13 @@ int launch_force(const Extent& ex, const SysDesc* sys, SysState* st, const DevAr
     return launch_force_staged(ex, sys, st, a, with_pe, second_half, sys_only, stream);
   if (precision == kMixed && !ex.unpacked && ex.n_part <= kMixedSplitMax)
     return launch_force_mixed(ex, sys, st, a, with_pe, second_half, sys_only, stream);
-#define XNB_FORCE_CASE(PP)                                                           \
-  if (precision == PP) {                                                             \
-    if (with_pe && second_half) force_dispatch<PP, true, true>(ex, sys, st, a, sys_only, stream);   \
-    else if (with_pe) force_dispatch<PP, true, false>(ex, sys, st, a, sys_only, stream);            \
-    else if (second_half) force_dispatch<PP, false, true>(ex, sys, st, a, sys_only, stream);        \
-    else force_dispatch<PP, false, false>(ex, sys, st, a, sys_only, stream);                        \
-    return 1;                                                                        \
-  }
-  XNB_FORCE_CASE(kFp64Exact)
-  XNB_FORCE_CASE(kFp64)
-  XNB_FORCE_CASE(kMixed)
-#undef XNB_FORCE_CASE
-  return 0;
+  if (precision != kMixed)
+    return launch_force_pairs(ex, sys, st, a, precision, false, with_pe, second_half, sys_only, stream);
+  if (with_pe && second_half) force_dispatch<true, true>(ex, sys, st, a, sys_only, stream);
+  else if (with_pe) force_dispatch<true, false>(ex, sys, st, a, sys_only, stream);
+  else if (second_half) force_dispatch<false, true>(ex, sys, st, a, sys_only, stream);
+  else force_dispatch<false, false>(ex, sys, st, a, sys_only, stream);
+  return 1;
 }
 
 int launch_mark_rebuild(const Extent& ex, SysState* st, int mode, int sys_only, unsigned int* any,
