@@ -30,6 +30,15 @@ struct SnapZ {
   uint32_t cg;  // offset of the (j1, j2, j) Clebsch-Gordan block [m1][m2]
 };
 
+// 32 tasks of the FP64 kernel's Z, one per lane: sums of products of U_tot
+// elements for nj values of j (offsets in units of 32 lanes).
+struct SnapBatch {
+  uint32_t idx, coef, out;  // first index line, coefficient line and output line
+  uint32_t n, nj;           // products per lane (0: no batch); values of j
+};
+constexpr int kSnapMaxJ = 3;          // values of j per task
+constexpr int kSnapMaxProducts = 16;  // products per task
+
 struct SnapArgs {
   int twojmax, nz, nu_unique, nu_full, ntypes, switchflag;
   int group, group_f;          // neighbours per round (shared-memory budget), FP64 / FP32 kernels
@@ -39,12 +48,18 @@ struct SnapArgs {
   double radelem[kSnapMaxTypes], wj[kSnapMaxTypes];
   double e0[kSnapMaxTypes];    // beta_0 - sum_k beta_k bzero_k per type
   double energy_unit;
-  const double* rootpq;        // [(J+1)^2], sqrt(p/q)
-  const double* cg;
+  // FP64 kernel
+  int n_batch, n_out;
+  const SnapBatch* batch;      // n_batch, warp w takes w, w + kSnapWarps, ...
+  const uint32_t* zidx;        // per product line: U_tot elements of each lane (16 bits each)
+  const double* zc;            // per product line and j: coefficients
+  const uint32_t* zout;        // per output line: unique and full index of the element (16 bits each), ~0 for none
+  const double *ztb, *zte;     // [ntypes][n_out lines]: multiplier of Z into Y; 2 w beta_k of canonical entries, else 0
+  const double *scale, *yscale;  // nu_unique: scale of an element; the same with the weight of the unique half
+  // FP32 kernel (mixed path)
   const SnapZ* z;              // nz
-  const double* zbeta;         // [ntypes][nz] multiplier of Z into Y
-  const double* zener;         // [ntypes][nz] 2 w beta_k of canonical entries, else 0
-  const float *rootpq_f, *cg_f, *zbeta_f, *zener_f;  // the same tables in FP32 (mixed path)
+  const float *rootpq_f;       // [(J+1)^2], sqrt(p/q)
+  const float *cg_f, *zbeta_f, *zener_f;  // [ntypes][nz], as ztb and zte
   size_t smem_bytes, smem_bytes_f;
 };
 
