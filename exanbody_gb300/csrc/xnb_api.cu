@@ -347,6 +347,18 @@ SysDesc make_desc(const xnb_lj_params& p) {
     d.image_tie_f = std::nextafter(
         static_cast<float>(2.0 * (16.0 * X * std::ldexp(1.0, -48) + 4.0 * (O + X) * std::ldexp(1.0, -53))), 1.0f);
   }
+  {
+    // Force factors pd of a fluid lie within a few powers of two of 24 eps /
+    // sigma^2 = 2^E: with Q = 2^(E - 44) every |pd| >= 2^(E - 21) is a multiple of
+    // Q, and sums of |pd| up to 2^(E + 8) = 2^52 Q are exact in FP64.
+    const double scale = d.sig2 > 0.0 ? std::fabs(d.eps24) / d.sig2 : 0.0;
+    int e = 1;
+    if (std::isfinite(scale) && scale > 1e-30 && scale < 1e30) std::frexp(scale, &e);
+    const int E = e - 1;
+    d.psum_quantum = std::ldexp(1.0, E - 44);
+    d.psum_exp = E + 106;  // 127 + 23 + (E - 44)
+    d.psum_max_f = std::ldexp(1.0f, E + 8);
+  }
   // FP32 cell index of the rebin: the mirror pf = fl32(x - origin) and
   // fl32(1/cell_size) put pf * inv within 3.01 u |q| of the quotient q of the
   // reference's division (|q| <= max dims + 2 before wrapping); a fraction farther

@@ -35,35 +35,6 @@ struct Row {
 };
 constexpr uint32_t kNone = 0xFFFFFFFFu;
 
-// The packed residual fields as FP32 numbers (a 10-bit field, its sign bit
-// flipped, under the exponent of 2^23): differences are exact, q_b - q_a for x
-// and z, 1024 (q_b - q_a) for y.
-__device__ __forceinline__ float field_x(uint32_t w) { return __uint_as_float((w & 0x3FFu) ^ 0x4B000200u); }
-__device__ __forceinline__ float field_y(uint32_t w) { return __uint_as_float((w & 0xFFC00u) ^ 0x4B080000u); }
-__device__ __forceinline__ float field_z(uint32_t w) { return __uint_as_float((w >> 20) ^ 0x4B000200u); }
-
-// One axis of an image entry's displacement in FP32 pairs: hi_b - hi_a by
-// TwoDiff (Knuth), the image offset added to its high part (exact: the two are
-// within a factor of two of each other), the small parts summed. The rounded
-// sum is the FP64 displacement's FP32 rounding unless its remainder lies within
-// `tie` (the bound on both errors) of half an ulp: those entries take FP64.
-__device__ __forceinline__ float image_axis(float hb, float ha, float lb, float la, uint32_t digit, float p, float pl,
-                                            float tie, bool& sure) {
-  const float s = __fadd_rn(hb, -ha);
-  const float t = __fadd_rn(s, -hb);
-  const float err = __fadd_rn(__fadd_rn(hb, -__fadd_rn(s, -t)), -__fadd_rn(ha, t));
-  const float sh = digit == 1u ? 0.f : (digit == 2u ? p : -p), sl = digit == 1u ? 0.f : (digit == 2u ? pl : -pl);
-  const float hi = __fadd_rn(s, sh);
-  const float rest = __fadd_rn(__fadd_rn(err, sl), __fadd_rn(lb, -la));
-  const float d = __fadd_rn(hi, rest);
-  const float lo = __fadd_rn(__fadd_rn(hi, -d), rest);
-  const uint32_t ex = __float_as_uint(d) & 0x7f800000u;
-  const float half = __uint_as_float(ex - (24u << 23));  // half an ulp of d (ex checked below)
-  sure = sure && ex > (40u << 23) && fabsf(__fadd_rn(fabsf(lo), -half)) > tie &&
-         fabsf(__fadd_rn(fabsf(lo), -0.5f * half)) > tie;
-  return d;
-}
-
 template <bool PE, bool KICK>
 __global__ void __launch_bounds__(256, 4)
     k_force_mixed(uint32_t n_part, BatchSource src, DevArrays a, uint32_t group, uint32_t chunk) {

@@ -80,6 +80,9 @@ struct SysDesc {
   float sub_reach_f;             // nbh_dist / cell_size widened by 1e-5: reach of the sub-cell box test (cells)
   float lo_step_f, lo_inv_f;     // quantum of the residual packed in DevArrays::pf.w (ulp(X)/1024) and its inverse
   float period_lo_f[3];          // period - period_f, rounded: the image offset in two FP32 words
+  double psum_quantum;           // Q of the exact sum of the mixed force factors (PairSum)
+  int32_t psum_exp;              // FP32 exponent field of 2^23 Q
+  float psum_max_f;              // 2^52 Q
   float image_tie_f;             // bound on the error of an image displacement formed from FP32 pairs
   int32_t packed_lo;             // 1: the mixed traversal reads the packed residuals (X < 1024); 0: DevArrays::pflo
   double inv_cell;               // fl(1/cell_size): reciprocal pre-decision of the backup encoding

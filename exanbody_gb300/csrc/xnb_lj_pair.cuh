@@ -31,19 +31,87 @@ __device__ __forceinline__ double rcp_nr(double d) {
   return fma(y, e, y);
 }
 
+// Sum of the FP32 force factors pd of one particle, as FP64 additions in list
+// order would give it, without the FP64 pipe: every pd is a multiple of a
+// quantum Q, 2^23 Q <= |pd| < 2^53 Q, and while the sum of |pd| stays within 2^52 Q
+// every partial sum is exact in FP64, so the sum is Q times the integer sum of
+// pd / Q in any order. A pd outside that range (near the zero crossing of the
+// force, some 10^-5 of the particles) sets `inexact`: that particle is summed in
+// FP64, in order. An FP64 instruction holds a quarter of an SM's FP64 pipe for 64
+// cycles; these are about twelve on the integer pipes.
+struct PairSum {
+  long long units;  // sum of pd / Q
+  float size;       // sum of |pd|
+  bool inexact;
+
+  __device__ __forceinline__ void clear() {
+    units = 0;
+    size = 0.f;
+    inexact = false;
+  }
+  __device__ __forceinline__ void add(const SysDesc& S, float pd) {
+    const uint32_t u = __float_as_uint(pd);
+    const int shift = static_cast<int>((u >> 23) & 0xFFu) - S.psum_exp;
+    inexact = inexact || static_cast<unsigned>(shift) > 29u;
+    const int mantissa = static_cast<int>((u & 0x007fffffu) | 0x00800000u);
+    const int power = 1 << (shift & 31);
+    units += static_cast<long long>(mantissa) * static_cast<long long>((u >> 31) ? -power : power);
+    size += fabsf(pd);
+  }
+  __device__ __forceinline__ void combine(const PairSum& o) {
+    units += o.units;
+    size += o.size;
+    inexact = inexact || o.inexact;
+  }
+  // (a NaN size is not exact)
+  __device__ __forceinline__ bool exact(const SysDesc& S) const { return !inexact && size <= S.psum_max_f; }
+  __device__ __forceinline__ double value(const SysDesc& S) const {
+    return __dmul_rn(static_cast<double>(units), S.psum_quantum);
+  }
+};
+
+// The packed residual fields as FP32 numbers (a 10-bit field, its sign bit
+// flipped, under the exponent of 2^23): differences are exact, q_b - q_a for x
+// and z, 1024 (q_b - q_a) for y.
+__device__ __forceinline__ float field_x(uint32_t w) { return __uint_as_float((w & 0x3FFu) ^ 0x4B000200u); }
+__device__ __forceinline__ float field_y(uint32_t w) { return __uint_as_float((w & 0xFFC00u) ^ 0x4B080000u); }
+__device__ __forceinline__ float field_z(uint32_t w) { return __uint_as_float((w >> 20) ^ 0x4B000200u); }
+
+// One axis of an image entry's displacement in FP32 pairs: hi_b - hi_a by
+// TwoDiff (Knuth), the image offset added to its high part (exact: the two are
+// within a factor of two of each other), the small parts summed. The rounded
+// sum is the FP64 displacement's FP32 rounding unless its remainder lies within
+// `tie` (the bound on both errors) of half an ulp: those entries take FP64.
+__device__ __forceinline__ float image_axis(float hb, float ha, float lb, float la, uint32_t digit, float p, float pl,
+                                            float tie, bool& sure) {
+  const float s = __fadd_rn(hb, -ha);
+  const float t = __fadd_rn(s, -hb);
+  const float err = __fadd_rn(__fadd_rn(hb, -__fadd_rn(s, -t)), -__fadd_rn(ha, t));
+  const float sh = digit == 1u ? 0.f : (digit == 2u ? p : -p), sl = digit == 1u ? 0.f : (digit == 2u ? pl : -pl);
+  const float hi = __fadd_rn(s, sh);
+  const float rest = __fadd_rn(__fadd_rn(err, sl), __fadd_rn(lb, -la));
+  const float d = __fadd_rn(hi, rest);
+  const float lo = __fadd_rn(__fadd_rn(hi, -d), rest);
+  const uint32_t ex = __float_as_uint(d) & 0x7f800000u;
+  const float half = __uint_as_float(ex - (24u << 23));  // half an ulp of d (ex checked below)
+  sure = sure && ex > (40u << 23) && fabsf(__fadd_rn(fabsf(lo), -half)) > tie &&
+         fabsf(__fadd_rn(fabsf(lo), -0.5f * half)) > tie;
+  return d;
+}
+
 // One marked entry of the mixed path: r^2 in FP32 (the compensated mirror
 // difference for an entry in the same periodic image: hi difference plus the
 // difference of the residuals packed in .w; the FP64 displacement converted for
 // an image entry), the cutoff decided in FP32 outside the proven band and in
-// FP64 inside it, then the FP32 force factor pd and the FP64 accumulation of
-// pd * r_b and pd.
+// FP64 inside it, then the FP32 force factor pd, the FP64 accumulation of pd * r_b
+// and the exact one of pd.
 // PACKED = false (batches holding a system of X >= 1024 sigma, whose packed
 // residuals are too coarse) takes the gathered residual mirrors lb and pal.
 template <bool PE, bool PACKED>
 __device__ __forceinline__ void mixed_pair(const SysDesc& S, uint32_t e, double xb, double yb, double zb, float4 hb,
                                            float4 lb, double xa, double ya, double za, float4 paf, float4 pal,
-                                           double rcut2, double& fx, double& fy, double& fz, double& psum,
-                                           double& pe) {
+                                           double rcut2, double& fx, double& fy, double& fz, PairSum& psum,
+                                           double& pe, float* factor = nullptr) {
   const uint32_t code = e & 31u;
   float dxf, dyf, dzf;
   if (code == static_cast<uint32_t>(kImageCenter)) {
@@ -81,7 +149,7 @@ __device__ __forceinline__ void mixed_pair(const SysDesc& S, uint32_t e, double 
   if (in) {
     // FP64 displacement folded into the FP64 accumulation:
     //   sum_b pd_b (r_b - r_a) = sum_b pd_b r_b - r_a sum_b pd_b,
-    // so a pair costs 3 DFMA + 1 DADD instead of 3 DADD + 3 DFMA; the
+    // so a pair costs 3 DFMA instead of 3 DADD + 3 DFMA; the
     // subtraction happens once per particle (cancellation error
     // <= ~u_64 |r| sum|pd|, about 1e-12 of |F| at box sizes of 10^3 sigma).
     // The hardware reciprocal (within 1 ulp) is part of the FP32 force magnitude.
@@ -94,8 +162,60 @@ __device__ __forceinline__ void mixed_pair(const SysDesc& S, uint32_t e, double 
     fx = fma(pdd, xb, fx);
     fy = fma(pdd, yb, fy);
     fz = fma(pdd, zb, fz);
-    psum += pdd;
+    psum.add(S, pd);
+    if (factor) *factor = pd;
     if (PE) pe += static_cast<double>(0.5f * fmaf(S.eps4_f * s6, s6 - 1.0f, -S.e_shift_f));
+  }
+}
+
+// Sum of pd in FP64, in list order (where PairSum is not exact).
+template <bool PACKED>
+static __device__ __noinline__ double psum_in_order(const SysDesc& S, const double* rx, const double* ry,
+                                                    const double* rz, const float4* pf, const float4* pflo, uint32_t i,
+                                                    const uint32_t* list, uint32_t n) {
+  const double xa = rx[i], ya = ry[i], za = rz[i];
+  const float4 hi = pf[i], lo = PACKED ? make_float4(0.f, 0.f, 0.f, 0.f) : pflo[i];
+  double psum = 0.0;
+  for (uint32_t k = 0; k < n; ++k) {
+    const uint32_t e = list[k], j = S.part_base + (e >> 5);
+    double fx = 0.0, fy = 0.0, fz = 0.0, pe = 0.0;
+    PairSum one;
+    one.clear();
+    float pd = 0.f;
+    mixed_pair<false, PACKED>(S, e, rx[j], ry[j], rz[j], pf[j], PACKED ? make_float4(0.f, 0.f, 0.f, 0.f) : pflo[j], xa,
+                              ya, za, hi, lo, S.rcut2, fx, fy, fz, one, pe, &pd);
+    psum += widen_f32_fast(pd);
+  }
+  return psum;
+}
+
+// A particle's sums to its force (and energy): the FP64 displacement folded out
+// of sum pd (r_b - r_a), the division by the mass, the second-half kick.
+template <bool PE, bool KICK, bool PACKED>
+__device__ __forceinline__ void finish_mixed(const SysDesc& S, const DevArrays& a, uint32_t i, const uint32_t* list,
+                                             uint32_t n, double fx, double fy, double fz, const PairSum& sum,
+                                             double pe) {
+  const double psum = sum.exact(S) ? sum.value(S)
+                                   : psum_in_order<PACKED>(S, a.rx, a.ry, a.rz, a.pf, a.pflo, i, list, n);
+  fx = fma(-a.rx[i], psum, fx);
+  fy = fma(-a.ry[i], psum, fy);
+  fz = fma(-a.rz[i], psum, fz);
+  if (S.divide_by_mass) {
+    // divide_force_by_type_scalar (compute/vec3_typescalar_op.cu:156, math_functors.h:140)
+    fx = __ddiv_rn(fx, S.mass);
+    fy = __ddiv_rn(fy, S.mass);
+    fz = __ddiv_rn(fz, S.mass);
+  }
+  a.fx[i] = fx;
+  a.fy[i] = fy;
+  a.fz[i] = fz;
+  if (PE) a.pe[i] = pe;
+  if (KICK) {
+    // verlet_second_half: push_f_v with dt_scale 0.5 (numerical-scheme.msp:17-18)
+    const double h = S.dt_half;
+    a.vx[i] = fma(fx, h, a.vx[i]);
+    a.vy[i] = fma(fy, h, a.vy[i]);
+    a.vz[i] = fma(fz, h, a.vz[i]);
   }
 }
 
@@ -113,7 +233,8 @@ __device__ __forceinline__ void mixed_pair(const SysDesc& S, uint32_t e, double 
 // the cutoff decision is made in FP32 where a proven margin allows and in FP64
 // otherwise, so the pair set is the FP64 one. The displacement is applied once
 // per particle (sum pd*r_b - r_a*sum pd, all in FP64) and the FP32 factor is
-// widened on the integer pipes: a pair costs 3 DFMA + 1 DADD on the FP64 pipe.
+// widened, and summed (PairSum), on the integer pipes: a pair costs 3 DFMA on the
+// FP64 pipe.
 // (The FP64 paths: xnb_force_pairs.cuh; small mixed batches, with these bits:
 // xnb_force_mixed.cu.)
 template <bool PE, bool KICK, bool PACKED = true>
@@ -121,7 +242,8 @@ struct LJForce {
   const SysDesc* __restrict__ sys;
   DevArrays a;
   struct Acc {
-    double fx, fy, fz, pe, psum;
+    double fx, fy, fz, pe;
+    PairSum psum;
   };
 
   __device__ __forceinline__ double rcut2(const pair::ParticleContext& c) const { return sys[c.sys].rcut2; }
@@ -130,7 +252,8 @@ struct LJForce {
     return S.rc2_f + S.pre_margin_f;
   }
   __device__ __forceinline__ bool start(Acc& q, const pair::ParticleContext&) const {
-    q.fx = q.fy = q.fz = q.pe = q.psum = 0.0;
+    q.fx = q.fy = q.fz = q.pe = 0.0;
+    q.psum.clear();
     return true;
   }
   __device__ __forceinline__ void entry(Acc& q, const pair::ParticleContext& c, const pair::RawEntry& r) const {
@@ -143,31 +266,10 @@ struct LJForce {
     q.fy += o.fy;
     q.fz += o.fz;
     q.pe += o.pe;
-    q.psum += o.psum;
+    q.psum.combine(o.psum);
   }
   __device__ __forceinline__ void stop(Acc& q, const pair::ParticleContext& c) const {
-    const SysDesc& S = sys[c.sys];
-    const uint32_t i = c.i;
-    double fx = fma(-c.x, q.psum, q.fx);
-    double fy = fma(-c.y, q.psum, q.fy);
-    double fz = fma(-c.z, q.psum, q.fz);
-    if (S.divide_by_mass) {
-      // divide_force_by_type_scalar (compute/vec3_typescalar_op.cu:156, math_functors.h:140)
-      fx = __ddiv_rn(fx, S.mass);
-      fy = __ddiv_rn(fy, S.mass);
-      fz = __ddiv_rn(fz, S.mass);
-    }
-    a.fx[i] = fx;
-    a.fy[i] = fy;
-    a.fz[i] = fz;
-    if (PE) a.pe[i] = q.pe;
-    if (KICK) {
-      // verlet_second_half: push_f_v with dt_scale 0.5 (numerical-scheme.msp:17-18)
-      const double h = S.dt_half;
-      a.vx[i] = fma(fx, h, a.vx[i]);
-      a.vy[i] = fma(fy, h, a.vy[i]);
-      a.vz[i] = fma(fz, h, a.vz[i]);
-    }
+    finish_mixed<PE, KICK, PACKED>(sys[c.sys], a, c.i, c.list, c.n, q.fx, q.fy, q.fz, q.psum, q.pe);
   }
 };
 
