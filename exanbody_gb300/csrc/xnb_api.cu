@@ -122,12 +122,15 @@ struct xnb_batch {
     e.far_coords = 0;
     e.unpacked = 0;
     e.list_slot = 0;
+    e.dense = 0;
     for (size_t s = 0; s < sys.size(); ++s)
       if (sys[s].active) {
         hw = static_cast<int>(s) + 1;
         if (sys[s].d.far_coords) e.far_coords = 1;
         if (!sys[s].d.packed_lo) e.unpacked = 1;
         e.list_slot = std::max(e.list_slot, sys[s].d.list_slot);
+        const SysDesc& d = sys[s].d;
+        if (d.amr_enabled && 2ull * d.npart >= static_cast<uint64_t>(d.amr_min_n) * d.ncells) e.dense = 1;
       }
     e.nsys = hw;
     e.sm_count = sm_count;
@@ -1128,13 +1131,15 @@ int xnb_step(xnb_batch* b, int32_t nsteps, int32_t precision, int32_t flags, voi
   const bool exact = precision == XNB_PREC_FP64_EXACT;
   const bool energy = (flags & XNB_STEP_ENERGY) != 0;
   const bool fused = !(flags & XNB_STEP_HOST_SYNC) && fused_rebin_fits(ex);
+  const bool build = fused && fused_build_fits(ex, b->build_form, b->subcell_prune != 0);
   for (int k = 0; k < nsteps; ++k) {
     // verlet_first_half + trigger_move_particles
     b->launches += launch_first_half(ex, b->d_sys, b->d_st, b->a, true, true, true, 1.0, 0.5, exact, -1, st);
     if (fused) {
-      b->launches += launch_rebin_fused(ex, b->d_sys, b->d_st, b->a, exact, st);
-      b->launches += launch_neighbors(ex, b->d_sys, b->d_st, b->a, b->stage_cap, list_buf(b), st, b->build_form,
-                                      b->subcell_prune != 0, false);
+      b->launches += launch_rebin_fused(ex, b->d_sys, b->d_st, b->a, exact, build, b->stage_cap, list_buf(b), st);
+      if (!build)
+        b->launches += launch_neighbors(ex, b->d_sys, b->d_st, b->a, b->stage_cap, list_buf(b), st, b->build_form,
+                                        b->subcell_prune != 0, false);
       b->launches += launch_force(ex, b->d_sys, b->d_st, b->a, precision, energy, true, -1, st, newton);
       continue;
     }

@@ -154,12 +154,12 @@ __device__ __forceinline__ void rebin_compact(uint32_t n_cells, const SysDesc* _
     }
     __syncwarp();
     if (lane == 0) {
+      // the holes from the top (only they matter to the scan)
       uint32_t ncur = n;
-      for (int q = static_cast<int>(n) - 1; q >= 0; --q) {
-        if (a.plocal[start + q] == kInvalid) {
-          if (static_cast<uint32_t>(q) + 1 < ncur) a.plocal[start + q] = a.plocal[start + ncur - 1];
-          --ncur;
-        }
+      for (uint32_t m = nmov; m-- > 0;) {
+        const uint32_t q = a.mover_list[start + m] - start;
+        if (q + 1 < ncur) a.plocal[start + q] = a.plocal[start + ncur - 1];
+        --ncur;
       }
       a.cell_stay[c] = ncur;
       a.cell_nmov[c] = nmov;
@@ -475,83 +475,6 @@ __device__ __forceinline__ void scan_cells_one_block(const uint32_t* in, uint32_
   }
 }
 
-// The trigger's decision and the whole rebin (K_r1 .. K_r6, the resets of the
-// build that follows) of a small batch in one cooperative launch. A step without
-// a rebuild costs one launch that returns at once, where the separate kernels
-// cost twelve (0.7 us each inside a graph, 2.3 us when launched one by one); a
-// rebuild costs six grid barriers. The phases are the separate kernels' bodies.
-template <int BACKUP>
-__global__ void __launch_bounds__(256)
-    k_rebin_fused(uint32_t n_part, uint32_t n_cells, int nsys, const SysDesc* __restrict__ sys, SysState* st,
-                  DevArrays a) {
-  int flagged = 0;
-  for (int s = static_cast<int>(threadIdx.x); s < nsys; s += static_cast<int>(blockDim.x))
-    flagged |= __ldcg(&st[s].moved) != 0ull ? 1 : 0;
-  if (!__syncthreads_or(flagged)) {
-    if (blockIdx.x == 0) {
-      for (int s = static_cast<int>(threadIdx.x); s < nsys; s += static_cast<int>(blockDim.x)) st[s].rebuild = 0;
-      if (threadIdx.x == 0) *a.any_rebuild = 0;
-    }
-    return;
-  }
-  if (blockIdx.x == 0) {
-    // what the other blocks read before the first barrier is `moved` alone
-    unsigned int mine = 0;
-    for (int s = static_cast<int>(threadIdx.x); s < nsys; s += static_cast<int>(blockDim.x)) {
-      const bool r = __ldcg(&st[s].moved) != 0ull;
-      st[s].rebuild = r ? 1u : 0u;
-      if (!r) continue;
-      ++mine;
-      st[s].rebuilds += 1;
-      st[s].rebuild_armed = 1;
-      st[s].keys_fresh = 1;
-      // the build that follows (k_nbr_reset)
-      st[s].list_used = 0;
-      st[s].max_nbr = 0;
-      st[s].lists_fresh = 1;
-      st[s].compact_bad = 0;
-      st[s].half_bad = 0;
-    }
-    if (threadIdx.x == 0) {
-      *a.any_rebuild = 0;
-      *a.nbr_wide_n = 0;
-      *a.nbr_sub_n = 0;
-    }
-    __syncthreads();
-    if (mine) atomicAdd(a.any_rebuild, mine);
-  }
-  bool ok = grid_barrier(a.grid_ctl, gridDim.x);
-  if (ok) {
-    if (blockIdx.x == 0)
-      for (int s = static_cast<int>(threadIdx.x); s < nsys; s += static_cast<int>(blockDim.x)) st[s].moved = 0;
-    rebin_dest(n_part, sys, st, a);
-    ok = grid_barrier(a.grid_ctl, gridDim.x);
-  }
-  if (ok) {
-    rebin_compact(n_cells, sys, st, a);
-    ok = grid_barrier(a.grid_ctl, gridDim.x);
-  }
-  if (ok) {
-    rebin_count(n_cells, sys, st, a);
-    ok = grid_barrier(a.grid_ctl, gridDim.x);
-  }
-  if (ok) {
-    if (blockIdx.x == 0) scan_cells_one_block(a.cell_cnt, n_cells, a.cell_scan);
-    ok = grid_barrier(a.grid_ctl, gridDim.x);
-  }
-  if (ok) {
-    rebin_scatter(n_cells, sys, st, a);
-    ok = grid_barrier(a.grid_ctl, gridDim.x);
-  }
-  if (ok) {
-    rebin_finalize<BACKUP>(n_cells, sys, st, a);
-  } else if (threadIdx.x == 0) {
-    // a barrier ran out of time: the systems being rebuilt stop
-    for (int s = 0; s < nsys; ++s)
-      if (__ldcg(&st[s].rebuild)) atomicOr(&st[s].error, kErrBarrier);
-  }
-}
-
 // ---------------------------------------------------------------------------
 // chunk_neighbors_execute (particle_neighbors/include/exanb/particle_neighbors/
 // chunk_neighbors_execute.h:110-244, 286-372): for each particle of cell a, the
@@ -595,12 +518,8 @@ __device__ __forceinline__ void finish_particle(const DevArrays& a, uint32_t* se
 // directly. A particle with more hits than the slot holds keeps its true count,
 // writes nothing past the slot and flags the system (kErrListOverflow); max_nbr
 // records the largest count for resizing.
-// 64 registers (8 blocks of 128 per SM): measured faster than the 90-register
-// schedule despite a few spills.
-__global__ void __launch_bounds__(128, 8)
-    k_neighbors(uint32_t n_cells, const SysDesc* __restrict__ sys, SysState* st, DevArrays a, int cap, int lbuf) {
-  if (*a.any_rebuild == 0) return;
-  extern __shared__ float4 stage_all[];
+__device__ __forceinline__ void neighbors_wide(uint32_t n_cells, const SysDesc* __restrict__ sys, SysState* st,
+                                               const DevArrays& a, int cap, int lbuf, float4* stage_all) {
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t wib = threadIdx.x >> 5;
   const uint32_t nwarp = blockDim.x >> 5;
@@ -791,6 +710,15 @@ __global__ void __launch_bounds__(128, 8)
   if (lane == 0) flush_list_stats(st, sys, acc_s, acc_max, acc_sum);
 }
 
+// 64 registers (8 blocks of 128 per SM): measured faster than the 90-register
+// schedule despite a few spills.
+__global__ void __launch_bounds__(128, 8)
+    k_neighbors(uint32_t n_cells, const SysDesc* __restrict__ sys, SysState* st, DevArrays a, int cap, int lbuf) {
+  if (*a.any_rebuild == 0) return;
+  extern __shared__ float4 stage_all[];
+  neighbors_wide(n_cells, sys, st, a, cap, lbuf, stage_all);
+}
+
 // ---------------------------------------------------------------------------
 // Warp-per-cell form of the same build. The warp stages the candidates that can
 // lie within nbh_dist of any of the cell's particles -- those within reach of
@@ -933,19 +861,19 @@ __device__ __forceinline__ void warp_pass(const SysDesc& S, const DevArrays& a, 
 
 // split warps share a cell (each stages it and takes every split-th group of
 // particles): batches with fewer cells than the GPU holds warps.
-__global__ void __launch_bounds__(128, 5)
-    k_neighbors_warp(uint32_t n_cells, const SysDesc* __restrict__ sys, SysState* st, DevArrays a, int cap,
-                     bool prune, bool half_form, uint32_t split) {
-  if (*a.any_rebuild == 0) return;
-  extern __shared__ float4 stage_w[];
+// (Plain loads: in the fused rebin the mirrors were written by this launch.)
+template <int WARPS>
+__device__ __forceinline__ void neighbors_warp(uint32_t n_cells, const SysDesc* __restrict__ sys, SysState* st,
+                                               const DevArrays& a, int cap, bool prune, bool half_form, uint32_t split,
+                                               float4* stage) {
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t wib = threadIdx.x >> 5;
   const uint32_t nwarp = blockDim.x >> 5;
-  float4* srel = stage_w + static_cast<size_t>(wib) * cap;
+  float4* srel = stage + static_cast<size_t>(wib) * cap;
   constexpr int kSteps = 32;
-  __shared__ uint4 lists[4][kSteps];
+  __shared__ uint4 lists[WARPS][kSteps];
   uint4* const list = lists[wib];  // first candidate, candidates left, image code
-  __shared__ uint32_t sink[4][kWarpP];  // hits of systems without list slots (blocks of 4 warps)
+  __shared__ uint32_t sink[WARPS][kWarpP];  // hits of systems without list slots
   WarpCell w;
   w.lt = lanemask_lt();
   w.sink = sink[wib];
@@ -1041,7 +969,7 @@ __global__ void __launch_bounds__(128, 5)
           for (uint32_t q = 0; q < 4u; ++q) {
             run[q] = list[min(t + q, t1 - 1u)];
             if (t + q >= t1) run[q].y = 0;
-            pb[q] = lane < run[q].y ? __ldg(a.pf + run[q].x + lane) : make_float4(0.f, 0.f, 0.f, 0.f);
+            pb[q] = lane < run[q].y ? a.pf[run[q].x + lane] : make_float4(0.f, 0.f, 0.f, 0.f);
           }
 #pragma unroll
           for (uint32_t q = 0; q < 4u; ++q) {
@@ -1108,6 +1036,102 @@ __global__ void __launch_bounds__(128, 5)
     __syncwarp();  // the stage is refilled for the next cell
   }
   if (lane == 0) flush_list_stats(st, sys, acc_s, acc_max, acc_sum);
+}
+
+__global__ void __launch_bounds__(128, 5)
+    k_neighbors_warp(uint32_t n_cells, const SysDesc* __restrict__ sys, SysState* st, DevArrays a, int cap,
+                     bool prune, bool half_form, uint32_t split) {
+  if (*a.any_rebuild == 0) return;
+  extern __shared__ float4 stage_w[];
+  neighbors_warp<4>(n_cells, sys, st, a, cap, prune, half_form, split, stage_w);
+}
+
+// The trigger's decision and the whole rebin (K_r1 .. K_r6, the resets of the
+// build that follows) of a small batch in one cooperative launch. A step without
+// a rebuild costs one launch that returns at once, where the separate kernels
+// cost twelve (0.7 us each inside a graph, 2.3 us when launched one by one); a
+// rebuild costs six grid barriers. The phases are the separate kernels' bodies.
+// BUILD: the lists of the flagged systems too (the warp-per-cell form without
+// sub-cell pruning, then the cells it passes on), two more barriers: a step
+// without a rebuild is then three launches, push, this one and the forces.
+template <int BACKUP, bool BUILD>
+__global__ void __launch_bounds__(256)
+    k_rebin_fused(uint32_t n_part, uint32_t n_cells, int nsys, const SysDesc* __restrict__ sys, SysState* st,
+                  DevArrays a, int cap, int lbuf, uint32_t split) {
+  extern __shared__ float4 fused_smem[];
+  int flagged = 0;
+  for (int s = static_cast<int>(threadIdx.x); s < nsys; s += static_cast<int>(blockDim.x))
+    flagged |= __ldcg(&st[s].moved) != 0ull ? 1 : 0;
+  if (!__syncthreads_or(flagged)) {
+    if (blockIdx.x == 0) {
+      for (int s = static_cast<int>(threadIdx.x); s < nsys; s += static_cast<int>(blockDim.x)) st[s].rebuild = 0;
+      if (threadIdx.x == 0) *a.any_rebuild = 0;
+    }
+    return;
+  }
+  if (blockIdx.x == 0) {
+    // what the other blocks read before the first barrier is `moved` alone
+    unsigned int mine = 0;
+    for (int s = static_cast<int>(threadIdx.x); s < nsys; s += static_cast<int>(blockDim.x)) {
+      const bool r = __ldcg(&st[s].moved) != 0ull;
+      st[s].rebuild = r ? 1u : 0u;
+      if (!r) continue;
+      ++mine;
+      st[s].rebuilds += 1;
+      st[s].rebuild_armed = 1;
+      st[s].keys_fresh = 1;
+      // the build that follows (k_nbr_reset)
+      st[s].list_used = 0;
+      st[s].max_nbr = 0;
+      st[s].lists_fresh = 1;
+      st[s].compact_bad = 0;
+      st[s].half_bad = 0;
+    }
+    if (threadIdx.x == 0) {
+      *a.any_rebuild = 0;
+      *a.nbr_wide_n = 0;
+      *a.nbr_sub_n = 0;
+    }
+    __syncthreads();
+    if (mine) atomicAdd(a.any_rebuild, mine);
+  }
+  bool ok = grid_barrier(a.grid_ctl, gridDim.x);
+  if (ok) {
+    if (blockIdx.x == 0)
+      for (int s = static_cast<int>(threadIdx.x); s < nsys; s += static_cast<int>(blockDim.x)) st[s].moved = 0;
+    rebin_dest(n_part, sys, st, a);
+    ok = grid_barrier(a.grid_ctl, gridDim.x);
+  }
+  if (ok) {
+    rebin_compact(n_cells, sys, st, a);
+    ok = grid_barrier(a.grid_ctl, gridDim.x);
+  }
+  if (ok) {
+    rebin_count(n_cells, sys, st, a);
+    ok = grid_barrier(a.grid_ctl, gridDim.x);
+  }
+  if (ok) {
+    if (blockIdx.x == 0) scan_cells_one_block(a.cell_cnt, n_cells, a.cell_scan);
+    ok = grid_barrier(a.grid_ctl, gridDim.x);
+  }
+  if (ok) {
+    rebin_scatter(n_cells, sys, st, a);
+    ok = grid_barrier(a.grid_ctl, gridDim.x);
+  }
+  if (ok) {
+    rebin_finalize<BACKUP>(n_cells, sys, st, a);
+    if (BUILD) ok = grid_barrier(a.grid_ctl, gridDim.x);
+  }
+  if (BUILD && ok) {
+    neighbors_warp<8>(n_cells, sys, st, a, cap, false, false, split, fused_smem);
+    ok = grid_barrier(a.grid_ctl, gridDim.x);
+  }
+  if (BUILD && ok) neighbors_wide(n_cells, sys, st, a, cap, lbuf, fused_smem);
+  if (!ok && threadIdx.x == 0) {
+    // a barrier ran out of time: the systems being rebuilt stop
+    for (int s = 0; s < nsys; ++s)
+      if (__ldcg(&st[s].rebuild)) atomicOr(&st[s].error, kErrBarrier);
+  }
 }
 
 // Clears the per-build list statistics of the flagged systems.
@@ -1270,21 +1294,37 @@ bool fused_rebin_fits(const Extent& ex) {
   return ex.n_part > 0 && ex.n_part <= kFusedRebinMaxParticles && ex.n_cells > 0 && ex.n_cells <= kFusedRebinMaxCells;
 }
 
+bool fused_build_fits(const Extent& ex, int form, bool prune) {
+  return ex.n_cells <= kFusedBuildMaxCells && form == kBuildWarp && ex.force_form != kForceStaged && !(prune && ex.dense);
+}
+
 int launch_rebin_fused(const Extent& ex, const SysDesc* sys, SysState* st, const DevArrays& a, bool exact_backup,
-                       cudaStream_t stream) {
-  // a warp per cell, at most one block per SM: always co-resident
-  const unsigned grid = std::min((ex.n_cells + 7u) / 8u, static_cast<unsigned>(ex.sm_count));
+                       bool build, int cap, int lbuf, cudaStream_t stream) {
+  constexpr unsigned warps = 8;
+  // at most one block per SM: always co-resident. The rebin takes a warp per
+  // cell, the build up to four
+  const unsigned want = build ? ex.n_cells * 4u : ex.n_cells;
+  const unsigned grid = std::min((want + warps - 1u) / warps, static_cast<unsigned>(ex.sm_count));
+  const uint32_t split = ex.n_cells * 4u <= grid * warps ? 4u : (ex.n_cells * 2u <= grid * warps ? 2u : 1u);
+  size_t smem = 0;
+  if (build) {
+    smem = std::max(static_cast<size_t>(warps) * cap * sizeof(float4),
+                    static_cast<size_t>(cap) * sizeof(float4) + static_cast<size_t>(warps) * 2 * lbuf * sizeof(uint32_t));
+  }
+  auto kern = exact_backup ? (build ? k_rebin_fused<kBackupExact, true> : k_rebin_fused<kBackupExact, false>)
+                           : (build ? k_rebin_fused<kBackupPlain, true> : k_rebin_fused<kBackupPlain, false>);
+  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(256);
+  cfg.blockDim = dim3(warps * 32u);
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeCooperative;
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, exact_backup ? k_rebin_fused<kBackupExact> : k_rebin_fused<kBackupPlain>, ex.n_part,
-                     ex.n_cells, ex.nsys, sys, st, a);
+  cudaLaunchKernelEx(&cfg, kern, ex.n_part, ex.n_cells, ex.nsys, sys, st, a, cap, lbuf, split);
   return 1;
 }
 

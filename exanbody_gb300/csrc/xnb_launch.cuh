@@ -20,6 +20,7 @@ struct Extent {
   int force_lanes;   // threads per particle of the FP64 / mixed full-list traversal (1, 2 or 4)
   int far_coords;    // some resident system lies far from the coordinate origin (SysDesc::far_coords)
   int unpacked;      // some resident system reads the residual mirror, not packed residuals (SysDesc::packed_lo)
+  int dense;         // some resident system's cells hold half of what gives them a sub-grid, on average
   uint32_t list_slot;  // largest list slot of the resident systems
   int force_form;    // kForceThread or kForceStaged (mixed full-list traversal)
   uint32_t n_seg;    // cell segments of the staged traversal (DevArrays::seg)
@@ -103,8 +104,14 @@ int launch_rebin(const Extent& ex, const SysDesc* sys, SysState* st, const DevAr
 constexpr uint32_t kFusedRebinMaxParticles = 100000;
 constexpr uint32_t kFusedRebinMaxCells = 16384;
 bool fused_rebin_fits(const Extent& ex);
+// build: the neighbour lists as well, for batches of few cells (one block per SM
+// builds 1,331 cells slower than a launch of their own: 50 steps of 32,000 atoms
+// 2.39 against 2.27 ms; 200 eager steps of 1,000 cells 13.2 against 16.6 ms) too sparse
+// for sub-cell pruning to matter.
+constexpr uint32_t kFusedBuildMaxCells = 1024;
+bool fused_build_fits(const Extent& ex, int form, bool prune);
 int launch_rebin_fused(const Extent& ex, const SysDesc* sys, SysState* st, const DevArrays& a, bool exact_backup,
-                       cudaStream_t stream);
+                       bool build, int cap, int lbuf, cudaStream_t stream);
 int launch_backup(const Extent& ex, const SysDesc* sys, SysState* st, const DevArrays& a, cudaStream_t stream);
 // chunk_neighbors for systems with rebuild != 0: one pass writing each list
 // into its particle's slot (statistics reset, the warp-per-cell build, and the

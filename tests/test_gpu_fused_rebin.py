@@ -27,17 +27,19 @@ def many():
     return [workloads.lj_fcc_system(2 + k % 4 + 2, 0.75 + 0.01 * k, 0.7 + 0.05 * k, k) for k in range(20)]
 
 
-@pytest.mark.parametrize("systems", [
-    lambda: [gas(25, 1500, 3)],                                    # 15,625 cells: eight scan passes
-    lambda: [workloads.lj_fcc_system(12, cell_factor=2.0)],        # ~190 atoms per cell, sub-grid side 3
-    many,
-], ids=["gas", "dense", "many"])
+@pytest.mark.parametrize("systems,cap", [
+    (lambda: [gas(25, 1500, 3)], 640),                              # 15,625 cells: eight scan passes
+    (lambda: [workloads.lj_fcc_system(12, cell_factor=2.0)], 640),  # ~190 atoms per cell, sub-grid side 3
+    (many, 640),                                                    # lists built by the same launch
+    (many, 192),                                                    # and part of them block per cell
+], ids=["gas", "dense", "many", "many_wide"])
 @pytest.mark.parametrize("precision", [xnb.PREC_FP64_EXACT, xnb.PREC_MIXED])
-def test_fused_rebin_equals_the_separate_kernels(systems, precision):
+def test_fused_rebin_equals_the_separate_kernels(systems, cap, precision):
     out = []
     for flags in (0, xnb.STEP_HOST_SYNC):
         ws = systems()
         b = new_batch([w["n_atoms"] for w in ws], [ncells(w["geom"]) for w in ws], max_systems=len(ws))
+        b.set_tuning(cap, 64)
         ss = [b.add_system(xnb.lj_params(w["geom"]), w["r"], w["v"], w["id"]) for w in ws]
         b.init_particles(-1, precision)
         b.step(40, precision, flags)
