@@ -1143,7 +1143,6 @@ int xnb_step(xnb_batch* b, int32_t nsteps, int32_t precision, int32_t flags, voi
       b->launches += launch_force(ex, b->d_sys, b->d_st, b->a, precision, energy, true, -1, st, newton);
       continue;
     }
-    b->launches += launch_mark_rebuild(ex, b->d_st, 1, -1, b->a.any_rebuild, st);
     bool rebuild = true;
     if (flags & XNB_STEP_HOST_SYNC) {
       int rc = pull_states(b, st);
@@ -1154,6 +1153,7 @@ int xnb_step(xnb_batch* b, int32_t nsteps, int32_t precision, int32_t flags, voi
     }
     if (rebuild) {
       // update_particles_full
+      b->launches += launch_mark_rebuild(ex, b->d_st, 1, -1, b->a.any_rebuild, st);
       b->launches += launch_rebin(ex, b->d_sys, b->d_st, b->a, st, exact);
       if (flags & XNB_STEP_HOST_SYNC) {
         int rc = neighbors_sync(b, st);
@@ -1162,10 +1162,10 @@ int xnb_step(xnb_batch* b, int32_t nsteps, int32_t precision, int32_t flags, voi
         b->launches += launch_neighbors(ex, b->d_sys, b->d_st, b->a, b->stage_cap, list_buf(b), st, b->build_form,
                                         b->subcell_prune != 0);
       }
+      b->launches += launch_clear_moved(ex, b->d_st, st);
     }
     // compute_all_forces_energy + verlet_second_half
     b->launches += launch_force(ex, b->d_sys, b->d_st, b->a, precision, energy, true, -1, st, newton);
-    b->launches += launch_clear_moved(ex, b->d_st, st);
   }
   return check_launch();
 }

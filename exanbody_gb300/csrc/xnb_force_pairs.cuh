@@ -253,12 +253,13 @@ __device__ __forceinline__ void eight_particles(uint32_t first, uint32_t n_part,
           if (!(w & kCheck) || (d2 > 0.0 && d2 <= S.rcut2)) {
             // lj_compute_energy (lennard_jones.cu:46-56) then pair_de *= w / r with w = 1
             const double rr = __dsqrt_rn(d2);
-            const double inv_r = __ddiv_rn(1.0, rr);
+            const double inv_r = __drcp_rn(rr);  // the rounded 1 / r, without the division's quotient steps
             const double ratio = __dmul_rn(S.sigma, inv_r);
             const double ratio2 = __dmul_rn(ratio, ratio);
             const double ratio6 = __dmul_rn(__dmul_rn(ratio2, ratio2), ratio2);
             const double ratio12 = __dmul_rn(ratio6, ratio6);
-            double de = __dmul_rn(__dmul_rn(S.m24eps, __dsub_rn(__dmul_rn(2.0, ratio12), ratio6)), inv_r);
+            // 2 ratio12 is exact: one rounding either way
+            double de = __dmul_rn(__dmul_rn(S.m24eps, __fma_rn(2.0, ratio12, -ratio6)), inv_r);
             de = __dmul_rn(de, inv_r);
             g[0] = __dmul_rn(de, dx);
             g[1] = __dmul_rn(de, dy);
