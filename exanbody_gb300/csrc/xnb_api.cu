@@ -121,6 +121,7 @@ struct xnb_batch {
     int hw = 0;
     e.far_coords = 0;
     e.unpacked = 0;
+    e.general = 0;
     e.list_slot = 0;
     e.dense = 0;
     for (size_t s = 0; s < sys.size(); ++s)
@@ -128,6 +129,7 @@ struct xnb_batch {
         hw = static_cast<int>(s) + 1;
         if (sys[s].d.far_coords) e.far_coords = 1;
         if (!sys[s].d.packed_lo) e.unpacked = 1;
+        if (!sys[s].d.packed_lo || !sys[s].d.origin_zero || sys[s].d.plain_sums) e.general = 1;
         e.list_slot = std::max(e.list_slot, sys[s].d.list_slot);
         const SysDesc& d = sys[s].d;
         if (d.amr_enabled && 2ull * d.npart >= static_cast<uint64_t>(d.amr_min_n) * d.ncells) e.dense = 1;
@@ -149,7 +151,7 @@ struct xnb_graph {
   // what the captured launches depend on besides device memory: the batch's
   // work extent and launch configuration at capture
   uint32_t n_part = 0, n_cells = 0;
-  int nsys = 0, lbuf = 0, stage_cap = 0, force_block = 0, force_lanes = 0, build_form = 0, far_coords = 0;
+  int nsys = 0, lbuf = 0, stage_cap = 0, force_block = 0, force_lanes = 0, build_form = 0, far_coords = 0, general = 0;
   int force_form = 0, subcell_prune = 0;
   uint32_t n_seg = 0;
 };
@@ -353,14 +355,20 @@ SysDesc make_desc(const xnb_lj_params& p) {
   {
     // Force factors pd of a fluid lie within a few powers of two of 24 eps /
     // sigma^2 = 2^E: with Q = 2^(E - 44) every |pd| >= 2^(E - 21) is a multiple of
-    // Q, and sums of |pd| up to 2^(E + 8) = 2^52 Q are exact in FP64.
-    const double scale = d.sig2 > 0.0 ? std::fabs(d.eps24) / d.sig2 : 0.0;
-    int e = 1;
-    if (std::isfinite(scale) && scale > 1e-30 && scale < 1e30) std::frexp(scale, &e);
-    const int E = e - 1;
-    d.psum_quantum = std::ldexp(1.0, E - 44);
-    d.psum_exp = E + 106;  // 127 + 23 + (E - 44)
-    d.psum_max_f = std::ldexp(1.0f, E + 8);
+    // Q, and sums of |pd| up to 2^(E + 8) = 2^52 Q are exact in FP64. Halved pair
+    // energies, with eps = 2^F: |pe| >= 2^(F - 24), sums up to 2^(F + 5).
+    const auto range = [](double scale, int below, int above) {
+      int e = 1;
+      if (std::isfinite(scale) && scale > 1e-30 && scale < 1e30) std::frexp(scale, &e);
+      const int q = e - 1 - below - 23;
+      return SumRange{std::ldexp(1.0, q), std::ldexp(1.0f, e - 1 + above), 127 + 23 + q};
+    };
+    const double scale = d.sig2 > 0.0 ? std::fabs(d.eps24) / d.sig2 : 0.0, well = std::fabs(d.eps4) * 0.25;
+    d.sum_pd = range(scale, 21, 8);
+    d.sum_pe = range(well, 24, 5);
+    // Energies pass through zero at the cutoff: the longer it is, the more of them
+    // fall below the range (2 in 10^4 particles at 2.5 sigma, 1 in 10^3 at 3).
+    d.plain_sums = !(scale > 1e-30 && scale < 1e30 && well > 1e-30 && well < 1e30 && d.rcut2 <= 9.0 * d.sig2);
   }
   // FP32 cell index of the rebin: the mirror pf = fl32(x - origin) and
   // fl32(1/cell_size) put pf * inv within 3.01 u |q| of the quotient q of the
@@ -574,6 +582,7 @@ int xnb_batch_create(const xnb_batch_config* cfg, xnb_batch** out) {
   rc = rc ? rc : dalloc(b, &a.id, P);
   rc = rc ? rc : dalloc(b, &a.pf, P);
   rc = rc ? rc : dalloc(b, &a.pflo, P);
+  rc = rc ? rc : dalloc(b, &a.pstep, P);
   rc = rc ? rc : dalloc(b, &a.rbf, P);
   rc = rc ? rc : dalloc(b, &a.nbr_half, P);
   rc = rc ? rc : dalloc(b, &a.any_rebuild, 4);
@@ -805,6 +814,7 @@ int place_system(xnb_batch* b, const xnb_lj_params* p, int64_t n, const double* 
     }
     XCK(cudaMemcpyAsync(a.pf + poff, hpf.data(), nb * sizeof(float4), cudaMemcpyHostToDevice, st));
     XCK(cudaMemcpyAsync(a.pflo + poff, hlo.data(), nb * sizeof(float4), cudaMemcpyHostToDevice, st));
+    XCK(cudaMemsetAsync(a.pstep + poff, 0xFF, nb * sizeof(int4), st));  // none: FP64 until the first rebin
     XCK(cudaMemsetAsync(a.fx + poff, 0, nb * sizeof(double), st));
     XCK(cudaMemsetAsync(a.fy + poff, 0, nb * sizeof(double), st));
     XCK(cudaMemsetAsync(a.fz + poff, 0, nb * sizeof(double), st));
@@ -1235,6 +1245,7 @@ int xnb_step_graph_create(xnb_batch* b, int32_t nsteps, int32_t precision, int32
   G->n_cells = ex.n_cells;
   G->nsys = ex.nsys;
   G->far_coords = ex.far_coords;
+  G->general = ex.general;
   G->force_form = ex.force_form;
   G->n_seg = ex.n_seg;
   G->lbuf = list_buf(b);
@@ -1258,6 +1269,7 @@ int xnb_graph_is_current(const xnb_graph* g) {
   const xnb_batch* b = g->batch;
   const Extent ex = b->extent();
   return (ex.n_part == g->n_part && ex.n_cells == g->n_cells && ex.nsys == g->nsys && ex.far_coords == g->far_coords &&
+          ex.general == g->general &&
           ex.force_form == g->force_form && ex.n_seg == g->n_seg &&
           list_buf(b) == g->lbuf &&
           b->stage_cap == g->stage_cap && b->force_block == g->force_block && b->force_lanes == g->force_lanes &&

@@ -209,6 +209,162 @@ void go(const Extent& ex, const SysDesc* sys, const SysState* st, const DevArray
   k_force_mixed<PE, KICK><<<grid, threads, smem, stream>>>(ex.n_part, src, a, group, chunk);
 }
 
+// ---------------------------------------------------------------------------
+// One thread per particle, for batches that fill the GPU so: every list entry
+// once, two at a time, their mirrors and position steps (DevArrays::pstep) in
+// flight together. A pair costs 3 DFMA on the FP64 pipe, which bounds the walk: a
+// warp makes about 100 rounds of three (its longest list), and at one million
+// atoms the pipe is busy 82% of the time (the general walk, which marks the
+// entries near the cutoff first and gathers those a second time: 73 rounds, the
+// pipe at 58% and the L1 data stage at 66%). 64 registers hold 16 blocks of 64
+// threads per SM. General walk / this one: 25 steps of 4M atoms 74.9 / 69.4 ms
+// (three such batches at once 75.0 / 73.7); 1M atoms with energies 728 / 683 us; a
+// batch of 96 small systems, 20 steps, three at once 45.2 / 42.6 ms. With 56
+// registers 71.7 ms and 773 us, four entries at a time 80.8 ms.
+// A pair's FP64 position is needed only within the cutoff.
+struct WalkParticle {
+  const double* rx;
+  const double* ry;
+  const double* rz;
+  const float4* pf;
+  const int4* pstep;
+  const uint32_t* list;
+  uint32_t i, n, pbase;
+  float4 own;
+};
+
+// b's FP64 position from its mirror and steps.
+__device__ __forceinline__ void position(const WalkParticle& w, uint32_t j, float4 hb, int4 d, double& x, double& y,
+                                         double& z) {
+  if (d.w) {
+    x = w.rx[j];
+    y = w.ry[j];
+    z = w.rz[j];
+    return;
+  }
+  x = step_coord(hb.x, d.x);
+  y = step_coord(hb.y, d.y);
+  z = step_coord(hb.z, d.z);
+}
+
+// One entry: the values of mixed_pair (xnb_lj_pair.cuh) with the packed residuals,
+// handed to sink(pd, s6, x_b, y_b, z_b) for a pair within the cutoff.
+template <class Sink>
+__device__ __forceinline__ void walk_entry(const SysDesc& S, const WalkParticle& w, uint32_t e, float4 hb, int4 d,
+                                           float step, float r2_in, float r2_out, float r2_min, const Sink& sink) {
+  const uint32_t code = e & 31u, j = w.pbase + (e >> 5);
+  float dx, dy, dz, r2;
+  double x, y, z;
+  if (code == static_cast<uint32_t>(kImageCenter)) {
+    // within 2u|d| + 2 lo_step of the FP64 displacement (u = 2^-24)
+    const uint32_t wb = __float_as_uint(hb.w), wa = __float_as_uint(w.own.w);
+    dx = fmaf(field_x(wb) - field_x(wa), step, hb.x - w.own.x);
+    dy = fmaf(field_y(wb) - field_y(wa), step * 0.0009765625f, hb.y - w.own.y);
+    dz = fmaf(field_z(wb) - field_z(wa), step, hb.z - w.own.z);
+    r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+    if (r2 > r2_out) return;
+    position(w, j, hb, d, x, y, z);
+  } else {
+    position(w, j, hb, d, x, y, z);
+    x = image_coord(x, S.period[0], static_cast<int>(code % 3u));
+    y = image_coord(y, S.period[1], static_cast<int>((code / 3u) % 3u));
+    z = image_coord(z, S.period[2], static_cast<int>(code / 9u));
+    dx = narrow_f64(__dsub_rn(x, w.rx[w.i]));
+    dy = narrow_f64(__dsub_rn(y, w.ry[w.i]));
+    dz = narrow_f64(__dsub_rn(z, w.rz[w.i]));
+    r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+    if (r2 > r2_out) return;
+  }
+  if (!(r2 < r2_in && r2 > r2_min)) {
+    // inside the FP32 band: the FP64 decision
+    const double d2 = norm2_rn(__dsub_rn(x, w.rx[w.i]), __dsub_rn(y, w.ry[w.i]), __dsub_rn(z, w.rz[w.i]));
+    if (!(d2 > 0.0 && d2 <= S.rcut2)) return;
+  }
+  // the hardware reciprocal (within 1 ulp) is part of the FP32 force magnitude
+  float ir2;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(ir2) : "f"(r2));
+  const float s2 = S.sig2_f * ir2;
+  const float s6 = s2 * s2 * s2;
+  sink(S.eps24_f * s6 * fmaf(-2.0f, s6, 1.0f) * ir2, s6, x, y, z);
+}
+
+__device__ __forceinline__ float pair_energy(const SysDesc& S, float s6) {
+  return 0.5f * fmaf(S.eps4_f * s6, s6 - 1.0f, -S.e_shift_f);
+}
+
+// Sum of pd, or of the energies, in FP64, in list order (where PairSum is not exact).
+template <bool ENERGY>
+__device__ __noinline__ double sum_in_order(const SysDesc& S, const double* rx, const double* ry, const double* rz,
+                                            const float4* pf, const int4* pstep, uint32_t i, const uint32_t* list,
+                                            uint32_t n) {
+  const WalkParticle w{rx, ry, rz, pf, pstep, list, i, n, S.part_base, pf[i]};
+  double sum = 0.0;
+  for (uint32_t k = 0; k < n; ++k) {
+    const uint32_t e = list[k], j = w.pbase + (e >> 5);
+    walk_entry(S, w, e, pf[j], pstep[j], S.lo_step_f, S.rc2_f - S.rc_margin_f, S.rc2_f + S.rc_margin_f, S.rc_margin_f,
+               [&](float pd, float s6, double, double, double) {
+                 sum += widen_f32_fast(ENERGY ? pair_energy(S, s6) : pd);
+               });
+  }
+  return sum;
+}
+
+template <bool PE, bool KICK>
+__global__ void __maxnreg__(64) k_force_walk(uint32_t n_part, BatchSource src, DevArrays a) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  uint32_t s, n;
+  const uint32_t* list;
+  if (i >= n_part || !src.locate(i, s, list, n)) return;
+  const SysDesc& S = src.sys[s];
+  const WalkParticle w{src.rx, src.ry, src.rz, src.pf, a.pstep, list, i, n, S.part_base, src.pf[i]};
+  const float step = S.lo_step_f, r2_in = S.rc2_f - S.rc_margin_f, r2_out = S.rc2_f + S.rc_margin_f,
+              r2_min = S.rc_margin_f;
+  const int pd_exp = S.sum_pd.exponent;
+  double fx = 0.0, fy = 0.0, fz = 0.0;
+  PairSum pds, pes;
+  pds.clear();
+  pes.clear();
+  const auto add = [&](float pd, float s6, double x, double y, double z) {
+    // the FP64 displacement folded into the accumulation (mixed_pair)
+    const double pdd = widen_f32_fast(pd);
+    fx = fma(pdd, x, fx);
+    fy = fma(pdd, y, fy);
+    fz = fma(pdd, z, fz);
+    pds.add(pd_exp, pd);
+    if (PE) pes.add(S.sum_pe.exponent, pair_energy(S, s6));
+  };
+  // entries past an odd list's end: the particle's own slot, not visited (list
+  // slots are multiples of 8 entries, 32-byte aligned)
+  const uint32_t self_e = ((i - w.pbase) << 5) | static_cast<uint32_t>(kImageCenter);
+  uint2 next = n ? __ldg(reinterpret_cast<const uint2*>(list)) : make_uint2(self_e, self_e);
+  for (uint32_t k = 0; k < n; k += 2u) {
+    const uint32_t e0 = next.x, e1 = k + 1u < n ? next.y : self_e;
+    const uint32_t j0 = w.pbase + (e0 >> 5), j1 = w.pbase + (e1 >> 5);
+    const float4 h0 = __ldg(w.pf + j0);
+    const int4 d0 = __ldg(w.pstep + j0);
+    const float4 h1 = __ldg(w.pf + j1);
+    const int4 d1 = __ldg(w.pstep + j1);
+    if (k + 2u < n) next = __ldg(reinterpret_cast<const uint2*>(list + k + 2u));
+    walk_entry(S, w, e0, h0, d0, step, r2_in, r2_out, r2_min, add);
+    if (k + 1u < n) walk_entry(S, w, e1, h1, d1, step, r2_in, r2_out, r2_min, add);
+  }
+  const double psum = pds.exact(S.sum_pd) ? pds.value(S.sum_pd)
+                                          : sum_in_order<false>(S, a.rx, a.ry, a.rz, a.pf, a.pstep, i, list, n);
+  double pe = 0.0;
+  if (PE)
+    pe = pes.exact(S.sum_pe) ? pes.value(S.sum_pe)
+                             : sum_in_order<true>(S, a.rx, a.ry, a.rz, a.pf, a.pstep, i, list, n);
+  finish_mixed<PE, KICK>(S, a, i, fx, fy, fz, psum, pe);
+}
+
+template <bool PE, bool KICK>
+void go_walk(const Extent& ex, const SysDesc* sys, const SysState* st, const DevArrays& a, int sys_only,
+             cudaStream_t stream) {
+  const unsigned threads = ex.force_block > 0 ? static_cast<unsigned>(ex.force_block) : 64u;
+  k_force_walk<PE, KICK><<<(ex.n_part + threads - 1u) / threads, threads, 0, stream>>>(
+      ex.n_part, BatchSource(sys, st, a, sys_only), a);
+}
+
 }  // namespace
 
 int launch_force_mixed(const Extent& ex, const SysDesc* sys, const SysState* st, const DevArrays& a, bool with_pe,
@@ -217,6 +373,15 @@ int launch_force_mixed(const Extent& ex, const SysDesc* sys, const SysState* st,
   else if (with_pe) go<true, false>(ex, sys, st, a, sys_only, stream);
   else if (second_half) go<false, true>(ex, sys, st, a, sys_only, stream);
   else go<false, false>(ex, sys, st, a, sys_only, stream);
+  return 1;
+}
+
+int launch_force_walk(const Extent& ex, const SysDesc* sys, const SysState* st, const DevArrays& a, bool with_pe,
+                      bool second_half, int sys_only, cudaStream_t stream) {
+  if (with_pe && second_half) go_walk<true, true>(ex, sys, st, a, sys_only, stream);
+  else if (with_pe) go_walk<true, false>(ex, sys, st, a, sys_only, stream);
+  else if (second_half) go_walk<false, true>(ex, sys, st, a, sys_only, stream);
+  else go_walk<false, false>(ex, sys, st, a, sys_only, stream);
   return 1;
 }
 

@@ -46,6 +46,13 @@ struct GridBarrier {
   unsigned int pad;
 };
 
+// Range of the terms whose sum is formed exactly in integers (PairSum).
+struct SumRange {
+  double quantum;    // Q
+  float limit;       // 2^52 Q
+  int32_t exponent;  // FP32 exponent field of 2^23 Q
+};
+
 // Per-system constants, device resident (SysDesc[nsys]).
 struct SysDesc {
   double origin[3];
@@ -80,9 +87,8 @@ struct SysDesc {
   float sub_reach_f;             // nbh_dist / cell_size widened by 1e-5: reach of the sub-cell box test (cells)
   float lo_step_f, lo_inv_f;     // quantum of the residual packed in DevArrays::pf.w (ulp(X)/1024) and its inverse
   float period_lo_f[3];          // period - period_f, rounded: the image offset in two FP32 words
-  double psum_quantum;           // Q of the exact sum of the mixed force factors (PairSum)
-  int32_t psum_exp;              // FP32 exponent field of 2^23 Q
-  float psum_max_f;              // 2^52 Q
+  SumRange sum_pd, sum_pe;       // of the mixed force factors and the halved pair energies
+  int32_t plain_sums;            // 1: these ranges do not fit the system's terms (a long cutoff, no force)
   float image_tie_f;             // bound on the error of an image displacement formed from FP32 pairs
   int32_t packed_lo;             // 1: the mixed traversal reads the packed residuals (X < 1024); 0: DevArrays::pflo
   double inv_cell;               // fl(1/cell_size): reciprocal pre-decision of the backup encoding
@@ -123,6 +129,7 @@ struct DevArrays {
   float4* pf;                      // FP32 hi part of (x - origin, y - origin, z - origin), refreshed with r;
                                    // .w packs the three residuals as 10-bit multiples of lo_step_f (lo_field)
   float4* pflo;                    // FP32 residual (x - origin) - hi, so hi + lo carries ~48 bits
+  int4* pstep;                     // rx, ry, rz as steps of their FP64 bit patterns from those of pf (origin zero)
   GridBarrier* grid_ctl;           // of the fused rebin
   unsigned int* any_rebuild;       // number of systems flagged for the rebuild path this step
   uint64_t* id;
@@ -265,6 +272,25 @@ __device__ __forceinline__ void make_pf2(const SysDesc& s, double x, double y, d
                    0.f);
   hi.w = __uint_as_float(lo_code(lo.x, s.lo_inv_f) | (lo_code(lo.y, s.lo_inv_f) << 10) |
                          (lo_code(lo.z, s.lo_inv_f) << 20));
+}
+
+// A coordinate's FP64 bit pattern from its FP32 mirror h (origin zero) and its
+// step d (DevArrays::pstep) from h's own pattern, that of a nonzero normal h.
+__device__ __forceinline__ double step_coord(float h, int d) {
+  const uint32_t u = __float_as_uint(h);
+  const uint32_t top = ((static_cast<uint32_t>(static_cast<int32_t>(u) >> 3)) & 0x8fffffffu) + 0x38000000u;
+  const uint64_t b = (static_cast<uint64_t>(top) << 32) | static_cast<uint64_t>(u << 29);
+  return __longlong_as_double(static_cast<long long>(b) + static_cast<long long>(d));
+}
+// The steps of a position from its mirrors; .w is set when one does not fit 32
+// bits (a mirror that is zero or not a normal number): those are read as FP64.
+__device__ __forceinline__ int4 make_steps(double x, double y, double z, float4 hi) {
+  const long long d[3] = {__double_as_longlong(x) - __double_as_longlong(step_coord(hi.x, 0)),
+                          __double_as_longlong(y) - __double_as_longlong(step_coord(hi.y, 0)),
+                          __double_as_longlong(z) - __double_as_longlong(step_coord(hi.z, 0))};
+  int4 r = make_int4(static_cast<int>(d[0]), static_cast<int>(d[1]), static_cast<int>(d[2]), 0);
+  r.w = (r.x != d[0] || r.y != d[1] || r.z != d[2]) ? 1 : 0;
+  return r;
 }
 
 __device__ __forceinline__ double widen_f32(float f) {

@@ -20,6 +20,8 @@ struct Extent {
   int force_lanes;   // threads per particle of the FP64 / mixed full-list traversal (1, 2 or 4)
   int far_coords;    // some resident system lies far from the coordinate origin (SysDesc::far_coords)
   int unpacked;      // some resident system reads the residual mirror, not packed residuals (SysDesc::packed_lo)
+  int general;       // some resident system is not one of launch_force_walk's: unpacked, its origin not zero or
+                     // SysDesc::plain_sums
   int dense;         // some resident system's cells hold half of what gives them a sub-grid, on average
   uint32_t list_slot;  // largest list slot of the resident systems
   int force_form;    // kForceThread or kForceStaged (mixed full-list traversal)
@@ -55,6 +57,13 @@ int launch_force(const Extent& ex, const SysDesc* sys, SysState* st, const DevAr
 constexpr uint32_t kMixedSplitMax = 50000;
 int launch_force_mixed(const Extent& ex, const SysDesc* sys, const SysState* st, const DevArrays& a, bool with_pe,
                        bool second_half, int sys_only, cudaStream_t stream);
+
+// The mixed full-list forces of larger batches, one thread per particle
+// (xnb_force_mixed.cu), the same bits again: systems with packed residuals, their
+// origin at zero and terms that PairSum takes (Extent::general is 0; other batches
+// keep the general walk, 1M atoms with energies 794 us where this takes 682).
+int launch_force_walk(const Extent& ex, const SysDesc* sys, const SysState* st, const DevArrays& a, bool with_pe,
+                      bool second_half, int sys_only, cudaStream_t stream);
 
 // FP64 and FP64_EXACT forces over full lists, or FP64 over their lower halves
 // with FP64 reductions into cleared fields (newton; no kick) (xnb_force_pairs.cu).

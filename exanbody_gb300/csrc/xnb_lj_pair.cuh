@@ -31,17 +31,18 @@ __device__ __forceinline__ double rcp_nr(double d) {
   return fma(y, e, y);
 }
 
-// Sum of the FP32 force factors pd of one particle, as FP64 additions in list
-// order would give it, without the FP64 pipe: every pd is a multiple of a
-// quantum Q, 2^23 Q <= |pd| < 2^53 Q, and while the sum of |pd| stays within 2^52 Q
-// every partial sum is exact in FP64, so the sum is Q times the integer sum of
-// pd / Q in any order. A pd outside that range (near the zero crossing of the
-// force, some 10^-5 of the particles) sets `inexact`: that particle is summed in
-// FP64, in order. An FP64 instruction holds a quarter of an SM's FP64 pipe for 64
-// cycles; these are about twelve on the integer pipes.
+// Sum of one FP32 term per pair, as FP64 additions in list order would give it,
+// without the FP64 pipe: every term is a multiple of a quantum Q, 2^23 Q <= |term|
+// < 2^53 Q, and while the sum of |term| stays within 2^52 Q every partial sum is
+// exact in FP64, so the sum is Q times the integer sum of term / Q in any order. A
+// term outside that range (a force factor near its zero crossing, some 10^-5 of
+// the particles; an energy within 3e-6 sigma of a cutoff of 2.5 sigma, some 10^-4)
+// sets `inexact`: that particle is summed in FP64, in order. An FP64 instruction
+// holds a quarter of an SM's FP64 pipe for 64 cycles; these are about twelve on
+// the integer pipes.
 struct PairSum {
-  long long units;  // sum of pd / Q
-  float size;       // sum of |pd|
+  long long units;  // sum of term / Q
+  float size;       // sum of |term|
   bool inexact;
 
   __device__ __forceinline__ void clear() {
@@ -49,24 +50,19 @@ struct PairSum {
     size = 0.f;
     inexact = false;
   }
-  __device__ __forceinline__ void add(const SysDesc& S, float pd) {
-    const uint32_t u = __float_as_uint(pd);
-    const int shift = static_cast<int>((u >> 23) & 0xFFu) - S.psum_exp;
+  __device__ __forceinline__ void add(int exponent, float term) {
+    const uint32_t u = __float_as_uint(term);
+    const int shift = static_cast<int>((u >> 23) & 0xFFu) - exponent;
     inexact = inexact || static_cast<unsigned>(shift) > 29u;
     const int mantissa = static_cast<int>((u & 0x007fffffu) | 0x00800000u);
     const int power = 1 << (shift & 31);
     units += static_cast<long long>(mantissa) * static_cast<long long>((u >> 31) ? -power : power);
-    size += fabsf(pd);
-  }
-  __device__ __forceinline__ void combine(const PairSum& o) {
-    units += o.units;
-    size += o.size;
-    inexact = inexact || o.inexact;
+    size += fabsf(term);
   }
   // (a NaN size is not exact)
-  __device__ __forceinline__ bool exact(const SysDesc& S) const { return !inexact && size <= S.psum_max_f; }
-  __device__ __forceinline__ double value(const SysDesc& S) const {
-    return __dmul_rn(static_cast<double>(units), S.psum_quantum);
+  __device__ __forceinline__ bool exact(const SumRange& R) const { return !inexact && size <= R.limit; }
+  __device__ __forceinline__ double value(const SumRange& R) const {
+    return __dmul_rn(static_cast<double>(units), R.quantum);
   }
 };
 
@@ -103,15 +99,15 @@ __device__ __forceinline__ float image_axis(float hb, float ha, float lb, float 
 // difference for an entry in the same periodic image: hi difference plus the
 // difference of the residuals packed in .w; the FP64 displacement converted for
 // an image entry), the cutoff decided in FP32 outside the proven band and in
-// FP64 inside it, then the FP32 force factor pd, the FP64 accumulation of pd * r_b
-// and the exact one of pd.
+// FP64 inside it, then the FP32 force factor pd and the FP64 accumulation of
+// pd * r_b and pd.
 // PACKED = false (batches holding a system of X >= 1024 sigma, whose packed
 // residuals are too coarse) takes the gathered residual mirrors lb and pal.
 template <bool PE, bool PACKED>
 __device__ __forceinline__ void mixed_pair(const SysDesc& S, uint32_t e, double xb, double yb, double zb, float4 hb,
                                            float4 lb, double xa, double ya, double za, float4 paf, float4 pal,
-                                           double rcut2, double& fx, double& fy, double& fz, PairSum& psum,
-                                           double& pe, float* factor = nullptr) {
+                                           double rcut2, double& fx, double& fy, double& fz, double& psum,
+                                           double& pe) {
   const uint32_t code = e & 31u;
   float dxf, dyf, dzf;
   if (code == static_cast<uint32_t>(kImageCenter)) {
@@ -149,7 +145,7 @@ __device__ __forceinline__ void mixed_pair(const SysDesc& S, uint32_t e, double 
   if (in) {
     // FP64 displacement folded into the FP64 accumulation:
     //   sum_b pd_b (r_b - r_a) = sum_b pd_b r_b - r_a sum_b pd_b,
-    // so a pair costs 3 DFMA instead of 3 DADD + 3 DFMA; the
+    // so a pair costs 3 DFMA + 1 DADD instead of 3 DADD + 3 DFMA; the
     // subtraction happens once per particle (cancellation error
     // <= ~u_64 |r| sum|pd|, about 1e-12 of |F| at box sizes of 10^3 sigma).
     // The hardware reciprocal (within 1 ulp) is part of the FP32 force magnitude.
@@ -162,41 +158,16 @@ __device__ __forceinline__ void mixed_pair(const SysDesc& S, uint32_t e, double 
     fx = fma(pdd, xb, fx);
     fy = fma(pdd, yb, fy);
     fz = fma(pdd, zb, fz);
-    psum.add(S, pd);
-    if (factor) *factor = pd;
-    if (PE) pe += static_cast<double>(0.5f * fmaf(S.eps4_f * s6, s6 - 1.0f, -S.e_shift_f));
+    psum += pdd;
+    if (PE) pe += widen_f32_fast(0.5f * fmaf(S.eps4_f * s6, s6 - 1.0f, -S.e_shift_f));
   }
-}
-
-// Sum of pd in FP64, in list order (where PairSum is not exact).
-template <bool PACKED>
-static __device__ __noinline__ double psum_in_order(const SysDesc& S, const double* rx, const double* ry,
-                                                    const double* rz, const float4* pf, const float4* pflo, uint32_t i,
-                                                    const uint32_t* list, uint32_t n) {
-  const double xa = rx[i], ya = ry[i], za = rz[i];
-  const float4 hi = pf[i], lo = PACKED ? make_float4(0.f, 0.f, 0.f, 0.f) : pflo[i];
-  double psum = 0.0;
-  for (uint32_t k = 0; k < n; ++k) {
-    const uint32_t e = list[k], j = S.part_base + (e >> 5);
-    double fx = 0.0, fy = 0.0, fz = 0.0, pe = 0.0;
-    PairSum one;
-    one.clear();
-    float pd = 0.f;
-    mixed_pair<false, PACKED>(S, e, rx[j], ry[j], rz[j], pf[j], PACKED ? make_float4(0.f, 0.f, 0.f, 0.f) : pflo[j], xa,
-                              ya, za, hi, lo, S.rcut2, fx, fy, fz, one, pe, &pd);
-    psum += widen_f32_fast(pd);
-  }
-  return psum;
 }
 
 // A particle's sums to its force (and energy): the FP64 displacement folded out
 // of sum pd (r_b - r_a), the division by the mass, the second-half kick.
-template <bool PE, bool KICK, bool PACKED>
-__device__ __forceinline__ void finish_mixed(const SysDesc& S, const DevArrays& a, uint32_t i, const uint32_t* list,
-                                             uint32_t n, double fx, double fy, double fz, const PairSum& sum,
-                                             double pe) {
-  const double psum = sum.exact(S) ? sum.value(S)
-                                   : psum_in_order<PACKED>(S, a.rx, a.ry, a.rz, a.pf, a.pflo, i, list, n);
+template <bool PE, bool KICK>
+__device__ __forceinline__ void finish_mixed(const SysDesc& S, const DevArrays& a, uint32_t i, double fx, double fy,
+                                             double fz, double psum, double pe) {
   fx = fma(-a.rx[i], psum, fx);
   fy = fma(-a.ry[i], psum, fy);
   fz = fma(-a.rz[i], psum, fz);
@@ -233,17 +204,15 @@ __device__ __forceinline__ void finish_mixed(const SysDesc& S, const DevArrays& 
 // the cutoff decision is made in FP32 where a proven margin allows and in FP64
 // otherwise, so the pair set is the FP64 one. The displacement is applied once
 // per particle (sum pd*r_b - r_a*sum pd, all in FP64) and the FP32 factor is
-// widened, and summed (PairSum), on the integer pipes: a pair costs 3 DFMA on the
-// FP64 pipe.
-// (The FP64 paths: xnb_force_pairs.cuh; small mixed batches, with these bits:
+// widened on the integer pipes: a pair costs 3 DFMA and 1 DADD on the FP64 pipe.
+// (The FP64 paths: xnb_force_pairs.cuh; the common mixed batches, with these bits:
 // xnb_force_mixed.cu.)
 template <bool PE, bool KICK, bool PACKED = true>
 struct LJForce {
   const SysDesc* __restrict__ sys;
   DevArrays a;
   struct Acc {
-    double fx, fy, fz, pe;
-    PairSum psum;
+    double fx, fy, fz, psum, pe;
   };
 
   __device__ __forceinline__ double rcut2(const pair::ParticleContext& c) const { return sys[c.sys].rcut2; }
@@ -252,8 +221,7 @@ struct LJForce {
     return S.rc2_f + S.pre_margin_f;
   }
   __device__ __forceinline__ bool start(Acc& q, const pair::ParticleContext&) const {
-    q.fx = q.fy = q.fz = q.pe = 0.0;
-    q.psum.clear();
+    q.fx = q.fy = q.fz = q.psum = q.pe = 0.0;
     return true;
   }
   __device__ __forceinline__ void entry(Acc& q, const pair::ParticleContext& c, const pair::RawEntry& r) const {
@@ -265,11 +233,11 @@ struct LJForce {
     q.fx += o.fx;
     q.fy += o.fy;
     q.fz += o.fz;
+    q.psum += o.psum;
     q.pe += o.pe;
-    q.psum.combine(o.psum);
   }
   __device__ __forceinline__ void stop(Acc& q, const pair::ParticleContext& c) const {
-    finish_mixed<PE, KICK, PACKED>(sys[c.sys], a, c.i, c.list, c.n, q.fx, q.fy, q.fz, q.psum, q.pe);
+    finish_mixed<PE, KICK>(sys[c.sys], a, c.i, q.fx, q.fy, q.fz, q.psum, q.pe);
   }
 };
 

@@ -82,6 +82,7 @@ __device__ __forceinline__ void first_half_body(uint32_t n_part, int nsys, const
         make_pf2(S, x, y, z, hi, lo);
         a.pf[i] = hi;
         a.pflo[i] = lo;
+        a.pstep[i] = make_steps(x, y, z, hi);
         cur_hi = hi;
       } else if (!EXACT && trigger) {
         cur_hi = a.pf[i];
@@ -559,6 +560,8 @@ int launch_force(const Extent& ex, const SysDesc* sys, SysState* st, const DevAr
     return launch_force_staged(ex, sys, st, a, with_pe, second_half, sys_only, stream);
   if (precision == kMixed && !ex.unpacked && ex.n_part <= kMixedSplitMax)
     return launch_force_mixed(ex, sys, st, a, with_pe, second_half, sys_only, stream);
+  if (precision == kMixed && !ex.general && ex.force_lanes == 1)
+    return launch_force_walk(ex, sys, st, a, with_pe, second_half, sys_only, stream);
   if (precision != kMixed)
     return launch_force_pairs(ex, sys, st, a, precision, false, with_pe, second_half, sys_only, stream);
   if (with_pe && second_half) force_dispatch<true, true>(ex, sys, st, a, sys_only, stream);
