@@ -49,12 +49,12 @@ int launch_force(const Extent& ex, const SysDesc* sys, SysState* st, const DevAr
 
 // The mixed full-list forces in the two-stage form (xnb_force_mixed.cu): the same
 // bits as one thread per particle, faster while the particles are too few to fill
-// the GPU that way. Per call, two-stage / one-thread: 864 atoms 10 / 87 us, 32,000
-// 43 / 96 us, 62,500 72 / 105 us, 131,072 135 / 137 us (178 / 165 us with
-// energies). The line lies where three batches stepping at once on their own
-// streams break even: 50 steps of 32,000 atoms 2.84 / 3.50 ms, 5 steps of 63,000
-// 0.594 / 0.586 ms.
-constexpr uint32_t kMixedSplitMax = 50000;
+// the GPU that way. Per call, two-stage / launch_force_walk: 864 atoms 10 / 87 us,
+// 32,000 43 / 106 us, 62,500 72 / 117 us, 87,808 96 / 121 us, 131,072 135 / 146 us
+// (170 / 157 us with energies). The line lies where three batches stepping at once
+// on their own streams break even: 10 steps of 32,000 atoms 453 / 687 us, 62,500
+// 896 / 939 us, 87,808 1251 / 1160 us.
+constexpr uint32_t kMixedSplitMax = 70000;
 int launch_force_mixed(const Extent& ex, const SysDesc* sys, const SysState* st, const DevArrays& a, bool with_pe,
                        bool second_half, int sys_only, cudaStream_t stream);
 

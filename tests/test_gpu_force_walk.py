@@ -1,4 +1,4 @@
-"""The one-thread mixed walk of larger batches (above 50,000 particles) against
+"""The one-thread mixed walk of larger batches (above 70,000 particles) against
 the sequential FP64 sums of the staged form: the same bits with images on every
 side, coordinates that are zero (no FP32 mirror to step from), sums outside the
 exact integer range (close contacts), odd list lengths, a partly filled block,
@@ -13,14 +13,14 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("noise,keep,rcut,mass,shift", [
-    (0.05, None, 2.5, 1.0, 0.0),    # a thermal fluid: 55,296 atoms
+    (0.05, None, 2.5, 1.0, 0.0),    # a thermal fluid: 70,304 atoms
     (0.0, None, 2.5, 1.0, 0.0),     # the lattice itself: a face of atoms at coordinate 0 on each axis
-    (0.2, 50001, 2.5, 2.0, 0.0),    # overlapping atoms, one past the two-stage form's range
+    (0.2, 70001, 2.5, 2.0, 0.0),    # overlapping atoms, one past the two-stage form's range
     (0.05, None, 2.5, 1.0, -17.0),  # origin off zero: the general walk
     (0.05, None, 3.2, 1.0, 0.0),    # a long cutoff: the general walk
 ])
 def test_walk_equals_the_sequential_sums(noise, keep, rcut, mass, shift):
-    w = workloads.lj_fcc_system(24, 0.8442, 1.2, 31, rcut=rcut)
+    w = workloads.lj_fcc_system(26, 0.8442, 1.2, 31, rcut=rcut)
     r, v, ids = (w[k][:keep] for k in ("r", "v", "id"))
     r = r + np.random.default_rng(5).normal(0.0, 1.0, r.shape) * noise if noise else r - r.min(axis=0)
     geom = dict(w["geom"])
