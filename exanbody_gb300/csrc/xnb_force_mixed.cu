@@ -210,18 +210,17 @@ void go(const Extent& ex, const SysDesc* sys, const SysState* st, const DevArray
 }
 
 // ---------------------------------------------------------------------------
-// One thread per particle, for batches that fill the GPU so: every list entry
-// once, two at a time, their mirrors and position steps (DevArrays::pstep) in
-// flight together. A pair costs 3 DFMA on the FP64 pipe, which bounds the walk: a
-// warp makes about 100 rounds of three (its longest list), and at one million
-// atoms the pipe is busy 82% of the time (the general walk, which marks the
-// entries near the cutoff first and gathers those a second time: 73 rounds, the
+// One thread per particle, for batches of many waves: every list entry once, two at
+// a time, their mirrors and position steps (DevArrays::pstep) in flight together;
+// a pair's FP64 position is formed only within the cutoff. A pair costs 3 DFMA on
+// the FP64 pipe, which bounds the walk: a warp makes about 100 rounds of three (its
+// longest list), and at one million atoms the pipe is busy 82% of the time (the
+// marking walk gathers the entries near the cutoff a second time: 73 rounds, the
 // pipe at 58% and the L1 data stage at 66%). 64 registers hold 16 blocks of 64
-// threads per SM. General walk / this one: 25 steps of 4M atoms 74.9 / 69.4 ms
-// (three such batches at once 75.0 / 73.7); 1M atoms with energies 728 / 683 us; a
-// batch of 96 small systems, 20 steps, three at once 45.2 / 42.6 ms. With 56
-// registers 71.7 ms and 773 us, four entries at a time 80.8 ms.
-// A pair's FP64 position is needed only within the cutoff.
+// threads per SM. Marking walk with the sums of PairSum / this one: 25 steps of 4M
+// atoms 74.9 / 69.4 ms (three such batches at once 75.0 / 73.7); 1M atoms with
+// energies 728 / 683 us; a batch of 96 small systems, 20 steps, three at once 45.2 /
+// 42.6 ms. With 56 registers 71.7 ms and 773 us, four entries at a time 80.8 ms.
 struct WalkParticle {
   const double* rx;
   const double* ry;

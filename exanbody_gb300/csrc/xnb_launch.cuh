@@ -49,19 +49,26 @@ int launch_force(const Extent& ex, const SysDesc* sys, SysState* st, const DevAr
 
 // The mixed full-list forces in the two-stage form (xnb_force_mixed.cu): the same
 // bits as one thread per particle, faster while the particles are too few to fill
-// the GPU that way. Per call, two-stage / launch_force_walk: 864 atoms 10 / 87 us,
-// 32,000 43 / 106 us, 62,500 72 / 117 us, 87,808 96 / 121 us, 131,072 135 / 146 us
-// (170 / 157 us with energies). The line lies where three batches stepping at once
-// on their own streams break even: 10 steps of 32,000 atoms 453 / 687 us, 62,500
-// 896 / 939 us, 87,808 1251 / 1160 us.
-constexpr uint32_t kMixedSplitMax = 70000;
+// the GPU that way. Per call, two-stage / one-thread: 864 atoms 10 / 87 us, 32,000
+// 43 / 96 us, 62,500 72 / 105 us, 131,072 135 / 137 us (178 / 165 us with
+// energies). The line lies where three batches stepping at once on their own
+// streams break even: 50 steps of 32,000 atoms 2.84 / 3.50 ms, 5 steps of 63,000
+// 0.594 / 0.586 ms, of eight systems of 2,048 to 16,384 atoms in a batch 0.595 / 0.552 ms.
+constexpr uint32_t kMixedSplitMax = 50000;
 int launch_force_mixed(const Extent& ex, const SysDesc* sys, const SysState* st, const DevArrays& a, bool with_pe,
                        bool second_half, int sys_only, cudaStream_t stream);
 
-// The mixed full-list forces of larger batches, one thread per particle
-// (xnb_force_mixed.cu), the same bits again: systems with packed residuals, their
-// origin at zero and terms that PairSum takes (Extent::general is 0; other batches
-// keep the general walk, 1M atoms with energies 794 us where this takes 682).
+// The mixed full-list forces of large batches, each list entry visited once by one
+// thread per particle (xnb_force_mixed.cu), the same bits again: systems with
+// packed residuals, their origin at zero and terms that PairSum takes
+// (Extent::general is 0; other batches keep the marking walk of
+// xnb_step_kernels.cu). The marking walk has the shorter chain per particle and
+// wins while a call is a few waves of blocks. A call, marking / single-visit: 78,732
+// atoms 113 / 135 us, 157,216 179 / 195 us, 364,500 299 / 310 us, 562,432 402 / 404
+// us (with energies 443 / 440), 1M 639 / 629 us (710 / 690), 2M 1201 / 1154 us (1334
+// / 1253). 10 steps, three batches at once: 562,432 atoms 5.31 / 4.70 ms, 2M 19.3 /
+// 16.3 ms.
+constexpr uint32_t kMixedWalkMin = 500000;
 int launch_force_walk(const Extent& ex, const SysDesc* sys, const SysState* st, const DevArrays& a, bool with_pe,
                       bool second_half, int sys_only, cudaStream_t stream);
 

@@ -560,7 +560,7 @@ int launch_force(const Extent& ex, const SysDesc* sys, SysState* st, const DevAr
     return launch_force_staged(ex, sys, st, a, with_pe, second_half, sys_only, stream);
   if (precision == kMixed && !ex.unpacked && ex.n_part <= kMixedSplitMax)
     return launch_force_mixed(ex, sys, st, a, with_pe, second_half, sys_only, stream);
-  if (precision == kMixed && !ex.general && ex.force_lanes == 1)
+  if (precision == kMixed && !ex.general && ex.force_lanes == 1 && ex.n_part >= kMixedWalkMin)
     return launch_force_walk(ex, sys, st, a, with_pe, second_half, sys_only, stream);
   if (precision != kMixed)
     return launch_force_pairs(ex, sys, st, a, precision, false, with_pe, second_half, sys_only, stream);

@@ -1,4 +1,4 @@
-"""The two-stage mixed force kernel (batches of up to 70,000 particles) against
+"""The two-stage mixed force kernel (batches of up to 50,000 particles) against
 the sequential walk of the staged form: the same bits at the edges of its rows
 and blocks -- particle counts off the block's group, lists longer than one
 chunk of shared memory, lists of none and one pair, images on every side."""
