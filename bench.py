@@ -41,10 +41,16 @@ sys.path.insert(0, ROOT)
 FLOP64_PER_ATOM_FP64_PATH = 669.6
 FLOP64_PER_ATOM_MIXED = 282.2
 FLOP32_PER_ATOM_MIXED = 387.4
-# DRAM bytes (read + write) per atom of one mixed k_force launch, from an ncu capture of
-# the 256,000-atom case of this workload (FCC 40^3); traffic grows with the atom count at
+# DRAM bytes (read + write) per atom of one mixed k_force_walk launch, from an ncu capture of
+# the 1,000,188-atom case of this workload (FCC 63^3); traffic grows with the atom count at
 # fixed density, so a launch moves this many bytes per atom.
-FORCE_DRAM_BYTES_PER_ATOM = 520.0
+FORCE_DRAM_BYTES_PER_ATOM = 479.0
+
+
+def mixed_force_kernel(n):
+    """Kernel of the mixed full-list forces of a batch of n particles (kMixedSplitMax, kMixedWalkMin)."""
+    return "k_force_mixed" if n <= 50000 else "k_force<mixed>" if n < 500000 else "k_force_walk"
+
 
 WORKLOAD = dict(n=100, rho=0.8442, T=1.44, seed=12345, rcut=2.5, skin=0.3, dt=0.005)
 METRIC = "atom-steps/s, 4M-atom LJ MD step (mixed precision; FP64 path and force error reported beside it)"
@@ -103,7 +109,7 @@ def parse():
     ap.add_argument("--build-form", default="", choices=["", "rows", "warp", "half"],
                     help="neighbour-build kernel (empty: library default)")
     ap.add_argument("--force-lanes", type=int, default=0, choices=[0, 1, 2, 4],
-                    help="threads per particle of the FP64 / mixed force traversal (0: library default)")
+                    help="threads per particle of the mixed force traversal (0: library default)")
     ap.add_argument("--force-form", default="", choices=["", "thread", "staged"],
                     help="mixed full-list force traversal form (empty: library default)")
     ap.add_argument("--cell-factor", type=float, default=1.0,
@@ -511,14 +517,14 @@ def run_ours(args):
             "gpu_launches": launches,
             "roofline": {"bound": "fp64",
                          "kernel": ("k_force_half<mixed> (+ zero/finish launches)" if MIXED & xnb.PREC_NEWTON
-                                    else "k_force<mixed>"),
+                                    else mixed_force_kernel(N)),
                          "achieved": achieved, "peak": peak64,
                          "unit": "TFLOP/s", "frac": achieved / peak64,
                          "peak_source": "cuBLAS DGEMM 4096^3 measured in this run",
                          "ms_per_launch": ms_force, "ms_per_launch_fp64_kernel": ms_force64,
                          "traffic": FORCE_DRAM_BYTES_PER_ATOM * N,
                          "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum per atom on the "
-                                           "256,000-atom case, scaled to %d atoms" % N,
+                                           "1,000,188-atom case, scaled to %d atoms" % N,
                          "hbm": {"achieved_gbs": FORCE_DRAM_BYTES_PER_ATOM * N / (ms_force * 1e-3) / 1e9,
                                  "peak_gbs": hbm_peak_gbs(),
                                  "frac": FORCE_DRAM_BYTES_PER_ATOM * N / (ms_force * 1e-3) / 1e9 / hbm_peak_gbs()}},
@@ -734,7 +740,7 @@ def run_snap(args):
                      "speedup_mixed_vs_fp64": ms64 / ms},
             "force_error_mixed_vs_fp64": {"max": err_max, "rms": err_rms, "tolerance": 1e-5},
             "clocks": ck.summary(), "e2e": e2e, "gpu_launches": launches,
-            "roofline": {"bound": "fp64", "kernel": "k_snap<double> (the FP64 path)", "achieved": achieved,
+            "roofline": {"bound": "fp64", "kernel": "k_snap64 (the FP64 path)", "achieved": achieved,
                          "peak": peak64, "unit": "TFLOP/s", "frac": achieved / peak64,
                          "peak_source": "cuBLAS DGEMM 4096^3 measured in this run",
                          "flop_per_atom": flop, "ms_per_launch": ms_force64, "ms_per_launch_mixed": ms_force,

@@ -736,8 +736,10 @@ __global__ void __launch_bounds__(128, 8)
 // band around nbh^2 (both then take the reference's FP64 decision). A cell whose
 // kept candidates exceed the stage (cap) is appended to a.nbr_wide for
 // k_neighbors.
-// The build is bound by instruction issue (479 warp instructions per atom before
-// the chunk test was split into nbr_chunk_clear and nbr_chunk). Four particles
+// The build is bound by instruction issue: 418 warp instructions per atom, the
+// schedulers busy 66% of the time (1,972,156 atoms: 1.52 ms with every candidate of
+// the 27 cells tested, six particles per load and one chunk test; 1.29 with the box
+// and the runs, 1.03 with nbr_chunk_clear, its rarely true conditions moved out). Four particles
 // per staged load fit 95 registers, 5 blocks of 4 warps per SM; six spill there
 // (1.18 against 1.03 ms per build of 1,972,156 atoms), four at 6 blocks 1.07 ms.
 // The last particles of a cell are tested two at a time, not padded to four.
@@ -1051,7 +1053,8 @@ __global__ void __launch_bounds__(128, 5)
 // build that follows) of a small batch in one cooperative launch. A step without
 // a rebuild costs one launch that returns at once, where the separate kernels
 // cost twelve (0.7 us each inside a graph, 2.3 us when launched one by one); a
-// rebuild costs six grid barriers. The phases are the separate kernels' bodies.
+// rebuild costs six grid barriers: 50 steps of 864 atoms 844 -> 511 us, of 32,000
+// 2.78 -> 2.42 ms. The phases are the separate kernels' bodies.
 // BUILD: the lists of the flagged systems too (the warp-per-cell form without
 // sub-cell pruning, then the cells it passes on), two more barriers: a step
 // without a rebuild is then three launches, push, this one and the forces.

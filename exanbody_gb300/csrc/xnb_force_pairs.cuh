@@ -19,6 +19,9 @@
 //     particle; a 4 x 4 transpose hands each lane one component of four
 //     consecutive pairs, which it adds in list order: the bits of the sequential
 //     walk.
+// The FP64 pipe is busy 85% of the time (kFp64, 119,164 atoms: 422 us with one
+// thread per particle, 282 now). Newton half lists, 5 steps of 256,000 atoms: 3.94
+// -> 1.89 ms; kFp64Exact, 5 host-synchronised steps of 8,788 atoms: 767 -> 424 us.
 #pragma once
 
 #include "xnb_lj_pair.cuh"

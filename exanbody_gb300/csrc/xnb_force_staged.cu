@@ -1,7 +1,7 @@
 // Mixed-precision Lennard-Jones traversal over cell segments staged in shared
 // memory (XNB_FORCE_STAGED).
 //
-// The one-thread-per-particle traversal (xnb_step_kernels.cu) gathers every
+// The marking one-thread traversal (xnb_step_kernels.cu) gathers every
 // neighbour's FP32 mirror (prefilter) and FP64 position and mirrors (marked
 // entries) from global memory: at 4M atoms it is bound by the latency and L1
 // throughput of those gathers, not by its FP64 work. Here a block takes a

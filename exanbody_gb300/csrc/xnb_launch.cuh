@@ -17,7 +17,7 @@ struct Extent {
   int nsys;
   int sm_count;
   int force_block;   // threads per block of the force traversal (multiple of 32, <= 256)
-  int force_lanes;   // threads per particle of the FP64 / mixed full-list traversal (1, 2 or 4)
+  int force_lanes;   // threads per particle of the mixed full-list traversal above kMixedSplitMax (1, 2 or 4)
   int far_coords;    // some resident system lies far from the coordinate origin (SysDesc::far_coords)
   int unpacked;      // some resident system reads the residual mirror, not packed residuals (SysDesc::packed_lo)
   int general;       // some resident system is not one of launch_force_walk's: unpacked, its origin not zero or

@@ -1,5 +1,6 @@
-// Pieces of the Lennard-Jones pair body shared by the force traversals
-// (xnb_step_kernels.cu: one thread per particle over global memory;
+// Pieces of the Lennard-Jones pair body shared by the mixed force traversals
+// (xnb_step_kernels.cu: one thread per particle, marking first; xnb_force_mixed.cu:
+// two stages, and one thread per particle visiting each entry once;
 // xnb_force_staged.cu: cell segments staged in shared memory).
 #pragma once
 

@@ -144,6 +144,7 @@ __global__ void __launch_bounds__(256)
   first_half_body<EXACT>(n_part, nsys, sys, st, a, push_r, push_v, trigger, scale_r, scale_v, sys_only, nullptr);
 }
 
+// The marking walk: the mixed batches that neither form of xnb_force_mixed.cu takes.
 // 72 registers: 7 blocks of 128 threads per SM (measured faster than the
 // unconstrained 79 despite a few spilled bytes).
 template <bool PE, bool KICK, bool PACKED = true>

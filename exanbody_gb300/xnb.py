@@ -467,7 +467,8 @@ class Batch:
         _ck(self.lib.xnb_batch_set_tuning(self.h, int(stage_cap), int(force_block)))
 
     def set_force_lanes(self, lanes):
-        """Threads per particle (1, 2 or 4) of the FP64 / mixed full-list force traversal."""
+        """Threads per particle (1, 2 or 4) of the mixed full-list force traversal of batches of more than 50,000
+        particles (others spread a list over threads by themselves)."""
         _ck(self.lib.xnb_batch_set_force_lanes(self.h, int(lanes)))
 
     def set_force_form(self, form):

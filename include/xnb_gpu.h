@@ -215,16 +215,17 @@ typedef struct xnb_tuning {
   int32_t trials;             /* configurations timed */
   double atom_steps_per_s;    /* the chosen configuration's measured rate */
   int32_t build_form;         /* XNB_BUILD_ROWS or XNB_BUILD_WARP */
-  int32_t force_lanes;        /* threads per particle of the FP64 / mixed full-list force traversal */
+  int32_t force_lanes;        /* threads per particle of the mixed full-list force traversal */
   int32_t force_form;         /* the batch's force form (XNB_FORCE_THREAD or XNB_FORCE_STAGED; not searched) */
   int32_t reserved;
 } xnb_tuning;
 
-/* Threads per particle (1, 2 or 4) of the FP64 and mixed full-list force
- * traversals: the particle's list is split in 8-entry blocks dealt round-robin
- * to the threads and their partial sums combined in a fixed order, so results
- * are reproducible and agree with one thread per particle to rounding.
- * FP64_EXACT always runs one thread per particle. */
+/* Threads per particle (1, 2 or 4) of the mixed full-list force traversal of
+ * batches of more than 50,000 particles: the particle's list is split in 8-entry
+ * blocks dealt round-robin to the threads and their partial sums combined in a
+ * fixed order, so results are reproducible and agree with one thread per particle
+ * to rounding. Smaller mixed batches and the FP64 paths spread a particle's list
+ * over threads by themselves, whatever is set here, with the same results. */
 int xnb_batch_set_force_lanes(xnb_batch* b, int32_t lanes);
 
 /* Form of the mixed-precision full-list force traversal:
