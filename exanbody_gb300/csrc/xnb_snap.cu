@@ -105,7 +105,7 @@ __device__ __forceinline__ void geometry_derivative(Geo& g, double x, double y, 
   g.db[1].r += r0inv;
 }
 
-__device__ __forceinline__ Geo geometry(double x, double y, double z, double rcut, const SnapArgs& t, bool deriv) {
+__device__ __forceinline__ Geo geometry(double x, double y, double z, double rcut, const SnapArgs& t) {
   Geo g;
   const double rsq = fma(x, x, fma(y, y, z * z));
   const double r = sqrt(rsq);
@@ -128,7 +128,6 @@ __device__ __forceinline__ Geo geometry(double x, double y, double z, double rcu
   }
   g.r0inv = r0inv;
   g.z0 = z0;
-  if (deriv) geometry_derivative(g, x, y, z, r0inv, z0, rscale0);
   return g;
 }
 
@@ -226,11 +225,10 @@ __global__ void __launch_bounds__(kSnapThreads)
   double* nx = sm;
   double* ny = nx + kSnapMaxNbr;
   double* nz = ny + kSnapMaxNbr;
-  double* nspare = nz + kSnapMaxNbr;                                       // (unused double slot)
-  uint32_t* nj = reinterpret_cast<uint32_t*>(nspare + kSnapMaxNbr);        // kSnapMaxNbr u32
+  double* ngeo = nz + kSnapMaxNbr;                                         // 4 per neighbour: r0inv, z0, sfac, dsfac
+  uint32_t* nj = reinterpret_cast<uint32_t*>(ngeo + 4 * kSnapMaxNbr);      // kSnapMaxNbr u32
   uint8_t* nt = reinterpret_cast<uint8_t*>(nj + kSnapMaxNbr);              // kSnapMaxNbr u8
-  double* red = nspare + kSnapMaxNbr + kSnapMaxNbr / 2 + kSnapMaxNbr / 8;  // kSnapThreads x 5
-  double* misc = red + kSnapThreads * 5;                                    // 8 doubles: fsum[3], wsum[4]
+  double* misc = ngeo + 4 * kSnapMaxNbr + kSnapMaxNbr / 2 + kSnapMaxNbr / 8;  // 8 doubles: fsum[3], wsum[4]
   int* icnt = reinterpret_cast<int*>(misc + 8);                             // 8 ints
   R* nab = reinterpret_cast<R*>(misc + 12);                                // 4 per neighbour: a, b
   R* nsw = nab + 4 * kSnapMaxNbr;                                           // wj sfac per neighbour
@@ -238,7 +236,9 @@ __global__ void __launch_bounds__(kSnapThreads)
   R* yv = utot + 2 * t.nu_full;                                             // 2 nu
   R* uacc = yv + 2 * nu;                                                    // 2 nu
   R* uall = uacc + 2 * nu;                                                  // group x 2 nu
-  R* adj = uall + static_cast<size_t>(group) * 2 * nu;                      // group x 2 x 2 lvl_max
+  R* adj = uall + static_cast<size_t>(group) * 2 * nu;                      // group x (top level, the one below)
+  const int adj_stride = 2 * (lvl_max + (J > 0 ? nunique(J - 1) : 1));
+  double* red = reinterpret_cast<double*>(adj);                             // kSnapThreads x 5, once a round's adjoint is done
 
   for (uint32_t i = blockIdx.x; i < n_part; i += gridDim.x) {
     const uint32_t c = a.pcell[i];
@@ -316,6 +316,25 @@ __global__ void __launch_bounds__(kSnapThreads)
       continue;
     }
 
+    // ---- every neighbour's geometry, once, a lane each: its FP64 chain (two
+    //      sincos, divisions) is a warp instruction per 64 cycles whatever the
+    //      lanes in it. By one lane of each neighbour's own, in every warp and
+    //      round, and again for the forces, it took a fifth of the time (8,192 Mo
+    //      atoms 901 -> 722 us) ----
+    for (int q = tid; q < nn; q += kSnapThreads) {
+      const double rcut = (radi + t.radelem[nt[q]]) * t.rcutfac;
+      const Geo geo = geometry(nx[q], ny[q], nz[q], rcut, t);
+      nab[4 * q] = R(geo.a.r);
+      nab[4 * q + 1] = R(geo.a.i);
+      nab[4 * q + 2] = R(geo.b.r);
+      nab[4 * q + 3] = R(geo.b.i);
+      nsw[q] = R(t.wj[nt[q]] * geo.sfac);
+      ngeo[4 * q] = geo.r0inv;
+      ngeo[4 * q + 1] = geo.z0;
+      ngeo[4 * q + 2] = geo.sfac;
+      ngeo[4 * q + 3] = geo.dsfac;
+    }
+
     // ---- U_tot = self + sum_j wj sfac U_j, neighbours in rounds of `group` ----
     for (int e = tid; e < 2 * nu; e += kSnapThreads) uacc[e] = R(0);
     for (int q0 = 0; q0 < nn; q0 += group) {
@@ -324,15 +343,7 @@ __global__ void __launch_bounds__(kSnapThreads)
       const int g = tid / lpn, slot = tid % lpn;
       const bool active = g < gr;
       R* ug = uall + static_cast<size_t>(active ? g : 0) * 2 * nu;
-      if (active && slot == 0) {  // the neighbour's Cayley-Klein parameters, once
-        const int q = q0 + g;
-        const double rcut = (radi + t.radelem[nt[q]]) * t.rcutfac;
-        const Geo geo = geometry(nx[q], ny[q], nz[q], rcut, t, false);
-        nab[4 * q] = R(geo.a.r);
-        nab[4 * q + 1] = R(geo.a.i);
-        nab[4 * q + 2] = R(geo.b.r);
-        nab[4 * q + 3] = R(geo.b.i);
-        nsw[q] = R(t.wj[nt[q]] * geo.sfac);
+      if (active && slot == 0) {
         ug[0] = R(1);
         ug[1] = R(0);
       }
@@ -433,7 +444,7 @@ __global__ void __launch_bounds__(kSnapThreads)
       const int g = tid / lpn, slot = tid % lpn;
       const bool active = g < gr;
       R* ug = uall + static_cast<size_t>(active ? g : 0) * 2 * nu;
-      R* adj0 = adj + static_cast<size_t>(active ? g : 0) * 4 * lvl_max;
+      R* adj0 = adj + static_cast<size_t>(active ? g : 0) * adj_stride;
       R* adj1 = adj0 + 2 * lvl_max;
       CX<R> ca{R(0), R(0)}, cb{R(0), R(0)};
       if (active) {
@@ -553,7 +564,10 @@ __global__ void __launch_bounds__(kSnapThreads)
         for (int sl = 0; sl < lpn; ++sl)
           for (int k = 0; k < 5; ++k) v[k] += red[(tid * lpn + sl) * 5 + k];
         const double rcut = (radi + t.radelem[nt[q]]) * t.rcutfac;
-        const Geo geo = geometry(nx[q], ny[q], nz[q], rcut, t, true);
+        Geo geo;
+        geometry_derivative(geo, nx[q], ny[q], nz[q], ngeo[4 * q], ngeo[4 * q + 1], t.rfac0 * M_PI / (rcut - t.rmin0));
+        geo.sfac = ngeo[4 * q + 2];
+        geo.dsfac = ngeo[4 * q + 3];
         const double wjq = t.wj[nt[q]];
         double f[3];
         for (int k = 0; k < 3; ++k) {
@@ -789,7 +803,7 @@ __global__ void __launch_bounds__(kSnapThreads)
     }
     for (int q = tid; q < nn; q += kSnapThreads) {
       SnapNbr& o = nb[q];
-      const Geo g = geometry(o.x, o.y, o.z, (radi + t.radelem[o.type]) * t.rcutfac, t, false);
+      const Geo g = geometry(o.x, o.y, o.z, (radi + t.radelem[o.type]) * t.rcutfac, t);
       o.a = g.a;
       o.b = g.b;
       o.r0inv = g.r0inv;
@@ -1369,10 +1383,14 @@ int snap_build(const xnb_snap_params& p, int device, SnapArgs& t, std::vector<vo
     err = "device memory for the SNAP tables";
     return XNB_ERR_NOMEM;
   }
-  // FP32 kernel: a double part (environment, reductions) and a compute-type part:
+  // FP32 kernel: a double part (environment, geometry) and a compute-type part:
   // U_tot, Y, the U accumulator and, per neighbour of a round, its forward U
-  // (unique half of every level) and two adjoint levels; rounds of at most 32
-  // within ~54 KB (four CTAs per SM with the per-CTA reserve)
+  // (unique half of every level) and two adjoint levels, which the force
+  // reduction overwrites; rounds of at most 32. The kernel waits for shared memory
+  // and barriers, so more CTAs per SM pay (twojmax 6, 8,192 Mo atoms: 722 us with
+  // four, 630 with five), but a second round costs more (930 us with six, whose
+  // rounds hold 20 of 26 neighbours): as many CTAs as leave the rounds alone, at
+  // least four.
   const int lvl_max = nunique(J);
   auto plan = [&](size_t base, size_t per, size_t budget, int most, int& group, size_t& bytes) {
     long long grp = budget > base ? static_cast<long long>((budget - base) / std::max<size_t>(per, 1)) : 1;
@@ -1380,9 +1398,21 @@ int snap_build(const xnb_snap_params& p, int device, SnapArgs& t, std::vector<vo
     group = static_cast<int>(grp);
     bytes = base + per * group;
   };
-  plan((4 * kSnapMaxNbr + kSnapMaxNbr / 2 + kSnapMaxNbr / 8 + kSnapThreads * 5 + 12) * 8 +
-           (5 * kSnapMaxNbr + 2 * t.nu_full + 4 * t.nu_unique) * 4,
-       (2 * t.nu_unique + 4 * lvl_max) * 4, 54 * 1024, kSnapMaxGroup, t.group_f, t.smem_bytes_f);
+  const size_t base_f = (7 * kSnapMaxNbr + kSnapMaxNbr / 2 + kSnapMaxNbr / 8 + 12) * 8 +
+                        (5 * kSnapMaxNbr + 2 * t.nu_full + 4 * t.nu_unique) * 4;
+  const size_t u_f = 2 * t.nu_unique * 4, adj_f = 2 * (lvl_max + nunique(std::max(J - 1, 0))) * 4;
+  // rounds of what 54 KB hold beside a reduction buffer of their own: a neighbour
+  // sum's order, and so its FP32 rounding, follows from the rounds
+  int most = 1;
+  size_t unused = 0;
+  plan(base_f - 3 * kSnapMaxNbr * 8 + kSnapThreads * 5 * 8, u_f + 4 * lvl_max * 4, 54 * 1024, kSnapMaxGroup, most,
+       unused);
+  for (int ctas = 8; ctas >= 4; --ctas) {
+    const size_t limit = 228 * 1024 / ctas - 1024;
+    plan(base_f, u_f + adj_f, limit, most, t.group_f, t.smem_bytes_f);
+    t.smem_bytes_f = std::max(t.smem_bytes_f, base_f + t.group_f * u_f + kSnapThreads * 5 * sizeof(double));
+    if (t.group_f == most && t.smem_bytes_f <= limit) break;
+  }
   // FP64 kernel: every neighbour's levels below the top; two CTAs per SM
   plan(kSnapMaxNbr * sizeof(SnapNbr) +
            (2 * t.nu_full + 4 * t.nu_unique + kSnapThreads * 4 + 4 * kSnapWarps + 4) * sizeof(double),
