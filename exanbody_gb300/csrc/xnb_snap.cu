@@ -237,6 +237,9 @@ __global__ void __launch_bounds__(kSnapThreads)
   R* uacc = yv + 2 * nu;                                                    // 2 nu
   R* uall = uacc + 2 * nu;                                                  // group x 2 nu
   R* adj = uall + static_cast<size_t>(group) * 2 * nu;                      // group x (top level, the one below)
+  // the neighbours' FP64 work by another warp, and so on another quarter of the SM,
+  // in each block (8,192 Mo atoms 630 -> 624 us with the conversions off its pipe)
+  const int turn = (tid + kSnapThreads - 32 * static_cast<int>(blockIdx.x % kSnapWarps)) % kSnapThreads;
   const int adj_stride = 2 * (lvl_max + (J > 0 ? nunique(J - 1) : 1));
   double* red = reinterpret_cast<double*>(adj);                             // kSnapThreads x 5, once a round's adjoint is done
 
@@ -321,7 +324,7 @@ __global__ void __launch_bounds__(kSnapThreads)
     //      lanes in it. By one lane of each neighbour's own, in every warp and
     //      round, and again for the forces, it took a fifth of the time (8,192 Mo
     //      atoms 901 -> 722 us) ----
-    for (int q = tid; q < nn; q += kSnapThreads) {
+    for (int q = turn; q < nn; q += kSnapThreads) {
       const double rcut = (radi + t.radelem[nt[q]]) * t.rcutfac;
       const Geo geo = geometry(nx[q], ny[q], nz[q], rcut, t);
       nab[4 * q] = R(geo.a.r);
@@ -552,17 +555,17 @@ __global__ void __launch_bounds__(kSnapThreads)
         Nx = tmp;
       }
       if (active && slot == 0) F += R(0.5) * yv[0];  // level 0: U = 1, centre weight 1/2
-      red[tid * 5 + 0] = active ? static_cast<double>(F) : 0.0;
-      red[tid * 5 + 1] = static_cast<double>(gar);
-      red[tid * 5 + 2] = static_cast<double>(gai);
-      red[tid * 5 + 3] = static_cast<double>(gbr);
-      red[tid * 5 + 4] = static_cast<double>(gbi);
+      red[tid * 5 + 0] = active ? widen_f32(F) : 0.0;
+      red[tid * 5 + 1] = widen_f32(gar);
+      red[tid * 5 + 2] = widen_f32(gai);
+      red[tid * 5 + 3] = widen_f32(gbr);
+      red[tid * 5 + 4] = widen_f32(gbi);
       __syncthreads();
-      if (tid < gr) {
-        const int q = q0 + tid;
+      if (turn < gr) {
+        const int q = q0 + turn;
         double v[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
         for (int sl = 0; sl < lpn; ++sl)
-          for (int k = 0; k < 5; ++k) v[k] += red[(tid * lpn + sl) * 5 + k];
+          for (int k = 0; k < 5; ++k) v[k] += red[(turn * lpn + sl) * 5 + k];
         const double rcut = (radi + t.radelem[nt[q]]) * t.rcutfac;
         Geo geo;
         geometry_derivative(geo, nx[q], ny[q], nz[q], ngeo[4 * q], ngeo[4 * q + 1], t.rfac0 * M_PI / (rcut - t.rmin0));
