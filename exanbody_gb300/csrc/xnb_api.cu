@@ -540,9 +540,9 @@ int xnb_version(void) { return 10000; }
 
 int64_t xnb_system_bytes(int64_t n, int64_t ncells, double list_per_particle) {
   // doubles r v f pe, restored backup, rebin scratch (22); ids (2); u32 cell, backup,
-  // rebin and list bookkeeping (10); FP32 hi/lo mirrors; types (2); sub-cell key;
+  // rebin and list bookkeeping (10); FP32 mirrors (3) and position steps; types (2); sub-cell key;
   // per cell: u32 tables (6), scan, the two build lists and the sub-grid side
-  const int64_t per_part = 22 * 8 + 2 * 8 + 10 * 4 + 3 * 16 + 2 + 2;
+  const int64_t per_part = 22 * 8 + 2 * 8 + 10 * 4 + 4 * 16 + 2 + 2;
   const int64_t per_cell = 4 * 6 + 8 + 4 + 4 + 1;
   return n * per_part + ncells * per_cell + static_cast<int64_t>(static_cast<double>(n) * list_per_particle) * 4;
 }
