@@ -198,8 +198,11 @@ void go(const Extent& ex, const SysDesc* sys, const SysState* st, const DevArray
         cudaStream_t stream) {
   constexpr uint32_t sums = PE ? 5 : 4, group = 32u / sums;
   const BatchSource src(sys, st, a, sys_only);
-  // list entries per chunk: a multiple of 32 that the usual lists fit
-  const uint32_t chunk = std::min(std::max((ex.list_slot * 2u / 3u + 31u) / 32u * 32u, 32u), 256u);
+  // list entries per chunk: a multiple of 32 that the usual lists fit, up to the 96
+  // that leave shared memory for the eight blocks per SM which the registers allow
+  // (23,328 atoms, lists of up to 84, 98, 157 and 335 entries: 40 / 35, 43 / 38, 82 /
+  // 60 and 201 / 118 us with chunks of up to 256 / 96; 64 costs lists of 87 a tenth)
+  const uint32_t chunk = std::min(std::max((ex.list_slot * 2u / 3u + 31u) / 32u * 32u, 32u), 96u);
   const size_t smem = group * (sizeof(Row) + static_cast<size_t>(chunk + 1u) * sums * sizeof(double));
   const unsigned grid = (ex.n_part + group - 1u) / group;
   // stage 1: a warp per particle while every block has an SM of its own, then

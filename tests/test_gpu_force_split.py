@@ -16,7 +16,7 @@ pytestmark = pytest.mark.gpu
     (6, 857, 2.5, 2.0),     # odd count, forces divided by the mass
     (6, 1, 2.5, 1.0),       # one atom, no pair
     (6, 2, 2.5, 1.0),       # two atoms, at most one pair
-    (11, None, 4.2, 1.0),   # ~325 list entries: two chunks of 256
+    (11, None, 4.2, 1.0),   # ~325 list entries: four chunks of 96
 ])
 def test_split_equals_the_sequential_walk(n, keep, rcut, mass):
     w = workloads.lj_fcc_system(n, 0.8442, 1.2, 40 + n, rcut=rcut)
