@@ -52,8 +52,9 @@ int launch_force(const Extent& ex, const SysDesc* sys, SysState* st, const DevAr
 // the GPU that way. Per call, two-stage / one-thread: 864 atoms 10 / 87 us, 32,000
 // 43 / 96 us, 62,500 72 / 105 us, 131,072 135 / 137 us (178 / 165 us with
 // energies). The line lies where three batches stepping at once on their own
-// streams break even: 50 steps of 32,000 atoms 2.84 / 3.50 ms, 5 steps of 63,000
-// 0.594 / 0.586 ms, of eight systems of 2,048 to 16,384 atoms in a batch 0.595 / 0.552 ms.
+// streams lose at no density: 10 steps of 55,296 atoms at 0.75, 0.84 and 1.0
+// 731 / 705, 757 / 780 and 808 / 858 us, of 62,500 atoms 832 / 770, 876 / 835 and
+// 933 / 950 us (one batch alone 920 / 1268 and 998 / 1289 us at 0.84).
 constexpr uint32_t kMixedSplitMax = 50000;
 int launch_force_mixed(const Extent& ex, const SysDesc* sys, const SysState* st, const DevArrays& a, bool with_pe,
                        bool second_half, int sys_only, cudaStream_t stream);
