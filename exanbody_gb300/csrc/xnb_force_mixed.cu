@@ -221,9 +221,9 @@ void go(const Extent& ex, const SysDesc* sys, const SysState* st, const DevArray
 // marking walk gathers the entries near the cutoff a second time: 73 rounds, the
 // pipe at 58% and the L1 data stage at 66%). 64 registers hold 16 blocks of 64
 // threads per SM. Marking walk with the sums of PairSum / this one: 25 steps of 4M
-// atoms 74.9 / 69.4 ms (three such batches at once 75.0 / 73.7); 1M atoms with
-// energies 728 / 683 us; a batch of 96 small systems, 20 steps, three at once 45.2 /
-// 42.6 ms. With 56 registers 71.7 ms and 773 us, four entries at a time 80.8 ms.
+// atoms 74.9 / 69.4 ms (three such batches at once 75.0 / 67.0); 1M atoms with
+// energies 728 / 690 us; a batch of 96 small systems, 20 steps, three at once 45.2 /
+// 35.4 ms. With 56 registers 71.7 ms and 773 us, four entries at a time 80.8 ms.
 struct WalkParticle {
   const double* rx;
   const double* ry;
@@ -363,6 +363,12 @@ template <bool PE, bool KICK>
 void go_walk(const Extent& ex, const SysDesc* sys, const SysState* st, const DevArrays& a, int sys_only,
              cudaStream_t stream) {
   const unsigned threads = ex.force_block > 0 ? static_cast<unsigned>(ex.force_block) : 64u;
+  // All of an SM's memory as L1: a block of it beside another batch's neighbour build,
+  // whose stages leave little L1, gathers from L2 and holds that SM's launch up.
+  // Three batches stepping at once: 25 steps of 4M atoms 69.6 to 77 -> 67.0 ms, 20
+  // steps of 96 small systems 42.2 -> 35.4 ms; one alone 69.7 / 70.0 and 38.3 / 38.6.
+  cudaFuncSetAttribute(k_force_walk<PE, KICK>, cudaFuncAttributePreferredSharedMemoryCarveout,
+                       cudaSharedmemCarveoutMaxL1);
   k_force_walk<PE, KICK><<<(ex.n_part + threads - 1u) / threads, threads, 0, stream>>>(
       ex.n_part, BatchSource(sys, st, a, sys_only), a);
 }
