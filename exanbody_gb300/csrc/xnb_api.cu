@@ -151,7 +151,8 @@ struct xnb_graph {
   // what the captured launches depend on besides device memory: the batch's
   // work extent and launch configuration at capture
   uint32_t n_part = 0, n_cells = 0;
-  int nsys = 0, lbuf = 0, stage_cap = 0, force_block = 0, force_lanes = 0, build_form = 0, far_coords = 0, general = 0;
+  int nsys = 0, lbuf = 0, stage_cap = 0, force_block = 0, force_lanes = 0, build_form = 0, far_coords = 0, general = 0,
+      unpacked = 0;
   int force_form = 0, subcell_prune = 0;
   uint32_t n_seg = 0;
 };
@@ -1246,6 +1247,7 @@ int xnb_step_graph_create(xnb_batch* b, int32_t nsteps, int32_t precision, int32
   G->nsys = ex.nsys;
   G->far_coords = ex.far_coords;
   G->general = ex.general;
+  G->unpacked = ex.unpacked;
   G->force_form = ex.force_form;
   G->n_seg = ex.n_seg;
   G->lbuf = list_buf(b);
@@ -1269,7 +1271,7 @@ int xnb_graph_is_current(const xnb_graph* g) {
   const xnb_batch* b = g->batch;
   const Extent ex = b->extent();
   return (ex.n_part == g->n_part && ex.n_cells == g->n_cells && ex.nsys == g->nsys && ex.far_coords == g->far_coords &&
-          ex.general == g->general &&
+          ex.general == g->general && ex.unpacked == g->unpacked &&
           ex.force_form == g->force_form && ex.n_seg == g->n_seg &&
           list_buf(b) == g->lbuf &&
           b->stage_cap == g->stage_cap && b->force_block == g->force_block && b->force_lanes == g->force_lanes &&
