@@ -730,7 +730,8 @@ __global__ void __launch_bounds__(128, 8)
 // particle appends its hits in order straight to the particle's list slot (an
 // entry past the slot lands on its last word; the count flags the overflow).
 // The candidates come as runs of x-adjacent cells, contiguous in memory, so no
-// lane searches for its cell; a ballot compacts them in order. Two rare cases
+// lane searches for its cell (few candidates: as a list of their entries); a
+// ballot compacts them in order. Two rare cases
 // leave the fast test through warp-uniform branches: a chunk holding a candidate
 // whose ghost filter is undecided in FP32, and an FP32 distance inside the error
 // band around nbh^2 (both then take the reference's FP64 decision). A cell whose
@@ -744,6 +745,13 @@ __global__ void __launch_bounds__(128, 8)
 // (1.18 against 1.03 ms per build of 1,972,156 atoms), four at 6 blocks 1.07 ms.
 // The last particles of a cell are tested two at a time, not padded to four.
 constexpr int kWarpP = 4;  // particles tested per staged candidate load in the warp-per-cell build
+
+// Cells of at most this many candidates list them one by one and test whole steps of
+// 32; more come as runs, whose last step of each is partly empty. A build of
+// 1,972,156 atoms, runs alone / this: 2.88 / 1.78 ms at density 0.05, 2.01 / 1.12 at
+// 0.2, 0.95 / 0.87 at 0.35 (8 particles per cell, 220 candidates), 0.99 / 1.02 at
+// 0.5, 1.11 / 1.11 at 0.84; listing up to 128 takes 1.48 ms at 0.2.
+constexpr uint32_t kPackedMax = 256;
 
 // FP32 values as integers in the same order (no NaN).
 __device__ __forceinline__ int ordered_int(float f) {
@@ -920,13 +928,6 @@ __device__ __forceinline__ void neighbors_warp(uint32_t n_cells, const SysDesc* 
       g_n = a.cell_n[src];
       g_code = static_cast<uint32_t>(img[0] + 3 * img[1] + 9 * img[2]);
     }
-    // the three cells of a row are one contiguous run unless x wraps around:
-    // the first lane of the row then takes them all
-    {
-      const uint32_t n1 = __shfl_down_sync(0xffffffffu, g_n, 1), n2 = __shfl_down_sync(0xffffffffu, g_n, 2);
-      if (ci > 0 && ci < S.dims[0] - 1) g_n = lane % 3u == 0u ? g_n + n1 + n2 : 0u;
-    }
-
     // the particles' bounding box
     float4 own = make_float4(0.f, 0.f, 0.f, 0.f);
     float bl[3] = {3.0e38f, 3.0e38f, 3.0e38f}, bh[3] = {-3.0e38f, -3.0e38f, -3.0e38f};
@@ -946,11 +947,63 @@ __device__ __forceinline__ void neighbors_warp(uint32_t n_cells, const SysDesc* 
       bh[ax] = from_ordered(__reduce_max_sync(0xffffffffu, ordered_int(bh[ax])));
     }
 
-    // stage: 32 candidates of a run per step, the steps listed first so that
-    // the loads of four are in flight together
     uint32_t m = 0, off_self = 0;
     bool undecided = false;  // a candidate whose ghost filter FP32 does not decide
-    {
+    // this lane's candidate j through its image, kept if it lies within reach of the
+    // box; candidate `self` of these 32 (if one is) is the cell's own first particle
+    // (kept, as all its own are: distance 0)
+    auto stage = [&](float4 pb, uint32_t j, uint32_t code, bool valid, uint32_t self) {
+      float4 rb = pb;
+      if (code == static_cast<uint32_t>(kImageCenter)) {
+        rb.w = __uint_as_float(((j - S.part_base) << 5) | static_cast<uint32_t>(kImageCenter));
+      } else {
+        rb = stage_from(S, pb, j, code);
+        undecided |= valid && __float_as_uint(rb.w) - kAmbiguousBit < kInvalid - kAmbiguousBit;
+      }
+      const float ex = fmaxf(fmaxf(bl[0] - rb.x, rb.x - bh[0]), 0.f);
+      const float ey = fmaxf(fmaxf(bl[1] - rb.y, rb.y - bh[1]), 0.f);
+      const float ez = fmaxf(fmaxf(bl[2] - rb.z, rb.z - bh[2]), 0.f);
+      const bool keep = valid && fmaf(ex, ex, fmaf(ey, ey, ez * ez)) <= w.nb_hi;
+      const unsigned km = __ballot_sync(0xffffffffu, keep);
+      if (self < 32u) off_self = m + __popc(km & ((1u << self) - 1u));
+      const uint32_t pos = m + __popc(km & w.lt);
+      if (keep && pos < static_cast<uint32_t>(cap)) srel[pos] = rb;
+      m += __popc(km);
+    };
+    uint32_t g_off = g_n;  // inclusive scan
+    for (int off = 1; off < 32; off <<= 1) {
+      const uint32_t v = __shfl_up_sync(0xffffffffu, g_off, off);
+      if (lane >= static_cast<uint32_t>(off)) g_off += v;
+    }
+    const uint32_t ncand = __shfl_sync(0xffffffffu, g_off, 31);
+    g_off -= g_n;
+    if (ncand <= kPackedMax && ncand + kPackedMax / 4u <= static_cast<uint32_t>(cap)) {
+      // few: entries listed one after the other (behind the stage), 32 per step
+      uint32_t* const map = reinterpret_cast<uint32_t*>(srel + cap) - kPackedMax;
+      for (uint32_t q = 0; q < g_n; ++q) map[g_off + q] = ((g_start + q - S.part_base) << 5) | g_code;
+      __syncwarp();
+      const uint32_t first = __shfl_sync(0xffffffffu, g_off, 13);
+      for (uint32_t t0 = 0; t0 < ncand; t0 += 128u) {
+        uint32_t ent[4];
+        float4 pb[4];
+#pragma unroll
+        for (uint32_t q = 0; q < 4u; ++q) {
+          const uint32_t u = t0 + 32u * q + lane;
+          ent[q] = u < ncand ? map[u] : static_cast<uint32_t>(kImageCenter);
+          pb[q] = u < ncand ? a.pf[S.part_base + (ent[q] >> 5)] : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+#pragma unroll
+        for (uint32_t q = 0; q < 4u; ++q) {
+          const uint32_t u0 = t0 + 32u * q;
+          if (u0 < ncand) stage(pb[q], S.part_base + (ent[q] >> 5), ent[q] & 31u, u0 + lane < ncand, first - u0);
+        }
+      }
+    } else {
+      // 32 candidates of a run per step, the steps listed first so that the loads
+      // of four are in flight together. The three cells of a row are one contiguous
+      // run unless x wraps around: the first lane of the row then takes them all
+      const uint32_t n1 = __shfl_down_sync(0xffffffffu, g_n, 1), n2 = __shfl_down_sync(0xffffffffu, g_n, 2);
+      if (ci > 0 && ci < S.dims[0] - 1) g_n = lane % 3u == 0u ? g_n + n1 + n2 : 0u;
       const uint32_t steps = lane < 27u ? (g_n + 31u) >> 5 : 0u;
       uint32_t at = steps;  // inclusive scan
       for (int off = 1; off < 32; off <<= 1) {
@@ -976,25 +1029,9 @@ __device__ __forceinline__ void neighbors_warp(uint32_t n_cells, const SysDesc* 
           }
 #pragma unroll
           for (uint32_t q = 0; q < 4u; ++q) {
-            float4 rb = pb[q];
-            if (run[q].z == static_cast<uint32_t>(kImageCenter)) {
-              rb.w = __uint_as_float(((run[q].x + lane - S.part_base) << 5) | static_cast<uint32_t>(kImageCenter));
-            } else {
-              rb = stage_from(S, pb[q], run[q].x + lane, run[q].z);
-              undecided |= __float_as_uint(rb.w) - kAmbiguousBit < kInvalid - kAmbiguousBit;
-            }
-            const float ex = fmaxf(fmaxf(bl[0] - rb.x, rb.x - bh[0]), 0.f);
-            const float ey = fmaxf(fmaxf(bl[1] - rb.y, rb.y - bh[1]), 0.f);
-            const float ez = fmaxf(fmaxf(bl[2] - rb.z, rb.z - bh[2]), 0.f);
-            const bool keep = lane < run[q].y && fmaf(ex, ex, fmaf(ey, ey, ez * ez)) <= w.nb_hi;
-            const unsigned km = __ballot_sync(0xffffffffu, keep);
-            // the cell's own particles are all kept (distance 0)
             const uint32_t self = sa - run[q].x;
-            if (run[q].z == static_cast<uint32_t>(kImageCenter) && self < 32u && self < run[q].y)
-              off_self = m + __popc(km & ((1u << self) - 1u));
-            const uint32_t pos = m + __popc(km & w.lt);
-            if (keep && pos < static_cast<uint32_t>(cap)) srel[pos] = rb;
-            m += __popc(km);
+            stage(pb[q], run[q].x + lane, run[q].z, lane < run[q].y,
+                  run[q].z == static_cast<uint32_t>(kImageCenter) && self < run[q].y ? self : 32u);
           }
         }
       }
