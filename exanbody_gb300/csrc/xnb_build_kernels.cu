@@ -318,8 +318,8 @@ __device__ __forceinline__ void store_backup(const SysDesc& S, const DevArrays& 
 // amr_grid_algorithm.h:131-374, when the cell is dense enough for a sub-grid),
 // cell table update, and backup_r (io/backup_r.cpp:56-79): kBackupExact keeps
 // the encoding (store_backup), kBackupPlain the position itself, both while the
-// position is in registers.
-constexpr int kBackupExact = 1, kBackupPlain = 2;
+// position is in registers; kBackupNone leaves it to backup_particles.
+constexpr int kBackupNone = 0, kBackupExact = 1, kBackupPlain = 2;
 template <int BACKUP>
 __device__ __forceinline__ void rebin_finalize(uint32_t n_cells, const SysDesc* __restrict__ sys, SysState* st,
                                                const DevArrays& a) {
@@ -386,7 +386,7 @@ __device__ __forceinline__ void rebin_finalize(uint32_t n_cells, const SysDesc* 
       a.pstep[dst] = make_steps(x, y, z, mhi);
       if constexpr (BACKUP == kBackupExact) {
         store_backup(S, a, dst, lo, x, y, z);
-      } else {
+      } else if constexpr (BACKUP == kBackupPlain) {
         a.rbx[dst] = x;
         a.rby[dst] = y;
         a.rbz[dst] = z;
@@ -409,10 +409,9 @@ __global__ void __launch_bounds__(128)
   rebin_finalize<BACKUP>(n_cells, sys, st, a);
 }
 
-// backup_r alone (io/backup_r.cpp:42-79) for flagged systems.
-__global__ void __launch_bounds__(256)
-    k_backup(uint32_t n_part, const SysDesc* __restrict__ sys, SysState* st, DevArrays a) {
-  if (*a.any_rebuild == 0) return;
+// backup_r (io/backup_r.cpp:42-79) for flagged systems, a thread per particle.
+__device__ __forceinline__ void backup_particles(uint32_t n_part, const SysDesc* __restrict__ sys, const SysState* st,
+                                                 const DevArrays& a) {
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n_part; i += gridDim.x * blockDim.x) {
     const uint32_t c = a.pcell[i];
     if (c == kInvalid) continue;
@@ -424,6 +423,11 @@ __global__ void __launch_bounds__(256)
     const double lo[3] = {cell_lo(S, 0, ci), cell_lo(S, 1, cj), cell_lo(S, 2, ck)};
     store_backup(S, a, i, lo, a.rx[i], a.ry[i], a.rz[i]);
   }
+}
+__global__ void __launch_bounds__(256)
+    k_backup(uint32_t n_part, const SysDesc* __restrict__ sys, SysState* st, DevArrays a) {
+  if (*a.any_rebuild == 0) return;
+  backup_particles(n_part, sys, st, a);
 }
 
 // backup_r done for the flagged systems; after a rebin their sub-cell keys
@@ -1095,7 +1099,7 @@ __global__ void __launch_bounds__(128, 5)
 // BUILD: the lists of the flagged systems too (the warp-per-cell form without
 // sub-cell pruning, then the cells it passes on), two more barriers: a step
 // without a rebuild is then three launches, push, this one and the forces.
-template <int BACKUP, bool BUILD>
+template <bool EXACT, bool BUILD>
 __global__ void __launch_bounds__(256)
     k_rebin_fused(uint32_t n_part, uint32_t n_cells, int nsys, const SysDesc* __restrict__ sys, SysState* st,
                   DevArrays a, int cap, int lbuf, uint32_t split) {
@@ -1160,9 +1164,10 @@ __global__ void __launch_bounds__(256)
     ok = grid_barrier(a.grid_ctl, gridDim.x);
   }
   if (ok) {
-    rebin_finalize<BACKUP>(n_cells, sys, st, a);
-    if (BUILD) ok = grid_barrier(a.grid_ctl, gridDim.x);
+    rebin_finalize<EXACT ? kBackupNone : kBackupPlain>(n_cells, sys, st, a);
+    if (EXACT || BUILD) ok = grid_barrier(a.grid_ctl, gridDim.x);
   }
+  if (EXACT && ok) backup_particles(n_part, sys, st, a);
   if (BUILD && ok) {
     neighbors_warp<8>(n_cells, sys, st, a, cap, false, false, split, fused_smem);
     ok = grid_barrier(a.grid_ctl, gridDim.x);
@@ -1316,6 +1321,16 @@ int launch_scan_u32_to_u64(const uint32_t* in, unsigned long long* out, uint32_t
   return 3;
 }
 
+// The encoding inside the rebin's last pass costs a warp's FP64 instructions per cell,
+// however few its particles: a pass of its own, a thread per particle, unless the
+// cells fill the warps and the batch is too small to hide one more launch. Rebin and
+// build, inside / alone: 8,788 atoms 111 / 112 us at density 0.35 (8 per cell), 111 /
+// 123 at 0.84; 32,000 atoms 221 / 160 us at 0.1, 134 / 136 at 0.84; 97,556 atoms 197
+// / 195 us at 0.84; 953,312 atoms 11.9 / 8.1 ms at 0.02, 1.06 / 1.00 ms at 0.84. (In
+// the fused rebin the pass is never slower: 50 steps of 8,788 atoms 73.0 / 73.0 us
+// each at 0.84, 69 / 63 at 0.02.)
+constexpr uint32_t kFoldBackupMax = 50000, kFoldBackupPerCell = 8;
+
 int launch_rebin(const Extent& ex, const SysDesc* sys, SysState* st, const DevArrays& a, cudaStream_t stream,
                  bool exact_backup) {
   if (ex.n_part == 0 || ex.n_cells == 0) return 0;
@@ -1325,10 +1340,18 @@ int launch_rebin(const Extent& ex, const SysDesc* sys, SysState* st, const DevAr
   k_rebin_count<<<wg, 128, 0, stream>>>(ex.n_cells, sys, st, a);
   const int ns = launch_scan_u32_to_u64(a.cell_cnt, a.cell_scan, ex.n_cells, a.scan_blocks, stream, a.any_rebuild);
   k_rebin_scatter<<<wg, 128, 0, stream>>>(ex.n_cells, sys, st, a);
-  if (exact_backup) k_rebin_finalize<kBackupExact><<<wg, 128, 0, stream>>>(ex.n_cells, sys, st, a);
-  else k_rebin_finalize<kBackupPlain><<<wg, 128, 0, stream>>>(ex.n_cells, sys, st, a);
+  int nb = 0;
+  if (!exact_backup) {
+    k_rebin_finalize<kBackupPlain><<<wg, 128, 0, stream>>>(ex.n_cells, sys, st, a);
+  } else if (ex.n_part <= kFoldBackupMax && ex.n_part >= kFoldBackupPerCell * ex.n_cells) {
+    k_rebin_finalize<kBackupExact><<<wg, 128, 0, stream>>>(ex.n_cells, sys, st, a);
+  } else {
+    k_rebin_finalize<kBackupNone><<<wg, 128, 0, stream>>>(ex.n_cells, sys, st, a);
+    k_backup<<<thread_grid(ex.n_part, 256, ex.sm_count), 256, 0, stream>>>(ex.n_part, sys, st, a);
+    nb = 1;
+  }
   k_arm<<<(ex.nsys + 127) / 128, 128, 0, stream>>>(ex.nsys, st, a.any_rebuild, true);
-  return 6 + ns;
+  return 6 + nb + ns;
 }
 
 bool fused_rebin_fits(const Extent& ex) {
@@ -1352,8 +1375,8 @@ int launch_rebin_fused(const Extent& ex, const SysDesc* sys, SysState* st, const
     smem = std::max(static_cast<size_t>(warps) * cap * sizeof(float4),
                     static_cast<size_t>(cap) * sizeof(float4) + static_cast<size_t>(warps) * 2 * lbuf * sizeof(uint32_t));
   }
-  auto kern = exact_backup ? (build ? k_rebin_fused<kBackupExact, true> : k_rebin_fused<kBackupExact, false>)
-                           : (build ? k_rebin_fused<kBackupPlain, true> : k_rebin_fused<kBackupPlain, false>);
+  auto kern = exact_backup ? (build ? k_rebin_fused<true, true> : k_rebin_fused<true, false>)
+                           : (build ? k_rebin_fused<false, true> : k_rebin_fused<false, false>);
   cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
