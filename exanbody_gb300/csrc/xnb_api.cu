@@ -435,7 +435,6 @@ int upload_segments(xnb_batch* b, cudaStream_t st) {
 // Per-warp list buffer of the neighbour build: the largest slot of the resident
 // systems, rounded up to 32 entries, at most kMaxListBuf (larger slots are
 // written without buffering).
-constexpr uint32_t kMaxListBuf = 1024;
 int list_buf(const xnb_batch* b) {
   uint32_t m = 0;
   for (const SysHost& h : b->sys)
@@ -559,7 +558,7 @@ int xnb_batch_create(const xnb_batch_config* cfg, xnb_batch** out) {
   b->device = cfg->device;
   b->cfg = *cfg;
   if (cfg->stage_cap > 0) b->stage_cap = (cfg->stage_cap + 31) / 32 * 32;
-  if (cfg->stage_cap > 1024) {
+  if (cfg->stage_cap > kStageCapMax) {
     delete b;
     return fail(XNB_ERR_ARG, "stage_cap above 1024 candidates");
   }
@@ -1134,8 +1133,8 @@ int xnb_step(xnb_batch* b, int32_t nsteps, int32_t precision, int32_t flags, voi
   if (!b) return fail(XNB_ERR_ARG, "null batch");
   int base = 0;
   bool newton = false;
-  int rc0 = decode_precision(precision, &base, &newton);
-  if (rc0) return rc0;
+  int rc = decode_precision(precision, &base, &newton);
+  if (rc) return rc;
   precision = base;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const Extent ex = b->extent();
@@ -1143,20 +1142,29 @@ int xnb_step(xnb_batch* b, int32_t nsteps, int32_t precision, int32_t flags, voi
   const bool energy = (flags & XNB_STEP_ENERGY) != 0;
   const bool fused = !(flags & XNB_STEP_HOST_SYNC) && fused_rebin_fits(ex);
   const bool build = fused && fused_build_fits(ex, b->build_form, b->subcell_prune != 0);
-  for (int k = 0; k < nsteps; ++k) {
+  // a launch that was refused ends the steps (the runtime forgets it at its next good call)
+  cudaGetLastError();
+  for (int k = 0; k < nsteps && rc == 0; ++k) {
     // verlet_first_half + trigger_move_particles
     b->launches += launch_first_half(ex, b->d_sys, b->d_st, b->a, true, true, true, 1.0, 0.5, exact, -1, st);
+    rc = check_launch();
+    if (rc) return rc;
     if (fused) {
       b->launches += launch_rebin_fused(ex, b->d_sys, b->d_st, b->a, exact, build, b->stage_cap, list_buf(b), st);
-      if (!build)
+      rc = check_launch();
+      if (!rc && !build) {
         b->launches += launch_neighbors(ex, b->d_sys, b->d_st, b->a, b->stage_cap, list_buf(b), st, b->build_form,
                                         b->subcell_prune != 0, false);
+        rc = check_launch();
+      }
+      if (rc) return rc;
       b->launches += launch_force(ex, b->d_sys, b->d_st, b->a, precision, energy, true, -1, st, newton);
+      rc = check_launch();
       continue;
     }
     bool rebuild = true;
     if (flags & XNB_STEP_HOST_SYNC) {
-      int rc = pull_states(b, st);
+      rc = pull_states(b, st);
       if (rc) return rc;
       rebuild = false;
       for (int q = 0; q < ex.nsys; ++q)
@@ -1166,19 +1174,24 @@ int xnb_step(xnb_batch* b, int32_t nsteps, int32_t precision, int32_t flags, voi
       // update_particles_full
       b->launches += launch_mark_rebuild(ex, b->d_st, 1, -1, b->a.any_rebuild, st);
       b->launches += launch_rebin(ex, b->d_sys, b->d_st, b->a, st, exact);
+      rc = check_launch();
+      if (rc) return rc;
       if (flags & XNB_STEP_HOST_SYNC) {
-        int rc = neighbors_sync(b, st);
+        rc = neighbors_sync(b, st);
         if (rc) return rc;
       } else {
         b->launches += launch_neighbors(ex, b->d_sys, b->d_st, b->a, b->stage_cap, list_buf(b), st, b->build_form,
                                         b->subcell_prune != 0);
       }
       b->launches += launch_clear_moved(ex, b->d_st, st);
+      rc = check_launch();
+      if (rc) return rc;
     }
     // compute_all_forces_energy + verlet_second_half
     b->launches += launch_force(ex, b->d_sys, b->d_st, b->a, precision, energy, true, -1, st, newton);
+    rc = check_launch();
   }
-  return check_launch();
+  return rc;
 }
 
 int xnb_step_persistent(xnb_batch* b, int32_t nsteps, int32_t precision, int32_t flags, void* stream) {
@@ -1314,7 +1327,7 @@ int xnb_check_errors(xnb_batch* b, void* stream) {
 
 int xnb_batch_set_tuning(xnb_batch* b, int32_t stage_cap, int32_t force_block) {
   if (!b) return fail(XNB_ERR_ARG, "null batch");
-  if (stage_cap <= 0 || stage_cap > 1024) return fail(XNB_ERR_ARG, "stage_cap must be in 1..1024");
+  if (stage_cap <= 0 || stage_cap > kStageCapMax) return fail(XNB_ERR_ARG, "stage_cap must be in 1..1024");
   if (force_block <= 0 || force_block % 32 || force_block > 256)
     return fail(XNB_ERR_ARG, "force_block must be a multiple of 32 and at most 256");
   b->stage_cap = (stage_cap + 31) / 32 * 32;

@@ -1377,7 +1377,7 @@ int launch_rebin_fused(const Extent& ex, const SysDesc* sys, SysState* st, const
   }
   auto kern = exact_backup ? (build ? k_rebin_fused<true, true> : k_rebin_fused<true, false>)
                            : (build ? k_rebin_fused<false, true> : k_rebin_fused<false, false>);
-  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+  if (build) raise_smem_limit(kern, warps * kStageCapMax * sizeof(float4));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(warps * 32u);
@@ -1405,9 +1405,8 @@ int launch_neighbors(const Extent& ex, const SysDesc* sys, SysState* st, const D
   const size_t smem = static_cast<size_t>(cap) * sizeof(float4) + static_cast<size_t>(4) * 2 * lbuf * sizeof(uint32_t);
   // warp-per-cell form: the stage alone (hits go straight to the slots)
   const size_t smem_w = 4 * static_cast<size_t>(cap) * sizeof(float4);
-  // per-device attributes: set them on the current device every time (host calls, no GPU work)
-  cudaFuncSetAttribute(k_neighbors, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
-  cudaFuncSetAttribute(k_neighbors_warp, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
+  raise_smem_limit(k_neighbors, kStageCapMax * sizeof(float4) + 4u * 2u * kMaxListBuf * sizeof(uint32_t));
+  raise_smem_limit(k_neighbors_warp, 4u * kStageCapMax * sizeof(float4));
   int per_sm = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_neighbors_warp, 128, smem_w) != cudaSuccess || per_sm < 1)
     per_sm = 1;

@@ -446,7 +446,7 @@ int launch_neighbors_rows(const Extent& ex, const SysDesc* sys, SysState* st, co
                           bool prune) {
   if (ex.n_cells == 0) return 0;
   const size_t smem = 4 * sizeof(RowsWarp);
-  cudaFuncSetAttribute(k_neighbors_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+  raise_smem_limit(k_neighbors_rows, smem);
   int per_sm = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_neighbors_rows, 128, smem) != cudaSuccess || per_sm < 1)
     per_sm = 1;

@@ -297,7 +297,7 @@ int launch_neighbors_sub(const Extent& ex, const SysDesc* sys, SysState* st, con
                          cudaStream_t stream) {
   if (ex.n_cells == 0) return 0;
   const size_t smem = sub_stage_offset(4) + static_cast<size_t>(4) * cap * sizeof(float4);
-  cudaFuncSetAttribute(k_neighbors_sub, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+  raise_smem_limit(k_neighbors_sub, sub_stage_offset(4) + 4u * kStageCapMax * sizeof(float4));
   int per_sm = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_neighbors_sub, 128, smem) != cudaSuccess || per_sm < 1)
     per_sm = 1;

@@ -202,13 +202,15 @@ void go(const Extent& ex, const SysDesc* sys, const SysState* st, const DevArray
   // that leave shared memory for the eight blocks per SM which the registers allow
   // (23,328 atoms, lists of up to 84, 98, 157 and 335 entries: 40 / 35, 43 / 38, 82 /
   // 60 and 201 / 118 us with chunks of up to 256 / 96; 64 costs lists of 87 a tenth)
-  const uint32_t chunk = std::min(std::max((ex.list_slot * 2u / 3u + 31u) / 32u * 32u, 32u), 96u);
+  constexpr uint32_t longest = 96u;
+  const uint32_t chunk = std::min(std::max((ex.list_slot * 2u / 3u + 31u) / 32u * 32u, 32u), longest);
+  static_assert(group * (sizeof(Row) + (longest + 1u) * sums * sizeof(double)) <= 48u * 1024u,
+                "more shared memory than a launch may have without raising its kernel's limit");
   const size_t smem = group * (sizeof(Row) + static_cast<size_t>(chunk + 1u) * sums * sizeof(double));
   const unsigned grid = (ex.n_part + group - 1u) / group;
   // stage 1: a warp per particle while every block has an SM of its own, then
   // two particles per warp (32,000 atoms: 43 us with 128 threads, 61 us with 256)
   const unsigned threads = grid <= static_cast<unsigned>(ex.sm_count) ? group * 32u : group * 16u;
-  cudaFuncSetAttribute(k_force_mixed<PE, KICK>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
   k_force_mixed<PE, KICK><<<grid, threads, smem, stream>>>(ex.n_part, src, a, group, chunk);
 }
 

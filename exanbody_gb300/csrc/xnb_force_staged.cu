@@ -291,7 +291,7 @@ int launch_force_staged(const Extent& ex, const SysDesc* sys, SysState* st, cons
   const size_t smem = sizeof(StagedSmem);
   const int grid = static_cast<int>(std::min<long long>(ex.n_seg, static_cast<long long>(ex.sm_count) * 2));
 #define XNB_STAGED(PE_, K_)                                                                                   \
-  cudaFuncSetAttribute(k_force_staged<PE_, K_>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)); \
+  raise_smem_limit(k_force_staged<PE_, K_>, sizeof(StagedSmem));                                              \
   k_force_staged<PE_, K_><<<grid, kStagedThreads, smem, stream>>>(ex.n_seg, sys, st, a, sys_only);
   if (with_pe && second_half) {
     XNB_STAGED(true, true)

@@ -1427,7 +1427,7 @@ template <class Kernel>
 void snap_go(Kernel kern, const Extent& ex, const SysDesc* sys, const SysState* st, const DevArrays& a,
              const SnapArgs& t, int group, size_t smem, int sys_only, bool with_pe, unsigned int* flags,
              cudaStream_t stream) {
-  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+  raise_smem_limit(kern, kSmemPerBlock);
   int per_sm = 1;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kSnapThreads, smem);
   long long g = static_cast<long long>(ex.sm_count) * std::max(1, per_sm) * 4;
