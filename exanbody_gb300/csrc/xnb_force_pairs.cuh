@@ -9,19 +9,26 @@
 //     entries in flight, against rc^2 plus the proven FP32 error bound; ballots
 //     append the entries to the particle's row in shared memory, in list order.
 //     Entries inside the band around rc^2 carry a flag.
-//   Stage 2 (FP64), kFp64: the rows of the eight particles lie one after the
-//     other and every lane takes an equal run of pairs, 18 FP64 instructions each
-//     (24 with the exact d2, a reciprocal of two Newton steps and a compare per
-//     pair); flagged entries take the reference's d2 test first. Where a run
-//     passes from one particle to the next the sums so far are put down; each
-//     particle's few pieces are then added in order.
+//   Stage 2 (FP64), kFp64: four lanes per particle take every fourth of its pairs,
+//     18 FP64 instructions each (24 with the exact d2, a reciprocal of two Newton
+//     steps and a compare per pair); flagged entries take the reference's d2 test
+//     first. The order of a particle's sums follows from its own list alone, so a
+//     system's forces are the same bits whatever else the batch holds.
+//     Half lists (NEWTON), whose lengths differ more and whose reactions arrive in
+//     any order anyway: the rows of the eight particles lie one after the other
+//     and every lane takes an equal run of pairs. Where a run passes from one
+//     particle to the next the sums so far are put down; each particle's few
+//     pieces are then added in order.
 //   kFp64Exact: the functor's own operations and roundings, four lanes per
 //     particle; a 4 x 4 transpose hands each lane one component of four
 //     consecutive pairs, which it adds in list order: the bits of the sequential
 //     walk.
 // The FP64 pipe is busy 85% of the time (kFp64, 119,164 atoms: 422 us with one
-// thread per particle, 282 now). Newton half lists, 5 steps of 256,000 atoms: 3.94
-// -> 1.89 ms; kFp64Exact, 5 host-synchronised steps of 8,788 atoms: 767 -> 424 us.
+// thread per particle, 280 now; 282 with equal runs of the eight particles' pairs
+// for full lists too, whose rounds are not those of the longest of eight lists but
+// whose ends cost as much; at density 0.35, 953,312 atoms, 1,181, 875 and 822 us).
+// Newton half lists, 5 steps of 256,000 atoms: 3.94 -> 1.89 ms; kFp64Exact, 5
+// host-synchronised steps of 8,788 atoms: 767 -> 424 us.
 #pragma once
 
 #include "xnb_lj_pair.cuh"
@@ -32,15 +39,15 @@ namespace pairs {
 
 constexpr uint32_t kPer = 8;             // particles per warp
 constexpr uint32_t kChunk = 96;          // list entries filtered per round
-constexpr uint32_t kRow = kChunk + 1;    // kFp64Exact: odd, the rows start on different banks
+constexpr uint32_t kRow = kChunk + 1;    // full lists: odd, the rows start on different banks
 constexpr uint32_t kCheck = 0x80000000u; // entry inside the FP32 band (list entries stay below 2^31)
 
 // A warp's shared memory.
 struct WarpSmem {
   double pos[kPer][3];          // the particles
-  double piece[32 + kPer][4];   // kFp64: piece (lane, particle) at lane + particle, unique along the runs
+  double piece[32 + kPer][4];   // half lists: piece (lane, particle) at lane + particle, unique along the runs
   uint32_t row[kPer * kRow];
-  uint32_t start[kPer + 1];     // kFp64: first pair of each particle
+  uint32_t start[kPer + 1];     // half lists: first pair of each particle
   uint32_t sys[kPer];
 };
 
@@ -80,6 +87,7 @@ __device__ __forceinline__ void eight_particles(uint32_t first, uint32_t n_part,
   const SysDesc& S = src.sys[s];
   const uint32_t longest = __reduce_max_sync(full, n);
   double sum = 0.0;  // component `sub` of particle `mine`
+  double part[4] = {0.0, 0.0, 0.0, 0.0};  // kFp64, full lists: the components over this lane's pairs
 
   for (uint32_t kb = 0; kb < longest; kb += kChunk) {
     // ---- stage 1 ----
@@ -87,7 +95,7 @@ __device__ __forceinline__ void eight_particles(uint32_t first, uint32_t n_part,
     for (uint32_t p = 0; p < kPer; ++p) {
       const int from = static_cast<int>(4u * p);
       const uint32_t np = __shfl_sync(full, n, from);
-      if (P == kFp64 && lane == 0) sm.start[p] = total;
+      if (NEWTON && lane == 0) sm.start[p] = total;
       if (np <= kb) continue;
       const uint32_t* L = reinterpret_cast<const uint32_t*>(
           __shfl_sync(full, reinterpret_cast<unsigned long long>(list), from));
@@ -103,7 +111,7 @@ __device__ __forceinline__ void eight_particles(uint32_t first, uint32_t n_part,
 #pragma unroll
       for (uint32_t t = 0; t < 3u; ++t)
         hb[t] = e[t] != 0xFFFFFFFFu ? src.pf[base + (e[t] >> 5)] : make_float4(1.0e18f, 0.f, 0.f, 0.f);
-      uint32_t* const out = sm.row + (P == kFp64 ? total : p * kRow);
+      uint32_t* const out = sm.row + (NEWTON ? total : p * kRow);
       uint32_t c = 0;
 #pragma unroll
       for (uint32_t t = 0; t < 3u; ++t) {
@@ -124,10 +132,10 @@ __device__ __forceinline__ void eight_particles(uint32_t first, uint32_t n_part,
       if (mine == p) count = c;
       total += c;
     }
-    if (P == kFp64 && lane == 0) sm.start[kPer] = total;
+    if (NEWTON && lane == 0) sm.start[kPer] = total;
     __syncwarp();
     // ---- stage 2 ----
-    if constexpr (P == kFp64) {
+    if constexpr (NEWTON) {
       const uint32_t run = (total + 31u) >> 5;
       const uint32_t f0 = min(total, lane * run), f1 = min(total, f0 + run);
       uint32_t p = 0, end = 0, pbase = 0, e = 0;
@@ -207,13 +215,11 @@ __device__ __forceinline__ void eight_particles(uint32_t first, uint32_t n_part,
             en = 0.5 * fma(T->eps4 * s6, s6 - 1.0, -T->e_shift);
             pe += en;
           }
-          if (NEWTON) {
-            const uint32_t j = pbase + ((w & ~kCheck) >> 5);
-            atomicAdd(a.fx + j, -(pd * dx));
-            atomicAdd(a.fy + j, -(pd * dy));
-            atomicAdd(a.fz + j, -(pd * dz));
-            if (PE) atomicAdd(a.pe + j, en);
-          }
+          const uint32_t j = pbase + ((w & ~kCheck) >> 5);
+          atomicAdd(a.fx + j, -(pd * dx));
+          atomicAdd(a.fy + j, -(pd * dy));
+          atomicAdd(a.fz + j, -(pd * dz));
+          if (PE) atomicAdd(a.pe + j, en);
         }
       }
       if (f0 < f1) put();
@@ -222,6 +228,48 @@ __device__ __forceinline__ void eight_particles(uint32_t first, uint32_t n_part,
       const uint32_t p0 = sm.start[mine], p1 = sm.start[mine + 1];
       if (p0 < p1 && (PE || sub < 3u))
         for (uint32_t l = p0 / run; l <= (p1 - 1u) / run; ++l) sum += sm.piece[l + mine][sub];
+    } else if constexpr (P == kFp64) {
+      // four lanes per particle, each every fourth of its pairs
+      const uint32_t* const row = sm.row + mine * kRow;
+      const uint32_t pbase = S.part_base;
+      const double xa = sm.pos[mine][0], ya = sm.pos[mine][1], za = sm.pos[mine][2];
+      const double sig2 = S.sig2, pd_a = S.pd_a, pd_b = S.pd_b;
+      uint32_t e = 0;
+      double xb = 0.0, yb = 0.0, zb = 0.0;
+      auto fetch = [&](uint32_t k) {
+        if (k < count) {
+          e = row[k];
+          const uint32_t j = pbase + ((e & ~kCheck) >> 5);
+          xb = src.rx[j];
+          yb = src.ry[j];
+          zb = src.rz[j];
+        }
+      };
+      fetch(sub);
+      for (uint32_t k = sub; k < count; k += 4u) {
+        const uint32_t w = e, code = w & 31u;
+        double x = xb, y = yb, z = zb;
+        fetch(k + 4u);  // the next pair's coordinates while this one is evaluated
+        if (code != static_cast<uint32_t>(kImageCenter)) {
+          const uint32_t cx = code % 3u, cy = (code / 3u) % 3u, cz = code / 9u;
+          if (cx != 1u) x = __dadd_rn(x, cx == 2u ? S.period[0] : -S.period[0]);
+          if (cy != 1u) y = __dadd_rn(y, cy == 2u ? S.period[1] : -S.period[1]);
+          if (cz != 1u) z = __dadd_rn(z, cz == 2u ? S.period[2] : -S.period[2]);
+        }
+        const double dx = __dsub_rn(x, xa), dy = __dsub_rn(y, ya), dz = __dsub_rn(z, za);
+        if (w & kCheck) {
+          const double d2 = norm2_rn(dx, dy, dz);
+          if (!(d2 > 0.0 && d2 <= S.rcut2)) continue;
+        }
+        const double s2 = sig2 * reciprocal(fma(dx, dx, fma(dy, dy, dz * dz)));
+        const double s6 = s2 * s2 * s2;
+        // 24 eps / sigma^2 (1 - 2 s6) s6 s2
+        const double pd = fma(pd_b, s6, pd_a) * s6 * s2;
+        part[0] = fma(pd, dx, part[0]);
+        part[1] = fma(pd, dy, part[1]);
+        part[2] = fma(pd, dz, part[2]);
+        if (PE) part[3] += 0.5 * fma(S.eps4 * s6, s6 - 1.0, -S.e_shift);
+      }
     } else {
       const uint32_t* const row = sm.row + mine * kRow;
       const uint32_t rounds = (__reduce_max_sync(full, count) + 3u) >> 2, pbase = S.part_base;
@@ -292,6 +340,13 @@ __device__ __forceinline__ void eight_particles(uint32_t first, uint32_t n_part,
     __syncwarp();  // the rows are refilled for the next round
   }
 
+  if (P == kFp64 && !NEWTON) {
+    // component c of the four lanes meets in lane c: (0 + 1) + (2 + 3)
+    const bool odd = (sub & 1u) != 0, high = (sub & 2u) != 0;
+    const double lo = (odd ? part[1] : part[0]) + shfl_xor(odd ? part[0] : part[1], 1);
+    const double hi = (odd ? part[3] : part[2]) + shfl_xor(odd ? part[2] : part[3], 1);
+    sum = (high ? hi : lo) + shfl_xor(high ? lo : hi, 2);
+  }
   const uint32_t ax = sub;
   double v = sum;
   if (!ok || (!PE && ax == 3u)) return;
