@@ -8,7 +8,12 @@
 //   Stage 1 (FP32): the warp filters one particle's list at a time, up to 96
 //     entries in flight, against rc^2 plus the proven FP32 error bound; ballots
 //     append the entries to the particle's row in shared memory, in list order.
-//     Entries inside the band around rc^2 carry a flag.
+//     Entries inside the band around rc^2 carry a flag. Short lists (the eight hold
+//     at most 96 entries) are filtered at once, a lane per entry: with one list at
+//     a time forces below a density of 0.1 were slower than by one thread per
+//     particle (953,312 atoms, kFp64 / Newton, at 0.02: 187 / 207 us by one thread
+//     per particle, 320 / 294 one list at a time, 188 / 204 now; at 0.05: 325 / 345,
+//     371 / 348 and 268 / 224).
 //   Stage 2 (FP64), kFp64: four lanes per particle take every fourth of its pairs,
 //     18 FP64 instructions each (24 with the exact d2, a reciprocal of two Newton
 //     steps and a compare per pair); flagged entries take the reference's d2 test
@@ -66,6 +71,27 @@ __device__ __forceinline__ double reciprocal(double d) {
 
 __device__ __forceinline__ double shfl_xor(double v, int mask) { return __shfl_xor_sync(0xffffffffu, v, mask); }
 
+// Entry e, whose particle's mirror is hb, of a particle at o: false when it is surely
+// beyond the cutoff, and e marked when FP32 does not decide.
+__device__ __forceinline__ bool filter(const SysDesc& S, uint32_t& e, float4 hb, float ox, float oy, float oz) {
+  const float r2_out = S.rc2_f + S.pre_margin_f, r2_in = S.rc2_f - S.pre_margin_f, r2_min = S.pre_margin_f;
+  const uint32_t code = e & 31u;
+  if (code != static_cast<uint32_t>(kImageCenter)) {
+    hb.x = image_coord_f(hb.x, S.period_f[0], static_cast<int>(code % 3u));
+    hb.y = image_coord_f(hb.y, S.period_f[1], static_cast<int>((code / 3u) % 3u));
+    hb.z = image_coord_f(hb.z, S.period_f[2], static_cast<int>(code / 9u));
+  }
+  const float dx = hb.x - ox, dy = hb.y - oy, dz = hb.z - oz;
+  const float d2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+  e |= d2 < r2_in && d2 > r2_min ? 0u : kCheck;
+  return d2 <= r2_out;
+}
+
+// Bits of the 32 from `base` on that lie below `end`.
+__device__ __forceinline__ unsigned below(uint32_t end, uint32_t base) {
+  return end <= base ? 0u : (end - base >= 32u ? 0xffffffffu : (1u << (end - base)) - 1u);
+}
+
 // Forces (and energies) of particles first .. first + 7; every lane of the warp
 // calls. NEWTON (kFp64): the lower half of each list, the reactions and the
 // particle's own sum by FP64 reductions into cleared fields.
@@ -86,51 +112,92 @@ __device__ __forceinline__ void eight_particles(uint32_t first, uint32_t n_part,
   if (sub == 3u) sm.sys[mine] = s;
   const SysDesc& S = src.sys[s];
   const uint32_t longest = __reduce_max_sync(full, n);
+  uint32_t off = n;  // entries of the particles before `mine`
+#pragma unroll
+  for (int d = 4; d < 32; d <<= 1) {
+    const uint32_t v = __shfl_up_sync(full, off, d);
+    if (lane >= static_cast<uint32_t>(d)) off += v;
+  }
+  const uint32_t entries = __shfl_sync(full, off, 31);
+  off -= n;
   double sum = 0.0;  // component `sub` of particle `mine`
   double part[4] = {0.0, 0.0, 0.0, 0.0};  // kFp64, full lists: the components over this lane's pairs
 
   for (uint32_t kb = 0; kb < longest; kb += kChunk) {
     // ---- stage 1 ----
-    uint32_t count = 0, total = 0;
-    for (uint32_t p = 0; p < kPer; ++p) {
-      const int from = static_cast<int>(4u * p);
-      const uint32_t np = __shfl_sync(full, n, from);
-      if (NEWTON && lane == 0) sm.start[p] = total;
-      if (np <= kb) continue;
-      const uint32_t* L = reinterpret_cast<const uint32_t*>(
-          __shfl_sync(full, reinterpret_cast<unsigned long long>(list), from));
-      const SysDesc& T = src.sys[__shfl_sync(full, s, from)];
-      const float ox = __shfl_sync(full, own.x, from), oy = __shfl_sync(full, own.y, from),
-                  oz = __shfl_sync(full, own.z, from);
-      const float r2_out = T.rc2_f + T.pre_margin_f, r2_in = T.rc2_f - T.pre_margin_f, r2_min = T.pre_margin_f;
-      const uint32_t base = T.part_base, left = np - kb;
-      uint32_t e[3];
-      float4 hb[3];
-#pragma unroll
-      for (uint32_t t = 0; t < 3u; ++t) e[t] = 32u * t + lane < left ? __ldg(L + kb + 32u * t + lane) : 0xFFFFFFFFu;
-#pragma unroll
-      for (uint32_t t = 0; t < 3u; ++t)
-        hb[t] = e[t] != 0xFFFFFFFFu ? src.pf[base + (e[t] >> 5)] : make_float4(1.0e18f, 0.f, 0.f, 0.f);
-      uint32_t* const out = sm.row + (NEWTON ? total : p * kRow);
-      uint32_t c = 0;
+    uint32_t count = 0, total = 0, row0 = mine * kRow;
+    if (entries <= kChunk) {
+      // short lists: all eight at once
+      unsigned kept[3] = {0u, 0u, 0u};
 #pragma unroll
       for (uint32_t t = 0; t < 3u; ++t) {
-        const uint32_t code = e[t] & 31u;
-        float bx = hb[t].x, by = hb[t].y, bz = hb[t].z;
-        if (code != static_cast<uint32_t>(kImageCenter) && e[t] != 0xFFFFFFFFu) {
-          bx = image_coord_f(bx, T.period_f[0], static_cast<int>(code % 3u));
-          by = image_coord_f(by, T.period_f[1], static_cast<int>((code / 3u) % 3u));
-          bz = image_coord_f(bz, T.period_f[2], static_cast<int>(code / 9u));
+        if (32u * t >= entries) break;
+        const uint32_t f = 32u * t + lane;
+        int p = 0;  // f's particle: the last that starts at or before it
+#pragma unroll
+        for (int step = 4; step > 0; step >>= 1) {
+          const uint32_t o = __shfl_sync(full, off, 4 * (p + step));
+          if (o <= f) p += step;
         }
-        const float dx = bx - ox, dy = by - oy, dz = bz - oz;
-        const float d2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-        const bool keep = e[t] != 0xFFFFFFFFu && d2 <= r2_out;
-        const unsigned m = __ballot_sync(full, keep);
-        if (keep) out[c + __popc(m & lt)] = e[t] | (d2 < r2_in && d2 > r2_min ? 0u : kCheck);
-        c += __popc(m);
+        const int from = 4 * p;
+        const uint32_t k = f - __shfl_sync(full, off, from);
+        const uint32_t* L = reinterpret_cast<const uint32_t*>(
+            __shfl_sync(full, reinterpret_cast<unsigned long long>(list), from));
+        const SysDesc& T = src.sys[__shfl_sync(full, s, from)];
+        const float ox = __shfl_sync(full, own.x, from), oy = __shfl_sync(full, own.y, from),
+                    oz = __shfl_sync(full, own.z, from);
+        uint32_t e = 0;
+        bool keep = false;
+        if (f < entries) {
+          e = __ldg(L + k);
+          const float4 hb = src.pf[T.part_base + (e >> 5)];
+          keep = filter(T, e, hb, ox, oy, oz);
+        }
+        kept[t] = __ballot_sync(full, keep);
+        if (keep) sm.row[total + __popc(kept[t] & lt)] = e;
+        total += __popc(kept[t]);
       }
-      if (mine == p) count = c;
-      total += c;
+      // entries kept before the particle's first, and before its end
+      row0 = 0;
+      uint32_t end = 0;
+#pragma unroll
+      for (uint32_t t = 0; t < 3u; ++t) {
+        row0 += __popc(kept[t] & below(off, 32u * t));
+        end += __popc(kept[t] & below(off + n, 32u * t));
+      }
+      count = end - row0;
+      if (NEWTON && sub == 0) sm.start[mine] = row0;
+    } else {
+      for (uint32_t p = 0; p < kPer; ++p) {
+        const int from = static_cast<int>(4u * p);
+        const uint32_t np = __shfl_sync(full, n, from);
+        if (NEWTON && lane == 0) sm.start[p] = total;
+        if (np <= kb) continue;
+        const uint32_t* L = reinterpret_cast<const uint32_t*>(
+            __shfl_sync(full, reinterpret_cast<unsigned long long>(list), from));
+        const SysDesc& T = src.sys[__shfl_sync(full, s, from)];
+        const float ox = __shfl_sync(full, own.x, from), oy = __shfl_sync(full, own.y, from),
+                    oz = __shfl_sync(full, own.z, from);
+        const uint32_t base = T.part_base, left = np - kb;
+        uint32_t e[3];
+        float4 hb[3];
+#pragma unroll
+        for (uint32_t t = 0; t < 3u; ++t) e[t] = 32u * t + lane < left ? __ldg(L + kb + 32u * t + lane) : 0xFFFFFFFFu;
+#pragma unroll
+        for (uint32_t t = 0; t < 3u; ++t)
+          hb[t] = e[t] != 0xFFFFFFFFu ? src.pf[base + (e[t] >> 5)] : make_float4(1.0e18f, 0.f, 0.f, 0.f);
+        uint32_t* const out = sm.row + (NEWTON ? total : p * kRow);
+        uint32_t c = 0;
+#pragma unroll
+        for (uint32_t t = 0; t < 3u; ++t) {
+          const bool keep = e[t] != 0xFFFFFFFFu && filter(T, e[t], hb[t], ox, oy, oz);
+          const unsigned m = __ballot_sync(full, keep);
+          if (keep) out[c + __popc(m & lt)] = e[t];
+          c += __popc(m);
+        }
+        if (mine == p) count = c;
+        total += c;
+      }
     }
     if (NEWTON && lane == 0) sm.start[kPer] = total;
     __syncwarp();
@@ -230,7 +297,7 @@ __device__ __forceinline__ void eight_particles(uint32_t first, uint32_t n_part,
         for (uint32_t l = p0 / run; l <= (p1 - 1u) / run; ++l) sum += sm.piece[l + mine][sub];
     } else if constexpr (P == kFp64) {
       // four lanes per particle, each every fourth of its pairs
-      const uint32_t* const row = sm.row + mine * kRow;
+      const uint32_t* const row = sm.row + row0;
       const uint32_t pbase = S.part_base;
       const double xa = sm.pos[mine][0], ya = sm.pos[mine][1], za = sm.pos[mine][2];
       const double sig2 = S.sig2, pd_a = S.pd_a, pd_b = S.pd_b;
@@ -271,7 +338,7 @@ __device__ __forceinline__ void eight_particles(uint32_t first, uint32_t n_part,
         if (PE) part[3] += 0.5 * fma(S.eps4 * s6, s6 - 1.0, -S.e_shift);
       }
     } else {
-      const uint32_t* const row = sm.row + mine * kRow;
+      const uint32_t* const row = sm.row + row0;
       const uint32_t rounds = (__reduce_max_sync(full, count) + 3u) >> 2, pbase = S.part_base;
       const double xa = sm.pos[mine][0], ya = sm.pos[mine][1], za = sm.pos[mine][2];
       uint32_t e = 0;
