@@ -68,7 +68,13 @@ int launch_force(const Extent& ex, const SysDesc* sys, SysState* st, const DevAr
 // streams lose at no density: 10 steps of 55,296 atoms at 0.75, 0.84 and 1.0
 // 731 / 705, 757 / 780 and 808 / 858 us, of 62,500 atoms 832 / 770, 876 / 835 and
 // 933 / 950 us (one batch alone 920 / 1268 and 998 / 1289 us at 0.84).
-constexpr uint32_t kMixedSplitMax = 50000;
+// Short lists leave its second stage little and one thread's walk short: batches of
+// more particles than kMixedSplitPerSlot times the list slot (which holds about 1.6
+// times the mean list, and 16) keep the walk. Per graph step, two-stage / one-thread:
+// at density 0.02 (slot 24) 16,384 atoms 67.6 / 67.3 us, 32,000 101 / 95, 48,668
+// 155 / 143; at 0.08 (32) 32,000 67.1 / 69.0, 42,592 78.4 / 76.1; at 0.15 (40)
+// 42,592 73.5 / 76.1, 48,668 84.9 / 84.2; at 0.2 (48) 48,668 80.7 / 83.8.
+constexpr uint32_t kMixedSplitMax = 50000, kMixedSplitPerSlot = 1200;
 int launch_force_mixed(const Extent& ex, const SysDesc* sys, const SysState* st, const DevArrays& a, bool with_pe,
                        bool second_half, int sys_only, cudaStream_t stream);
 

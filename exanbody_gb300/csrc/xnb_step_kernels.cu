@@ -444,6 +444,13 @@ void force_dispatch(const Extent& ex, const SysDesc* sys, const SysState* st, co
   else
     k_force<PE, KICK><<<grid_for(ex.n_part, threads), threads, 0, stream>>>(ex.n_part, src, f);
 }
+void force_dispatch(const Extent& ex, const SysDesc* sys, const SysState* st, const DevArrays& a, bool with_pe,
+                    bool second_half, int sys_only, cudaStream_t stream) {
+  if (with_pe && second_half) force_dispatch<true, true>(ex, sys, st, a, sys_only, stream);
+  else if (with_pe) force_dispatch<true, false>(ex, sys, st, a, sys_only, stream);
+  else if (second_half) force_dispatch<false, true>(ex, sys, st, a, sys_only, stream);
+  else force_dispatch<false, false>(ex, sys, st, a, sys_only, stream);
+}
 
 // ---------------------------------------------------------------------------
 // Persistent step loop: one cooperative launch advances the batch step after
@@ -559,16 +566,19 @@ int launch_force(const Extent& ex, const SysDesc* sys, SysState* st, const DevAr
   }
   if (precision == kMixed && ex.force_form == kForceStaged && a.nbr16 && a.seg && !ex.unpacked)
     return launch_force_staged(ex, sys, st, a, with_pe, second_half, sys_only, stream);
-  if (precision == kMixed && !ex.unpacked && ex.n_part <= kMixedSplitMax)
-    return launch_force_mixed(ex, sys, st, a, with_pe, second_half, sys_only, stream);
+  if (precision == kMixed && !ex.unpacked && ex.n_part <= kMixedSplitMax) {
+    if (ex.n_part <= kMixedSplitPerSlot * ex.list_slot)
+      return launch_force_mixed(ex, sys, st, a, with_pe, second_half, sys_only, stream);
+    Extent one = ex;
+    one.force_lanes = 1;  // the same bits
+    force_dispatch(one, sys, st, a, with_pe, second_half, sys_only, stream);
+    return 1;
+  }
   if (precision == kMixed && !ex.general && ex.force_lanes == 1 && ex.n_part >= kMixedWalkMin)
     return launch_force_walk(ex, sys, st, a, with_pe, second_half, sys_only, stream);
   if (precision != kMixed)
     return launch_force_pairs(ex, sys, st, a, precision, false, with_pe, second_half, sys_only, stream);
-  if (with_pe && second_half) force_dispatch<true, true>(ex, sys, st, a, sys_only, stream);
-  else if (with_pe) force_dispatch<true, false>(ex, sys, st, a, sys_only, stream);
-  else if (second_half) force_dispatch<false, true>(ex, sys, st, a, sys_only, stream);
-  else force_dispatch<false, false>(ex, sys, st, a, sys_only, stream);
+  force_dispatch(ex, sys, st, a, with_pe, second_half, sys_only, stream);
   return 1;
 }
 
