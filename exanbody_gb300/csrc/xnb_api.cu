@@ -1150,7 +1150,8 @@ int xnb_step(xnb_batch* b, int32_t nsteps, int32_t precision, int32_t flags, voi
     rc = check_launch();
     if (rc) return rc;
     if (fused) {
-      b->launches += launch_rebin_fused(ex, b->d_sys, b->d_st, b->a, exact, build, b->stage_cap, list_buf(b), st);
+      b->launches += launch_rebin_fused(ex, b->d_sys, b->d_st, b->a, exact, build, b->stage_cap, list_buf(b),
+                                        (flags & XNB_STEP_BARRIER_CHECK) != 0, st);
       rc = check_launch();
       if (!rc && !build) {
         b->launches += launch_neighbors(ex, b->d_sys, b->d_st, b->a, b->stage_cap, list_buf(b), st, b->build_form,

@@ -1102,11 +1102,14 @@ __global__ void __launch_bounds__(128, 5)
 template <bool EXACT, bool BUILD>
 __global__ void __launch_bounds__(256)
     k_rebin_fused(uint32_t n_part, uint32_t n_cells, int nsys, const SysDesc* __restrict__ sys, SysState* st,
-                  DevArrays a, int cap, int lbuf, uint32_t split) {
+                  DevArrays a, int cap, int lbuf, uint32_t split, bool check) {
   extern __shared__ float4 fused_smem[];
+  const auto triggered = [&](int s) {
+    return __ldcg(&st[s].moved) != 0ull && !(__ldcg(&st[s].error) & kErrBarrier);
+  };
   int flagged = 0;
   for (int s = static_cast<int>(threadIdx.x); s < nsys; s += static_cast<int>(blockDim.x))
-    flagged |= __ldcg(&st[s].moved) != 0ull ? 1 : 0;
+    flagged |= triggered(s) ? 1 : 0;
   if (!__syncthreads_or(flagged)) {
     if (blockIdx.x == 0) {
       for (int s = static_cast<int>(threadIdx.x); s < nsys; s += static_cast<int>(blockDim.x)) st[s].rebuild = 0;
@@ -1115,10 +1118,10 @@ __global__ void __launch_bounds__(256)
     return;
   }
   if (blockIdx.x == 0) {
-    // what the other blocks read before the first barrier is `moved` alone
+    // what the other blocks read before the first barrier is `moved` and `error`
     unsigned int mine = 0;
     for (int s = static_cast<int>(threadIdx.x); s < nsys; s += static_cast<int>(blockDim.x)) {
-      const bool r = __ldcg(&st[s].moved) != 0ull;
+      const bool r = triggered(s);
       st[s].rebuild = r ? 1u : 0u;
       if (!r) continue;
       ++mine;
@@ -1140,7 +1143,8 @@ __global__ void __launch_bounds__(256)
     __syncthreads();
     if (mine) atomicAdd(a.any_rebuild, mine);
   }
-  bool ok = grid_barrier(a.grid_ctl, gridDim.x);
+  // check: one block more than there are, for 20 ms
+  bool ok = check ? grid_barrier(a.grid_ctl, gridDim.x + 1u, 20000000ull) : grid_barrier(a.grid_ctl, gridDim.x);
   if (ok) {
     if (blockIdx.x == 0)
       for (int s = static_cast<int>(threadIdx.x); s < nsys; s += static_cast<int>(blockDim.x)) st[s].moved = 0;
@@ -1363,7 +1367,7 @@ bool fused_build_fits(const Extent& ex, int form, bool prune) {
 }
 
 int launch_rebin_fused(const Extent& ex, const SysDesc* sys, SysState* st, const DevArrays& a, bool exact_backup,
-                       bool build, int cap, int lbuf, cudaStream_t stream) {
+                       bool build, int cap, int lbuf, bool check, cudaStream_t stream) {
   constexpr unsigned warps = 8;
   // at most one block per SM: always co-resident. The rebin takes a warp per
   // cell, the build up to four
@@ -1388,7 +1392,7 @@ int launch_rebin_fused(const Extent& ex, const SysDesc* sys, SysState* st, const
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, kern, ex.n_part, ex.n_cells, ex.nsys, sys, st, a, cap, lbuf, split);
+  cudaLaunchKernelEx(&cfg, kern, ex.n_part, ex.n_cells, ex.nsys, sys, st, a, cap, lbuf, split, check);
   return 1;
 }
 

@@ -38,7 +38,9 @@ enum ErrorBits : uint32_t {
   kErrBarrier = 1u << 4,        // a grid barrier of the fused rebin ran out of time
 };
 
-// State of a grid barrier (xnb_grid_barrier.cuh); zeroed once, left ready by each launch.
+// State of a grid barrier (xnb_grid_barrier.cuh). Left ready by a launch whose waits
+// all ended; `arrive` and `error` are cleared before each launch (the persistent
+// loop's by a memset, the fused rebin's by the push before it).
 struct GridBarrier {
   unsigned int arrive;      // blocks arrived at the current barrier
   unsigned int generation;  // barriers completed

@@ -147,7 +147,7 @@ bool fused_rebin_fits(const Extent& ex);
 constexpr uint32_t kFusedBuildMaxCells = 1024;
 bool fused_build_fits(const Extent& ex, int form, bool prune);
 int launch_rebin_fused(const Extent& ex, const SysDesc* sys, SysState* st, const DevArrays& a, bool exact_backup,
-                       bool build, int cap, int lbuf, cudaStream_t stream);
+                       bool build, int cap, int lbuf, bool check, cudaStream_t stream);
 int launch_backup(const Extent& ex, const SysDesc* sys, SysState* st, const DevArrays& a, cudaStream_t stream);
 // chunk_neighbors for systems with rebuild != 0: one pass writing each list
 // into its particle's slot (statistics reset, the warp-per-cell build, and the

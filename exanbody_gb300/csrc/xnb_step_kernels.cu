@@ -141,6 +141,11 @@ template <bool EXACT>
 __global__ void __launch_bounds__(256)
     k_first_half(uint32_t n_part, int nsys, const SysDesc* __restrict__ sys, SysState* __restrict__ st, DevArrays a,
                  bool push_r, bool push_v, bool trigger, double scale_r, double scale_v, int sys_only) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    // what a fused rebin whose barrier ran out of time left behind
+    a.grid_ctl->arrive = 0;
+    a.grid_ctl->error = 0;
+  }
   first_half_body<EXACT>(n_part, nsys, sys, st, a, push_r, push_v, trigger, scale_r, scale_v, sys_only, nullptr);
 }
 
@@ -394,7 +399,8 @@ __global__ void k_mark_rebuild(int nsys, SysState* st, int mode, int sys_only, u
     return;
   }
   // mode 0: every system (init); mode 1: systems whose trigger fired; mode 2: none
-  const uint32_t r = mode == 0 ? 1u : (mode == 1 ? (st[s].moved > 0 ? 1u : 0u) : 0u);
+  const bool whole = !(st[s].error & kErrBarrier);
+  const uint32_t r = whole && (mode == 0 || (mode == 1 && st[s].moved > 0)) ? 1u : 0u;
   st[s].rebuild = r;
   if (r) {
     st[s].rebuilds += 1;

@@ -52,13 +52,20 @@ extern "C" {
 #define XNB_STEP_ENERGY 2    /* also write per-particle potential energy */
 /* xnb_step_persistent diagnostic: the loop's first grid barrier waits for one
  * block more than the launch has, so every wait runs out after 20 ms; the call
- * returns XNB_ERR_DEVICE and no state changes (tests the barrier's time limit) */
+ * returns XNB_ERR_DEVICE and no state changes (tests the barrier's time limit).
+ * xnb_step: the same for the first grid barrier of a rebuild that runs as one
+ * cooperative launch (asynchronous steps of up to 100,000 particles); the systems
+ * that were to be rebuilt get XNB_ERRBIT_BARRIER. */
 #define XNB_STEP_BARRIER_CHECK 0x100
 
 /* Error bits of xnb_system_info.error_bits */
 #define XNB_ERRBIT_LIST_OVERFLOW 1u
 #define XNB_ERRBIT_FAR_MOVER 2u
 #define XNB_ERRBIT_CELL_INDEX 4u
+/* a grid barrier of the system's rebuild ran out of time: it is not rebuilt any more
+ * (its cell tables may be half written); remove it. The batch's other systems, and
+ * those added later, go on. */
+#define XNB_ERRBIT_BARRIER 16u
 
 typedef struct xnb_batch xnb_batch;
 typedef struct xnb_graph xnb_graph;
