@@ -1442,9 +1442,14 @@ int xnb_autotune(xnb_batch* b, int32_t trial_steps, int32_t precision, void* str
   // coordinate search: one parameter at a time, the others at their best so far
   // (neighbour-build form, the stage cap of the forms that stage whole
   // neighbourhoods, the force block size, threads per particle of the force
-  // traversal and the Newton traversal)
+  // traversal and the Newton traversal); a knob that the batch's forces do not read
+  // keeps its value: trials would time the same kernels
+  const Extent ex = b->extent();
+  const ForceRoute route = force_route(ex, b->a, precision);
+  const bool searched[5] = {true, true, reads_force_block(route), reads_force_lanes(ex, route), true};
   const int nvals[5] = {2, 3, 3, 3, 2};
   for (int pass = 0; pass < 5 && rc == 0; ++pass) {
+    if (!searched[pass]) continue;
     // the pass's knob at its value when the pass starts was timed already (the
     // other knobs stay as they are through the pass): it is not timed again
     // after another value of the knob took the lead

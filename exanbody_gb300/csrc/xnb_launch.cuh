@@ -74,7 +74,7 @@ int launch_force(const Extent& ex, const SysDesc* sys, SysState* st, const DevAr
 // at density 0.02 (slot 24) 16,384 atoms 67.6 / 67.3 us, 32,000 101 / 95, 48,668
 // 155 / 143; at 0.08 (32) 32,000 67.1 / 69.0, 42,592 78.4 / 76.1; at 0.15 (40)
 // 42,592 73.5 / 76.1, 48,668 84.9 / 84.2; at 0.2 (48) 48,668 80.7 / 83.8.
-constexpr uint32_t kMixedSplitMax = 50000, kMixedSplitPerSlot = 1200;
+constexpr uint32_t kMixedSplitMax = XNB_MIXED_SPLIT_MAX, kMixedSplitPerSlot = 1200;
 int launch_force_mixed(const Extent& ex, const SysDesc* sys, const SysState* st, const DevArrays& a, bool with_pe,
                        bool second_half, int sys_only, cudaStream_t stream);
 
@@ -91,6 +91,24 @@ int launch_force_mixed(const Extent& ex, const SysDesc* sys, const SysState* st,
 constexpr uint32_t kMixedWalkMin = 500000;
 int launch_force_walk(const Extent& ex, const SysDesc* sys, const SysState* st, const DevArrays& a, bool with_pe,
                       bool second_half, int sys_only, cudaStream_t stream);
+
+// The kernel of launch_force for full lists.
+enum class ForceRoute {
+  kPairs,       // FP64, FP64_EXACT: launch_force_pairs
+  kStaged,      // mixed: launch_force_staged
+  kTwoStage,    // launch_force_mixed
+  kShortLists,  // the marking walk in its place, one thread per particle
+  kWalk,        // launch_force_walk
+  kMarks,       // the marking walk, force_lanes threads per particle
+};
+ForceRoute force_route(const Extent& ex, const DevArrays& a, int precision);
+// whether it reads the batch's threads per particle, and threads per block
+inline bool reads_force_lanes(const Extent& ex, ForceRoute r) {
+  return (r == ForceRoute::kMarks || r == ForceRoute::kWalk) && !ex.unpacked;
+}
+inline bool reads_force_block(ForceRoute r) {
+  return r == ForceRoute::kMarks || r == ForceRoute::kWalk || r == ForceRoute::kShortLists;
+}
 
 // FP64 and FP64_EXACT forces over full lists, or FP64 over their lower halves
 // with FP64 reductions into cleared fields (newton; no kick) (xnb_force_pairs.cu).

@@ -549,6 +549,16 @@ int launch_first_half(const Extent& ex, const SysDesc* sys, SysState* st, const 
   return 1;
 }
 
+ForceRoute force_route(const Extent& ex, const DevArrays& a, int precision) {
+  if (precision != kMixed) return ForceRoute::kPairs;
+  if (ex.unpacked) return ForceRoute::kMarks;
+  if (ex.force_form == kForceStaged && a.nbr16 && a.seg) return ForceRoute::kStaged;
+  if (ex.n_part <= kMixedSplitMax)
+    return ex.n_part <= kMixedSplitPerSlot * ex.list_slot ? ForceRoute::kTwoStage : ForceRoute::kShortLists;
+  if (!ex.general && ex.force_lanes == 1 && ex.n_part >= kMixedWalkMin) return ForceRoute::kWalk;
+  return ForceRoute::kMarks;
+}
+
 int launch_force(const Extent& ex, const SysDesc* sys, SysState* st, const DevArrays& a, int precision, bool with_pe,
                   bool second_half, int sys_only, cudaStream_t stream, bool newton) {
   if (ex.n_part == 0) return 0;
@@ -570,22 +580,21 @@ int launch_force(const Extent& ex, const SysDesc* sys, SysState* st, const DevAr
     k_force_finish<<<g, threads, 0, stream>>>(ex.n_part, sys, st, a, sys_only, second_half);
     return 3;
   }
-  if (precision == kMixed && ex.force_form == kForceStaged && a.nbr16 && a.seg && !ex.unpacked)
-    return launch_force_staged(ex, sys, st, a, with_pe, second_half, sys_only, stream);
-  if (precision == kMixed && !ex.unpacked && ex.n_part <= kMixedSplitMax) {
-    if (ex.n_part <= kMixedSplitPerSlot * ex.list_slot)
-      return launch_force_mixed(ex, sys, st, a, with_pe, second_half, sys_only, stream);
-    Extent one = ex;
-    one.force_lanes = 1;  // the same bits
-    force_dispatch(one, sys, st, a, with_pe, second_half, sys_only, stream);
-    return 1;
+  switch (force_route(ex, a, precision)) {
+    case ForceRoute::kPairs:
+      return launch_force_pairs(ex, sys, st, a, precision, false, with_pe, second_half, sys_only, stream);
+    case ForceRoute::kStaged: return launch_force_staged(ex, sys, st, a, with_pe, second_half, sys_only, stream);
+    case ForceRoute::kTwoStage: return launch_force_mixed(ex, sys, st, a, with_pe, second_half, sys_only, stream);
+    case ForceRoute::kWalk: return launch_force_walk(ex, sys, st, a, with_pe, second_half, sys_only, stream);
+    case ForceRoute::kShortLists: {
+      Extent one = ex;
+      one.force_lanes = 1;  // the bits of the two-stage form
+      force_dispatch(one, sys, st, a, with_pe, second_half, sys_only, stream);
+      return 1;
+    }
+    case ForceRoute::kMarks: force_dispatch(ex, sys, st, a, with_pe, second_half, sys_only, stream); return 1;
   }
-  if (precision == kMixed && !ex.general && ex.force_lanes == 1 && ex.n_part >= kMixedWalkMin)
-    return launch_force_walk(ex, sys, st, a, with_pe, second_half, sys_only, stream);
-  if (precision != kMixed)
-    return launch_force_pairs(ex, sys, st, a, precision, false, with_pe, second_half, sys_only, stream);
-  force_dispatch(ex, sys, st, a, with_pe, second_half, sys_only, stream);
-  return 1;
+  return 0;
 }
 
 int launch_mark_rebuild(const Extent& ex, SysState* st, int mode, int sys_only, unsigned int* any,

@@ -89,7 +89,8 @@ def trial(systems, cfg, steps, precision, stream):
 
 
 def autotune(systems, precision=xnb.PREC_MIXED, steps=40, tune_skin=False, stream=None):
-    """Coordinate search over the tunables on the given systems (a sample of the batch)."""
+    """Coordinate search over the tunables on the given systems (a sample of the batch). The force settings that
+    their forces do not read (FP64, and mixed up to MIXED_SPLIT_MAX particles) keep their defaults."""
     import torch
 
     stream = stream or torch.cuda.Stream()
@@ -101,6 +102,8 @@ def autotune(systems, precision=xnb.PREC_MIXED, steps=40, tune_skin=False, strea
         "newton": [False, True],
         "skin": [0.3, 0.4, 0.5] if tune_skin else [0.3],
     }
+    if systems and (precision != xnb.PREC_MIXED or sum(w["n_atoms"] for w in systems) <= xnb.MIXED_SPLIT_MAX):
+        space["force_block"], space["force_lanes"] = [DEFAULTS["force_block"]], [DEFAULTS["force_lanes"]]
     best = dict(DEFAULTS)
     best_rate = trial(systems, best, steps, precision, stream)
     log = [dict(best, rate=best_rate)]

@@ -38,6 +38,7 @@ ERRBIT_LIST_OVERFLOW = 1
 ERRBIT_FAR_MOVER = 2
 ERRBIT_CELL_INDEX = 4
 ERRBIT_BARRIER = 16
+MIXED_SPLIT_MAX = 50000
 
 EXPORTED = [
     "xnb_last_error_string", "xnb_version", "xnb_batch_create", "xnb_batch_destroy", "xnb_system_bytes",

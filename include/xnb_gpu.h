@@ -227,6 +227,10 @@ typedef struct xnb_tuning {
   int32_t reserved;
 } xnb_tuning;
 
+/* Mixed batches of up to this many particles spread a particle's list over threads by
+ * themselves. */
+#define XNB_MIXED_SPLIT_MAX 50000
+
 /* Threads per particle (1, 2 or 4) of the mixed full-list force traversal of
  * batches of more than 50,000 particles: the particle's list is split in 8-entry
  * blocks dealt round-robin to the threads and their partial sums combined in a
@@ -291,7 +295,9 @@ int xnb_batch_set_tuning(xnb_batch* b, int32_t stage_cap, int32_t force_block);
 /* Online autotuner: coordinate search over the neighbour-build form
  * {ROWS, WARP}, stage_cap {384, 640, 1024}, force_block {64, 128, 256}, force
  * threads per particle {1, 2, 4} and the Newton traversal (the batch's force
- * form is kept), each configuration timed
+ * form is kept, and so are the two force settings where the batch's forces of that
+ * precision do not read them: FP64, and mixed up to XNB_MIXED_SPLIT_MAX particles),
+ * each configuration timed
  * (CUDA events on `stream`) over trial_steps of xnb_step without host sync
  * after one untimed step. The trials are real MD steps: the batch advances
  * (1 + trial_steps) x trials steps. The batch is left on the fastest
