@@ -582,7 +582,7 @@ int xnb_batch_create(const xnb_batch_config* cfg, xnb_batch** out) {
   rc = rc ? rc : dalloc(b, &a.id, P);
   rc = rc ? rc : dalloc(b, &a.pf, P);
   rc = rc ? rc : dalloc(b, &a.pflo, P);
-  rc = rc ? rc : dalloc(b, &a.pstep, P);
+  if (P >= kMixedWalkMin) rc = rc ? rc : dalloc(b, &a.pstep, P);
   rc = rc ? rc : dalloc(b, &a.rbf, P);
   rc = rc ? rc : dalloc(b, &a.nbr_half, P);
   rc = rc ? rc : dalloc(b, &a.any_rebuild, 4);
@@ -814,7 +814,8 @@ int place_system(xnb_batch* b, const xnb_lj_params* p, int64_t n, const double* 
     }
     XCK(cudaMemcpyAsync(a.pf + poff, hpf.data(), nb * sizeof(float4), cudaMemcpyHostToDevice, st));
     XCK(cudaMemcpyAsync(a.pflo + poff, hlo.data(), nb * sizeof(float4), cudaMemcpyHostToDevice, st));
-    XCK(cudaMemsetAsync(a.pstep + poff, 0xFF, nb * sizeof(int4), st));  // none: FP64 until the first rebin
+    if (a.pstep)
+      XCK(cudaMemsetAsync(a.pstep + poff, 0xFF, nb * sizeof(int4), st));  // none: FP64 until the first rebin
     XCK(cudaMemsetAsync(a.fx + poff, 0, nb * sizeof(double), st));
     XCK(cudaMemsetAsync(a.fy + poff, 0, nb * sizeof(double), st));
     XCK(cudaMemsetAsync(a.fz + poff, 0, nb * sizeof(double), st));

@@ -383,7 +383,7 @@ __device__ __forceinline__ void rebin_finalize(uint32_t n_cells, const SysDesc* 
       make_pf2(S, x, y, z, mhi, mlo);
       a.pf[dst] = mhi;
       a.pflo[dst] = mlo;
-      a.pstep[dst] = make_steps(x, y, z, mhi);
+      if (a.pstep) a.pstep[dst] = make_steps(x, y, z, mhi);
       if constexpr (BACKUP == kBackupExact) {
         store_backup(S, a, dst, lo, x, y, z);
       } else if constexpr (BACKUP == kBackupPlain) {

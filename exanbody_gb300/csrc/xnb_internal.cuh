@@ -131,7 +131,8 @@ struct DevArrays {
   float4* pf;                      // FP32 hi part of (x - origin, y - origin, z - origin), refreshed with r;
                                    // .w packs the three residuals as 10-bit multiples of lo_step_f (lo_field)
   float4* pflo;                    // FP32 residual (x - origin) - hi, so hi + lo carries ~48 bits
-  int4* pstep;                     // rx, ry, rz as steps of their FP64 bit patterns from those of pf (origin zero)
+  int4* pstep;                     // rx, ry, rz as steps of their FP64 bit patterns from those of pf (origin zero);
+                                   // null in batches too small for the one kernel that reads it (k_force_walk)
   GridBarrier* grid_ctl;           // of the fused rebin
   unsigned int* any_rebuild;       // number of systems flagged for the rebuild path this step
   uint64_t* id;

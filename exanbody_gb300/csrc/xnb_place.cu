@@ -86,7 +86,7 @@ __global__ void __launch_bounds__(128)
       a.pflo[dst] = make_float4(static_cast<float>(ox - static_cast<double>(hi.x)),
                                 static_cast<float>(oy - static_cast<double>(hi.y)),
                                 static_cast<float>(oz - static_cast<double>(hi.z)), 0.f);
-      a.pstep[dst] = make_int4(0, 0, 0, 1);  // none: FP64 until the first rebin
+      if (a.pstep) a.pstep[dst] = make_int4(0, 0, 0, 1);  // none: FP64 until the first rebin
       a.fx[dst] = 0.0;
       a.fy[dst] = 0.0;
       a.fz[dst] = 0.0;

@@ -82,7 +82,7 @@ __device__ __forceinline__ void first_half_body(uint32_t n_part, int nsys, const
         make_pf2(S, x, y, z, hi, lo);
         a.pf[i] = hi;
         a.pflo[i] = lo;
-        a.pstep[i] = make_steps(x, y, z, hi);
+        if (a.pstep) a.pstep[i] = make_steps(x, y, z, hi);
         cur_hi = hi;
       } else if (!EXACT && trigger) {
         cur_hi = a.pf[i];
