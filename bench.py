@@ -43,13 +43,34 @@ FLOP64_PER_ATOM_MIXED = 282.2
 FLOP32_PER_ATOM_MIXED = 387.4
 # DRAM bytes (read + write) per atom of one mixed k_force_walk launch, from an ncu capture of
 # the 1,000,188-atom case of this workload (FCC 63^3); traffic grows with the atom count at
-# fixed density, so a launch moves this many bytes per atom.
+# fixed density, so a launch moves this many bytes per atom. (The other kernels have none: below
+# 500,000 atoms their state stays in L2.)
 FORCE_DRAM_BYTES_PER_ATOM = 479.0
 
 
-def mixed_force_kernel(n):
-    """Kernel of the mixed full-list forces of a batch of n particles (kMixedSplitMax, kMixedWalkMin)."""
-    return "k_force_mixed" if n <= 50000 else "k_force<mixed>" if n < 500000 else "k_force_walk"
+def mixed_force_kernel(n, lanes=0, form=""):
+    """Kernel of the mixed full-list forces of this workload's n particles (force_route, xnb_step_kernels.cu)."""
+    from exanbody_gb300 import xnb
+
+    if form == "staged":
+        return "k_force_staged"
+    if n <= xnb.MIXED_SPLIT_MAX:
+        return "k_force_mixed"
+    if lanes > 1:
+        return "k_force_lanes"
+    return "k_force<mixed>" if n < 500000 else "k_force_walk"
+
+
+def force_traffic(kernel, n, ms):
+    """The roofline record's DRAM fields of one force launch: of the captured kernel only."""
+    if kernel != "k_force_walk":
+        return {"traffic": None, "traffic_source": "no capture of %s" % kernel, "hbm": None}
+    moved = FORCE_DRAM_BYTES_PER_ATOM * n
+    gbs = moved / (ms * 1e-3) / 1e9
+    return {"traffic": moved,
+            "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum per atom on the "
+                              "1,000,188-atom case, scaled to %d atoms" % n,
+            "hbm": {"achieved_gbs": gbs, "peak_gbs": hbm_peak_gbs(), "frac": gbs / hbm_peak_gbs()}}
 
 
 WORKLOAD = dict(n=100, rho=0.8442, T=1.44, seed=12345, rcut=2.5, skin=0.3, dt=0.005)
@@ -90,7 +111,8 @@ def cpu_model():
 
 def config_of(n, atoms, **extra):
     c = {"workload": "lj_fcc_%d^3_rho0.8442_T1.44" % n, "atoms": atoms, "rcut": 2.5, "skin": 0.3, "dt": 0.005,
-         "flush": "state %.1f GB > L2 (129 MB)" % (atoms * 600 / 1e9)}
+         "flush": ("state %.1f GB > L2 (129 MB)" % (atoms * 600 / 1e9) if atoms * 600 > 129e6 else
+                   "none: the state (%.1f MB) stays in L2, as in a run" % (atoms * 600 / 1e6))}
     c.update(extra)
     return c
 
@@ -487,6 +509,8 @@ def run_ours(args):
         del so
 
     if rank == 0:
+        kernel = ("k_force_half<mixed> (+ zero/finish launches)" if MIXED & xnb.PREC_NEWTON
+                  else mixed_force_kernel(N, args.force_lanes, args.force_form))
         line = {
             "metric": METRIC,
             "value": value,
@@ -516,18 +540,12 @@ def run_ours(args):
             "e2e": e2e,
             "gpu_launches": launches,
             "roofline": {"bound": "fp64",
-                         "kernel": ("k_force_half<mixed> (+ zero/finish launches)" if MIXED & xnb.PREC_NEWTON
-                                    else mixed_force_kernel(N)),
+                         "kernel": kernel,
                          "achieved": achieved, "peak": peak64,
                          "unit": "TFLOP/s", "frac": achieved / peak64,
                          "peak_source": "cuBLAS DGEMM 4096^3 measured in this run",
                          "ms_per_launch": ms_force, "ms_per_launch_fp64_kernel": ms_force64,
-                         "traffic": FORCE_DRAM_BYTES_PER_ATOM * N,
-                         "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum per atom on the "
-                                           "1,000,188-atom case, scaled to %d atoms" % N,
-                         "hbm": {"achieved_gbs": FORCE_DRAM_BYTES_PER_ATOM * N / (ms_force * 1e-3) / 1e9,
-                                 "peak_gbs": hbm_peak_gbs(),
-                                 "frac": FORCE_DRAM_BYTES_PER_ATOM * N / (ms_force * 1e-3) / 1e9 / hbm_peak_gbs()}},
+                         **force_traffic(kernel, N, ms_force)},
             "cpu_baseline": cpu,
         }
         print(json.dumps(line), flush=True)
