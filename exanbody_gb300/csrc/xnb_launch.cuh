@@ -153,15 +153,23 @@ int launch_rebin(const Extent& ex, const SysDesc* sys, SysState* st, const DevAr
 // The displacement trigger's decision, the rebin and the build's resets in one
 // cooperative launch, for batches it fits: a step without a rebuild then takes
 // one launch here instead of twelve (a 50-step graph of 864 atoms: 0.84 -> 0.51 ms).
-// Beyond 100,000 particles the phases want more warps than one block per SM has;
-// one block scans the cell counts, hence the limit on cells.
+// The gain shrinks as the phases want more warps than one block per SM has; one
+// block scans the cell counts, hence the limit on cells. A step of a graph (of an
+// eager loop), fused / separate, mixed, density 0.84: 32,000 atoms 66 / 78 us (78 /
+// 119), 97,556 151 / 159 (164 / 197), 131,072 182 / 191 (193 / 228), 256,000 322 /
+// 323 (334 / 359); density 0.1: 9,261 cells 54 / 58 us (68 / 99), 13,824 66 / 64 (80 /
+// 101), 17,576 80 / 75 (95 / 113), 42,875 132 / 101 (147 / 141). Both limits are on
+// the near side of where a graph breaks even.
 constexpr uint32_t kFusedRebinMaxParticles = 100000;
 constexpr uint32_t kFusedRebinMaxCells = 16384;
 bool fused_rebin_fits(const Extent& ex);
-// build: the neighbour lists as well, for batches of few cells (one block per SM
-// builds 1,331 cells slower than a launch of their own: 50 steps of 32,000 atoms
-// 2.39 against 2.27 ms; 200 eager steps of 1,000 cells 13.2 against 16.6 ms) too sparse
-// for sub-cell pruning to matter.
+// build: the neighbour lists as well, for batches of few cells too sparse for
+// sub-cell pruning to matter. One block per SM builds the lists slower than a launch
+// of their own and saves two launches in each step. A step of a graph (of an eager
+// loop), in here / on their own: 343 cells 28.6 / 31.1 us (35 / 46), 1,000 51.7 / 53.9
+// (57 / 68), 1,331 66.5 / 65.5 at 32,000 atoms (71 / 79) and 57.0 / 57.5 at 27,436,
+// 2,744 129.5 / 128.7 (134 / 142), 4,096 151 / 149 (157 / 162): graphs break even from
+// 1,331 cells on, eager steps not by 4,913. The line is the graph's.
 constexpr uint32_t kFusedBuildMaxCells = 1024;
 bool fused_build_fits(const Extent& ex, int form, bool prune);
 int launch_rebin_fused(const Extent& ex, const SysDesc* sys, SysState* st, const DevArrays& a, bool exact_backup,

@@ -52,9 +52,10 @@ __device__ __forceinline__ CX<R> cmul(CX<R> a, CX<R> b) {
   return CX<R>{fma(a.r, b.r, -(a.i * b.i)), fma(a.r, b.i, a.i * b.r)};
 }
 
+using R = float;  // what the FP32 kernel computes in
+
 // element (r, c) of level L from its unique-half buffer (stride `st` values
 // per element, complex at offset `off`)
-template <class R>
 __device__ __forceinline__ CX<R> level_get(const R* buf, int st, int off, int L, int r, int c) {
   const int idx = r * (L + 1) + c;
   if (idx < nunique(L)) return CX<R>{buf[idx * st + off], buf[idx * st + off + 1]};
@@ -63,15 +64,11 @@ __device__ __forceinline__ CX<R> level_get(const R* buf, int st, int off, int L,
   return CX<R>{s * buf[k * st + off], -s * buf[k * st + off + 1]};
 }
 
-// the potential's tables in the compute type
-template <class R>
+// the potential's tables of the FP32 kernel
 struct Tabs {
   const R *rootpq, *cg, *zbeta, *zener;
 };
-template <class R>
-__device__ __forceinline__ Tabs<R> tabs(const SnapArgs& t) {
-  return Tabs<float>{t.rootpq_f, t.cg_f, t.zbeta_f, t.zener_f};
-}
+__device__ __forceinline__ Tabs tabs(const SnapArgs& t) { return Tabs{t.rootpq_f, t.cg_f, t.zbeta_f, t.zener_f}; }
 
 __device__ __forceinline__ double warp_sum(double v) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -174,7 +171,6 @@ __device__ __forceinline__ bool uq(int j, int r, int c) {
 // Forward U levels 1..J of one neighbour into its unique-half buffer u (level j
 // at ublk[j]); level 0 is set by the caller. Threads slot, slot + lpn, ... of the
 // neighbour take the elements of each level; the CTA synchronises between levels.
-template <class R>
 __device__ __forceinline__ void forward_levels(R* u, bool active, int slot, int lpn, CX<R> a, CX<R> b,
                                                const SnapArgs& t, const R* rootpq) {
   const int J = t.twojmax;
@@ -209,9 +205,8 @@ __device__ __forceinline__ void forward_levels(R* u, bool active, int slot, int 
   }
 }
 
-// R: the type of the U, Z, Y and adjoint arithmetic (double, or float for the
-// mixed path); geometry, switching and the force sums stay in double.
-template <class R>
+// The mixed path: U, Z, Y and the adjoint in R; geometry, switching and the force
+// sums stay in double.
 __global__ void __launch_bounds__(kSnapThreads)
     k_snap(uint32_t n_part, const SysDesc* __restrict__ sys, const SysState* __restrict__ st, DevArrays a,
            SnapArgs t, int group, int sys_only, bool with_pe, unsigned int* flags) {
@@ -220,8 +215,8 @@ __global__ void __launch_bounds__(kSnapThreads)
   const int J = t.twojmax;
   const int lvl_max = nunique(J);
   const int nu = t.nu_unique;
-  const Tabs<R> T = tabs<R>(t);
-  // shared layout: double part, then the compute-type part
+  const Tabs T = tabs(t);
+  // shared layout: double part, then that of R
   double* nx = sm;
   double* ny = nx + kSnapMaxNbr;
   double* nz = ny + kSnapMaxNbr;
@@ -1386,7 +1381,7 @@ int snap_build(const xnb_snap_params& p, int device, SnapArgs& t, std::vector<vo
     err = "device memory for the SNAP tables";
     return XNB_ERR_NOMEM;
   }
-  // FP32 kernel: a double part (environment, geometry) and a compute-type part:
+  // FP32 kernel: a double part (environment, geometry) and one of floats:
   // U_tot, Y, the U accumulator and, per neighbour of a round, its forward U
   // (unique half of every level) and two adjoint levels, which the force
   // reduction overwrites; rounds of at most 32. The kernel waits for shared memory
@@ -1445,7 +1440,7 @@ int launch_snap(const Extent& ex, const SysDesc* sys, const SysState* st, const 
     k_snap_zero<<<g, 256, 0, stream>>>(ex.n_part, sys, st, a, sys_only, !accumulate, with_pe);
     ++launches;
   }
-  if (mixed) snap_go(k_snap<float>, ex, sys, st, a, t, t.group_f, t.smem_bytes_f, sys_only, with_pe, flags, stream);
+  if (mixed) snap_go(k_snap, ex, sys, st, a, t, t.group_f, t.smem_bytes_f, sys_only, with_pe, flags, stream);
   else snap_go(k_snap64, ex, sys, st, a, t, t.group, t.smem_bytes, sys_only, with_pe, flags, stream);
   return launches + 1;
 }

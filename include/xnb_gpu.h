@@ -38,7 +38,7 @@ extern "C" {
 
 /* Precision of the force traversal. */
 #define XNB_PREC_FP64_EXACT 0 /* the reference functor's operations, bit-identical to its CPU path */
-#define XNB_PREC_FP64 1       /* FP64, same pair set, reciprocal by Newton-Raphson, FMA */
+#define XNB_PREC_FP64 1       /* FP64, same pair set, reciprocal from an FP32 seed by one third-order step, FMA */
 #define XNB_PREC_MIXED 2      /* FP64 positions/displacements/accumulation/integration; FP32 r^2, r^-6, |F| */
 /* Flag OR-ed into XNB_PREC_FP64 or XNB_PREC_MIXED: each pair inside rc is evaluated
  * once (lower half of the sorted list, the reference's symmetric split) and the
@@ -240,7 +240,8 @@ typedef struct xnb_tuning {
 int xnb_batch_set_force_lanes(xnb_batch* b, int32_t lanes);
 
 /* Form of the mixed-precision full-list force traversal:
- * XNB_FORCE_THREAD: one thread per particle, neighbours gathered from global memory (default);
+ * XNB_FORCE_THREAD: neighbours gathered from global memory, one thread per particle above
+ *   XNB_MIXED_SPLIT_MAX particles (default);
  * XNB_FORCE_STAGED: one block per segment of 8 x-adjacent cells of a row, whose
  *   neighbourhood (9 rows of 10 cells, periodic images included) is copied into
  *   shared memory first; the lists are read in a compact (cell group, index in
@@ -260,8 +261,8 @@ int xnb_batch_set_force_form(xnb_batch* b, int32_t form);
  *   x-adjacent cells, each cell's mirrors one bulk copy (cp.async.bulk) into
  *   shared memory, the next row's copy in flight while the current row is tested.
  * XNB_BUILD_WARP: one warp per cell, one lane per candidate; the whole 27-cell
- *   block (up to stage_cap candidates) staged by the warp, six particles tested
- *   per staged load with a ballot each.
+ *   block (up to stage_cap candidates within reach) staged by the warp, four
+ *   particles tested per staged load with a ballot each.
  * Cells neither form takes (more than 64 particles, or candidates over the
  * stage) are built block-per-cell. */
 #define XNB_BUILD_ROWS 0
