@@ -1143,7 +1143,7 @@ int xnb_step(xnb_batch* b, int32_t nsteps, int32_t precision, int32_t flags, voi
   const bool energy = (flags & XNB_STEP_ENERGY) != 0;
   const bool fused = !(flags & XNB_STEP_HOST_SYNC) && fused_rebin_fits(ex);
   const bool build = fused && fused_build_fits(ex, b->build_form, b->subcell_prune != 0);
-  // a launch that was refused ends the steps (the runtime forgets it at its next good call)
+  // a launch that was refused ends the steps
   cudaGetLastError();
   for (int k = 0; k < nsteps && rc == 0; ++k) {
     // verlet_first_half + trigger_move_particles

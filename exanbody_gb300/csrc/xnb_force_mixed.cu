@@ -369,8 +369,7 @@ void go_walk(const Extent& ex, const SysDesc* sys, const SysState* st, const Dev
   // whose stages leave little L1, gathers from L2 and holds that SM's launch up.
   // Three batches stepping at once: 25 steps of 4M atoms 69.6 to 77 -> 67.0 ms, 20
   // steps of 96 small systems 42.2 -> 35.4 ms; one alone 69.7 / 70.0 and 38.3 / 38.6.
-  cudaFuncSetAttribute(k_force_walk<PE, KICK>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                       cudaSharedmemCarveoutMaxL1);
+  set_attribute(k_force_walk<PE, KICK>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxL1);
   k_force_walk<PE, KICK><<<(ex.n_part + threads - 1u) / threads, threads, 0, stream>>>(
       ex.n_part, BatchSource(sys, st, a, sys_only), a);
 }

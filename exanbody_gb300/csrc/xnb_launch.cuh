@@ -11,12 +11,18 @@ constexpr int kStageCapMax = 1024;       // candidates per stage of the neighbou
 constexpr uint32_t kMaxListBuf = 1024;   // entries per list buffer of its block-per-cell form
 constexpr size_t kSmemPerBlock = 227 * 1024;  // what a block of an sm_103 may have
 
-// Raises a kernel's limit on dynamic shared memory on the current device. `most` is
-// the largest that any launch of the kernel asks for, not this launch's: the limit
-// belongs to the kernel, and a second host thread's launch may follow it.
+// Sets a kernel's attribute on the current device. Setting one that succeeds clears the
+// thread's last error: that of a launch refused before it is kept for check_launch.
+template <class Kernel>
+inline void set_attribute(Kernel kern, cudaFuncAttribute what, int value) {
+  if (cudaPeekAtLastError() == cudaSuccess) cudaFuncSetAttribute(kern, what, value);
+}
+// Raises a kernel's limit on dynamic shared memory. `most` is the largest that any
+// launch of the kernel asks for, not this launch's: the limit belongs to the kernel,
+// and a second host thread's launch may follow it.
 template <class Kernel>
 inline void raise_smem_limit(Kernel kern, size_t most) {
-  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(most));
+  set_attribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(most));
 }
 
 enum Precision : int { kFp64Exact = 0, kFp64 = 1, kMixed = 2 };

@@ -469,13 +469,13 @@ class Batch:
         _ck(self.lib.xnb_batch_set_tuning(self.h, int(stage_cap), int(force_block)))
 
     def set_force_lanes(self, lanes):
-        """Threads per particle (1, 2 or 4) of the mixed full-list force traversal of batches of more than 50,000
-        particles (others spread a list over threads by themselves)."""
+        """Threads per particle (1, 2 or 4) of the mixed full-list force traversal of batches of more than
+        MIXED_SPLIT_MAX particles (others spread a list over threads by themselves)."""
         _ck(self.lib.xnb_batch_set_force_lanes(self.h, int(lanes)))
 
     def set_force_form(self, form):
-        """FORCE_THREAD (one thread per particle, default) or FORCE_STAGED (cell
-        segments staged in shared memory) for the mixed full-list traversal."""
+        """FORCE_THREAD (neighbours gathered from global memory, default) or FORCE_STAGED
+        (cell segments staged in shared memory) for the mixed full-list traversal."""
         _ck(self.lib.xnb_batch_set_force_form(self.h, int(form)))
 
     def set_build_form(self, form):
